@@ -30,7 +30,7 @@
 // Layout (internal order unless noted):
 //   x4 = (position, mass), v4 = (velocity, 0), ps[b] = (predicted position, mass), rref = rank of
 //   the particle in the reference order; neighbour lists in uint4 tiles (pbf_pairs.cuh) of
-//   internal indices; xref[r] = (predicted position, mass) in reference order, Kr[r] = its hash.
+//   internal indices; Kr[r] = the hash of the particle of reference rank r.
 #pragma once
 
 #include <cstdint>
@@ -189,8 +189,7 @@ __global__ void __launch_bounds__(kIoBlock)
 
 // Moves the state into the new internal order (slot s holds the particle of import index
 // sp_import[s], reference rank rank_of_import[...]) and writes the predicted positions, both maps
-// between ranks and slots, the reference-ordered predicted positions and the debug order
-// (pre-sort record index per rank).
+// between ranks and slots and the debug order (pre-sort record index per rank).
 __global__ void __launch_bounds__(kElemBlock)
     k_gather(const StepParams* __restrict__ P, const uint32_t* __restrict__ sp_import,
              const uint32_t* __restrict__ rank_of_import, const float4* __restrict__ x4,
@@ -198,7 +197,7 @@ __global__ void __launch_bounds__(kElemBlock)
              const float* __restrict__ size, const uint32_t* __restrict__ rref_old,
              float4* __restrict__ x4g, float4* __restrict__ col4g, float* __restrict__ sizeg,
              float4* __restrict__ ps0, uint32_t* __restrict__ r2i, uint32_t* __restrict__ rank_of,
-             float4* __restrict__ xref, uint32_t* __restrict__ order_out,
+             uint32_t* __restrict__ order_out,
              const float* __restrict__ rho_in, const float* __restrict__ lam_in,
              const float4* __restrict__ dp_in, float* __restrict__ rho_out,
              float* __restrict__ lam_out, float4* __restrict__ dp_out, int carry,
@@ -230,7 +229,6 @@ __global__ void __launch_bounds__(kElemBlock)
         ps0[s] = q;
         r2i[r] = (uint32_t)s;
         rank_of[s] = r;
-        xref[r] = q;
         order_out[r] = rref_old[o];
         if (carry) {
             rho_out[s] = rho_in[o];

@@ -33,14 +33,17 @@ __device__ __forceinline__ float2 len2_2(float2 x, float2 y, float2 z) {
     return fma2(z, z, fma2(x, x, mul2(y, y)));
 }
 
+// IN_REACH: the caller knows r2 <= h2 (a list's entries at the positions that made the list).
+template <bool IN_REACH = false>
 __device__ __forceinline__ float2 poly6_2(const StepParams& p, float2 r2) {
     const float2 d = sub2(f2(p.h2), r2);
     const float2 w = mul2(f2(p.kp), mul2(mul2(d, d), d));
+    if (IN_REACH) return w;
     return make_float2(r2.x > p.h2 ? 0.0f : w.x, r2.y > p.h2 ? 0.0f : w.y);
 }
 
 // Spiky gradient coefficient c with grad W = c * r (per lane).
-template <bool EXACT>
+template <bool EXACT, bool IN_REACH = false>
 __device__ __forceinline__ void spiky2(const StepParams& p, float2 sx, float2 sy, float2 sz,
                                        float2 r2, float2& gx, float2& gy, float2& gz) {
     if constexpr (EXACT) {
@@ -57,8 +60,8 @@ __device__ __forceinline__ void spiky2(const StepParams& p, float2 sx, float2 sy
         const float2 r = mul2(r2, ir);
         const float2 q = sub2(f2(p.h), r);
         float2 c = mul2(mul2(f2(p.ks), mul2(q, q)), ir);
-        if (r2.x > p.h2 || r2.x < 1e-10f) c.x = 0.f;
-        if (r2.y > p.h2 || r2.y < 1e-10f) c.y = 0.f;
+        if ((!IN_REACH && r2.x > p.h2) || r2.x < 1e-10f) c.x = 0.f;
+        if ((!IN_REACH && r2.y > p.h2) || r2.y < 1e-10f) c.y = 0.f;
         gx = mul2(c, sx);
         gy = mul2(c, sy);
         gz = mul2(c, sz);
@@ -105,15 +108,16 @@ struct DensityLambda2 {
         rho = mi * p.w0;
         gx = gy = gz = sum = 0.f;
     }
+    template <bool IN_REACH = false>
     __device__ __forceinline__ void add2(const StepParams& p, float4 xi, float4 a, float4 b,
                                          bool two) {
         const float2 sx = sub2(f2(xi.x), make_float2(a.x, b.x));
         const float2 sy = sub2(f2(xi.y), make_float2(a.y, b.y));
         const float2 sz = sub2(f2(xi.z), make_float2(a.z, b.z));
         const float2 r2 = len2_2(sx, sy, sz);
-        const float2 w = poly6_2(p, r2);
+        const float2 w = poly6_2<IN_REACH>(p, r2);
         float2 ux, uy, uz;
-        spiky2<EXACT>(p, sx, sy, sz, r2, ux, uy, uz);
+        spiky2<EXACT, IN_REACH>(p, sx, sy, sz, r2, ux, uy, uz);
         const float2 s = mul2(f2(-p.inv_rho0), make_float2(a.w, b.w));
         const float2 l = len2_2(mul2(s, ux), mul2(s, uy), mul2(s, uz));
         rho = __fmaf_rn(a.w, w.x, rho);

@@ -8,26 +8,46 @@
 // The internal order sorts particles by the Morton code of their cell and, inside a cell, by
 // reference rank.  A bucket that holds one cell is therefore a contiguous run of internal slots in
 // the same order the reference walks it: a candidate's slot is directly its list entry.  Buckets
-// flagged as mixed (several cells on one hash, or cells sharing a clamped Morton key) are read in
-// reference order through the reference-ordered positions, their ranks mapped to slots.  Both give
-// the reference's list, entry for entry.
+// flagged as mixed (several cells on one hash, or cells sharing a clamped Morton key) are walked in
+// reference order, their ranks mapped to slots.  Both give the reference's list, entry for entry.
 //
-// Warp-cooperative walk.  A warp takes 32 consecutive particles; consecutive particles of the same
-// cell (a run) share one candidate sequence: the concatenation of the 27 buckets in walk order.
-// For each run, lanes 0..26 look up one bucket each and a warp scan gives each bucket's offset in
-// the sequence.  The sequence is then read 32 candidates at a time, one per lane (coalesced: the
-// buckets are contiguous runs), and every particle of the run tests the whole chunk at once; a
-// ballot and a population count place each hit at the particle's running count plus the hits of
-// lower lanes, which is the reference's order.  Each candidate is loaded once per run instead of
-// once per particle, and no lane idles on another lane's bucket length.  Two particles are tested
-// per round (independent ballots and placements, distances in packed FP32x2): their dependency
-// chains interleave, which a lane-serial walk or a windowed one (both measured slower) cannot.
+// Warp-cooperative walk.  A warp takes 32 consecutive particles (8 or 16 in small scenes, see
+// search_per_warp); consecutive particles of the same cell (a run) share one candidate sequence: the concatenation of the 27 buckets in walk order.
 //
-// The first STAGE entries of each list are staged in shared memory and written out as coalesced
-// uint4 tiles (pbf_pairs.cuh).  The block size and STAGE (the walk's tile shape) are template
-// parameters; the solver's autotuner picks them by measurement (lists do not depend on them).
-// When `density` is set, the first Jacobi iteration's density and lambda are accumulated over the
-// finished list, one thread per particle (same terms, same order as k_density_lambda).
+//   stage    lanes 0..26 look up one bucket each (the next run's lookups are in flight meanwhile),
+//            a warp scan gives each bucket's offset, and the lanes write the sequence's slots into
+//            the warp's pool of shared memory;
+//   cull     candidates out of reach of the box around the run's particles leave the sequence (the
+//            rest keep their order): half of them, as a run is about seven particles that fill
+//            part of a cell.  The test is the pair test at the box's nearest point; rounding is
+//            monotonic, so nothing a particle could accept is dropped;
+//   test     64 candidates at a time, two per lane, against the run's particles, two per round in
+//            packed FP32x2.  A round's four ballots are all it leaves behind (hit masks in the
+//            pool): no counts, no placement and no self test, two shared loads, twelve packed
+//            operations, four compares and ballots and one store per 128 pairs.  A particle's
+//            own slot is cleared from its mask by the lane that holds it as a candidate;
+//   extract  once the pool is full or the warp's runs are staged, every lane turns its own
+//            particle's masks into its list, all 32 lanes at once (a run alone would keep a fifth
+//            of them busy): four set bits at a time become a tile, written as one coalesced uint4,
+//            and its four candidates feed the first Jacobi iteration's density and lambda (same
+//            terms, same order as k_density_lambda), so the list is not read back.
+//
+// What bounds it is instruction issue (70% of the issue slots at 32 warps per SM; 207 M warp
+// instructions at 1M particles with 35 neighbours, against 319 M for a walk that placed every hit
+// as it was found): the distance tests (210-270 candidates a particle before the cull) and the
+// extraction.  Measured on that scene, 394 us before: hit masks and extraction 358 us, with one
+// pool for masks and candidates 316, 64 candidates per round 279, masks with hits named by a bit
+// and the reach tests of list entries dropped 265, the next run's lookup in flight 262; the cull
+// makes the pool a third smaller and the walk's chain shorter: 270 at 1M, 2,196 against 2,231 at
+// 8M, 30 against 36 at 27k.
+//
+// A run whose sequence does not fit the pool (pile-ups, or a walk cell much wider than h) goes
+// through the same stages in segments of the sequence and stops once every list is full; its
+// lists are placed entry by entry and read back for the density.
+//
+// The block size and STAGE (the walk's tile shape: a pool of 32 x STAGE words per warp) are
+// template parameters; the solver's autotuner picks them by measurement (lists do not depend on
+// them).
 #pragma once
 
 #include <cstdint>
@@ -39,43 +59,66 @@
 
 namespace akua {
 
-constexpr int kSearchBlock = 128;  // default tile shape: 128 threads, 32 staged entries
+// Default tile shape.  At 1M particles the walk takes 273 us with 64 or 128 threads and 32 x 32
+// words, 294 with 32 x 48 (fewer warps fit an SM) and 404 with 32 x 16 (a warp's runs no longer
+// fit the pool at once, so the extraction runs several times with few lanes).
+constexpr int kSearchBlock = 128;
 constexpr int kListStage = 32;
-// Row stride in words of STAGE staged entries: STAGE + 4 words, an odd number of 16-byte units
-// (9 for 32, 5 for 16), so the uint4 rows of a warp's lanes fall in different banks.
-__host__ __device__ constexpr int list_row(int stage) { return stage + 4; }
-__host__ __device__ constexpr size_t search_smem(int block, int stage) {
-    return sizeof(uint32_t) * block * list_row(stage) + sizeof(float4) * block;
+
+// Particles per warp.  32 keep every lane of the extraction busy, but a warp works through its runs
+// one after another, so with few warps the walk lasts as long as one warp: a scene whose warps of
+// 8 (or 16) particles still all fit the chip at once (32 warps per SM: 64 registers per thread)
+// takes them.  Measured (us, at 8 / 16 / 32): 1,000 particles 18 / 21 / 25, 27,000 26 / 27 / 30,
+// 50,000 39 / 32 / 36, 70,000 48 / 36 / 40, 100,000 63 / 51 / 45.
+constexpr int kSearchWarps = 32;
+inline int search_per_warp(int n, int sms) {
+    for (int w = 8; w < 32; w *= 2)
+        if (n <= w * kSearchWarps * sms) return w;
+    return 32;
 }
-constexpr size_t kSearchSmem = search_smem(kSearchBlock, kListStage);
+constexpr int kPairWords = 3 * 32;  // a run's positions, two particles interleaved
+// Words of shared memory per warp: the pool of candidates and hit masks, then the positions.
+__host__ __device__ constexpr int search_words(int stage) { return 32 * stage + kPairWords; }
+__host__ __device__ constexpr size_t search_smem(int block, int stage) {
+    return sizeof(uint32_t) * (block / 32) * search_words(stage);
+}
+constexpr uint32_t kRunMax = 32 * 32;  // candidates whose chunks one 32-bit mask can name
 constexpr uint32_t kFullWarp = 0xffffffffu;
 constexpr uint32_t kMixedBucket = 0x80000000u;  // bucket table: y bit for a mixed bucket
-constexpr uint32_t kDenseRun = 2048;  // candidates of a run beyond which the walk may stop early
+
+// The smallest value of a warp's lanes (NaN is ignored).
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
 
 template <bool EXACT, int BLOCK, int STAGE>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
     k_search(const StepParams* __restrict__ P, const float4* __restrict__ ps,
-             const float4* __restrict__ xref, const uint2* __restrict__ table,
-             const uint32_t* __restrict__ r2i, uint32_t* __restrict__ nbr,
-             uint32_t* __restrict__ cnt, float* __restrict__ rho_out, float* __restrict__ lam_out,
-             uint32_t* __restrict__ flags, int density, const float* __restrict__ speed,
-             const float* __restrict__ lprev, float* __restrict__ lacc,
-             float* __restrict__ feat, float4* __restrict__ psl) {
-    extern __shared__ __align__(16) uint32_t stage[];
+             const uint2* __restrict__ table, const uint32_t* __restrict__ r2i,
+             uint32_t* __restrict__ nbr, uint32_t* __restrict__ cnt, float* __restrict__ rho_out,
+             float* __restrict__ lam_out, uint32_t* __restrict__ flags, int density,
+             const float* __restrict__ speed, const float* __restrict__ lprev,
+             float* __restrict__ lacc, float* __restrict__ feat, float4* __restrict__ psl,
+             int per_warp) {
+    extern __shared__ __align__(16) uint32_t smem[];
     const StepParams& p = *P;
     const int n = p.n;
     const int lane = threadIdx.x & 31;
-    const int wbase = threadIdx.x & ~31;
-    constexpr int kListRow = list_row(STAGE);
-    const int base = blockIdx.x * BLOCK + wbase;  // this warp's first particle
-    if (base >= n) return;                               // uniform over the warp
+    // this warp's first particle (at most n plus a block's particles)
+    const int base = (blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5)) * per_warp;
+    if (base >= n) return;  // uniform over the warp
     const int i = base + lane;
-    const bool valid = i < n;
-    float4* xs = reinterpret_cast<float4*>(stage + BLOCK * kListRow) + wbase;
-    uint32_t* rows = stage + wbase * kListRow;
+    const int nvalid = min(per_warp, n - base);
+    const bool valid = lane < nvalid;
+    constexpr uint32_t kPool = 32 * STAGE;
+    uint32_t* pool = smem + (threadIdx.x >> 5) * search_words(STAGE);
+    float* pairs = reinterpret_cast<float*>(pool + kPool);
+    const float4* pair_xy = reinterpret_cast<const float4*>(pairs);  // (xa, xb, ya, yb)
+    const float2* pair_z = reinterpret_cast<const float2*>(pairs + 64);
 
     const float4 xi = valid ? ps[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    xs[lane] = xi;
     const int cx = cell_coord(xi.x, p.search_cell);
     const int cy = cell_coord(xi.y, p.search_cell);
     const int cz = cell_coord(xi.z, p.search_cell);
@@ -87,135 +130,126 @@ __global__ void __launch_bounds__(BLOCK)
     const int ps_ = __shfl_up_sync(kFullWarp, sid, 1);
     uint32_t starts = __ballot_sync(
         kFullWarp, valid && (lane == 0 || px != cx || py != cy || pz != cz || ps_ != sid));
-    const int nvalid = min(32, n - base);
-    __syncwarp();
 
     const float h2 = p.h2;
     const int cap = p.cap;
     const uint32_t below = (1u << lane) - 1u;
-    int count = 0;  // lane q: running list length of particle base + q
-    while (starts) {
-        const int q0 = __ffs(starts) - 1;
-        starts &= starts - 1;
-        const int q1 = starts ? __ffs(starts) - 1 : nvalid;
-        const int rx = __shfl_sync(kFullWarp, cx, q0);
-        const int ry = __shfl_sync(kFullWarp, cy, q0);
-        const int rz = __shfl_sync(kFullWarp, cz, q0);
-        const StepParams& pr = P[__shfl_sync(kFullWarp, sid, q0)];  // the run's scene
-        // lane b < 27 holds bucket b of the walk (dx = b/9 - 1, dy = b/3%3 - 1, dz = b%3 - 1)
+    const float inf = __int_as_float(0x7f800000);
+    uint4* out4 = reinterpret_cast<uint4*>(nbr);
+
+    // the bucket of the walk this lane looks up (dx = b/9 - 1, dy = b/3%3 - 1, dz = b%3 - 1)
+    const int bdx = lane / 9 - 1, bdy = lane / 3 % 3 - 1, bdz = lane % 3 - 1;
+    auto lookup = [&](uint32_t runs) {  // for the run starting at the lowest bit of `runs`
+        const int q = __ffs(runs) - 1;
+        const int rx = __shfl_sync(kFullWarp, cx, q);
+        const int ry = __shfl_sync(kFullWarp, cy, q);
+        const int rz = __shfl_sync(kFullWarp, cz, q);
+        const StepParams& pr = P[__shfl_sync(kFullWarp, sid, q)];  // the run's scene
         uint2 e = make_uint2(0u, 0u);
         if (lane < 27)
             e = __ldg(table + pr.table_offset +
-                      cell_hash(rx + lane / 9 - 1, ry + lane / 3 % 3 - 1, rz + lane % 3 - 1,
-                                pr.table_size, pr.table_magic));
-        const uint32_t blen = e.y & ~kMixedBucket;
-        uint32_t incl = blen;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFullWarp, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const uint32_t off = incl - blen;  // lanes 27..31: the sequence length
-        const uint32_t total = __shfl_sync(kFullWarp, incl, 31);
+                      cell_hash(rx + bdx, ry + bdy, rz + bdz, pr.table_size, pr.table_magic));
+        return e;
+    };
 
-        // one chunk of 32 candidates of the run's sequence
-        auto chunk = [&](uint32_t c0) {
-            const uint32_t at = c0 + lane;
-            int b = 0;  // the last bucket starting at or before `at`
-#pragma unroll
-            for (int step = 16; step; step >>= 1)
-                if (__shfl_sync(kFullWarp, off, b + step) <= at) b += step;
-            const uint32_t bx = __shfl_sync(kFullWarp, e.x, b);
-            const uint32_t by = __shfl_sync(kFullWarp, e.y, b);
-            const uint32_t bo = __shfl_sync(kFullWarp, off, b);
-            const bool live = at < total;
-            float4 c = make_float4(__int_as_float(0x7f800000), __int_as_float(0x7f800000),
-                                   __int_as_float(0x7f800000), 0.f);
-            uint32_t j = 0xffffffffu;
-            if (live) {
-                const uint32_t t = bx + (at - bo);
-                if (by & kMixedBucket) {
-                    c = __ldg(xref + t);
-                    j = __ldg(r2i + t);
-                } else {
-                    c = __ldg(ps + t);
-                    j = t;
-                }
+    // Culls `total` staged candidates at `seq` (the first word of an even offset) against the run
+    // of particles [q0, q0 + m) and tests the rest: returns their number; their masks follow them,
+    // [64 candidates][particle][2 words], from the next even word.
+    auto test = [&](uint32_t* seq, uint32_t total, int q0, int m) {
+        const bool own = lane >= q0 && lane < q0 + m;
+        if (own) {
+            const int r = lane - q0;
+            pairs[4 * (r >> 1) + (r & 1)] = xi.x;
+            pairs[4 * (r >> 1) + 2 + (r & 1)] = xi.y;
+            pairs[64 + r] = xi.z;
+        }
+        const float lx = warp_min(own ? xi.x : inf), hx = warp_min(own ? -xi.x : inf);
+        const float ly = warp_min(own ? xi.y : inf), hy = warp_min(own ? -xi.y : inf);
+        const float lz = warp_min(own ? xi.z : inf), hz = warp_min(own ? -xi.z : inf);
+        __syncwarp();
+        uint32_t kept = 0;
+        uint32_t jn = lane < total ? seq[lane] : 0u;
+        float4 cn = __ldg(ps + jn);
+        for (uint32_t c0 = 0; c0 < total; c0 += 32) {
+            const uint32_t j = jn;
+            const float4 c = cn;
+            const bool live = c0 + lane < total;
+            if (c0 + 32 < total) {
+                jn = c0 + 32 + lane < total ? seq[c0 + 32 + lane] : 0u;
+                cn = __ldg(ps + jn);
             }
-            // two particles per round: independent tests, ballots and placements
-            const uint32_t jrel = j - (uint32_t)base;  // == q for particle q's own slot
-            const float2 cxx = f2(c.x), cyy = f2(c.y), czz = f2(c.z);
-            auto place = [&](int q, int pos) {
-                if (pos < STAGE) rows[q * kListRow + pos] = j;
-                else if (pos < cap) nbr[4 * ((size_t)(pos >> 2) * n + base + q) + (pos & 3)] = j;
-            };
-            int q = q0;
-            for (; q + 1 < q1; q += 2) {
-                const float4 xa = xs[q], xb = xs[q + 1];
-                const float2 d2 = len2_2(sub2(make_float2(xa.x, xb.x), cxx),
-                                         sub2(make_float2(xa.y, xb.y), cyy),
-                                         sub2(make_float2(xa.z, xb.z), czz));
-                const bool ha = d2.x < h2 && jrel != (uint32_t)q;
-                const bool hb = d2.y < h2 && jrel != (uint32_t)(q + 1);
-                const uint32_t ba = __ballot_sync(kFullWarp, ha);
-                const uint32_t bb = __ballot_sync(kFullWarp, hb);
-                const int pa = __shfl_sync(kFullWarp, count, q) + __popc(ba & below);
-                const int pb = __shfl_sync(kFullWarp, count, q + 1) + __popc(bb & below);
-                if (ha) place(q, pa);
-                if (hb) place(q + 1, pb);
-                count += lane == q ? __popc(ba) : (lane == q + 1 ? __popc(bb) : 0);
-            }
-            if (q < q1) {
-                const float4 xq = xs[q];
-                const bool hit = len2(xq.x - c.x, xq.y - c.y, xq.z - c.z) < h2 && jrel != (uint32_t)q;
-                const uint32_t bal = __ballot_sync(kFullWarp, hit);
-                const int pos = __shfl_sync(kFullWarp, count, q) + __popc(bal & below);
-                if (hit) place(q, pos);
-                if (lane == q) count += __popc(bal);
-            }
+            const float dx = fmaxf(fmaxf(lx - c.x, c.x + hx), 0.f);
+            const float dy = fmaxf(fmaxf(ly - c.y, c.y + hy), 0.f);
+            const float dz = fmaxf(fmaxf(lz - c.z, c.z + hz), 0.f);
+            const bool keep = live && len2(dx, dy, dz) < h2;
+            const uint32_t bal = __ballot_sync(kFullWarp, keep);
+            if (keep) seq[kept + __popc(bal & below)] = j;  // at or before what is still to be read
+            kept += __popc(bal);
+        }
+        __syncwarp();
+        uint2* put = reinterpret_cast<uint2*>(seq + ((kept + 1u) & ~1u));
+        auto fetch = [&](uint32_t at, uint32_t& j) {
+            j = at < kept ? seq[at] : 0xffffffffu;
+            return at < kept ? __ldg(ps + j) : make_float4(inf, inf, inf, 0.f);
         };
-        if (total <= kDenseRun) {
-            for (uint32_t c0 = 0; c0 < total; c0 += 32) chunk(c0);
-        } else {
-            // a pile-up far denser than any cell of a resting fluid: stop once every list of the
-            // run is full (later hits are neither stored nor needed for the overflow flag; a list
-            // fills only after at least cap candidates), or such a run would cost run size x
-            // sequence length tests
-            for (uint32_t c0 = 0; c0 < total; c0 += 32) {
-                if (c0 >= (uint32_t)cap &&
-                    __all_sync(kFullWarp, lane < q0 || lane >= q1 || count >= cap))
-                    break;
-                chunk(c0);
+        for (uint32_t c0 = 0; c0 < kept; c0 += 64, put += m) {
+            uint32_t j0, j1;
+            const float4 c = fetch(c0 + lane, j0), d = fetch(c0 + 32 + lane, j1);
+            const float2 cx2 = f2(-c.x), cy2 = f2(-c.y), cz2 = f2(-c.z);
+            const float2 dx2 = f2(-d.x), dy2 = f2(-d.y), dz2 = f2(-d.z);
+            for (int r = 0; r < m; r += 2) {
+                const float4 a = pair_xy[r >> 1];
+                const float2 z = pair_z[r >> 1];
+                const float2 ax = make_float2(a.x, a.y), ay = make_float2(a.z, a.w);
+                const float2 rc = len2_2(add2(ax, cx2), add2(ay, cy2), add2(z, cz2));
+                const float2 rd = len2_2(add2(ax, dx2), add2(ay, dy2), add2(z, dz2));
+                const uint32_t ca = __ballot_sync(kFullWarp, rc.x < h2);
+                const uint32_t cb = __ballot_sync(kFullWarp, rc.y < h2);
+                const uint32_t da = __ballot_sync(kFullWarp, rd.x < h2);
+                const uint32_t db = __ballot_sync(kFullWarp, rd.y < h2);
+                if (lane < min(2, m - r))  // lanes 0 and 1 store a particle's masks each
+                    put[r + lane] = lane ? make_uint2(cb, db) : make_uint2(ca, da);
+            }
+            __syncwarp();
+            const uint32_t s0 = j0 - (uint32_t)(base + q0), s1 = j1 - (uint32_t)(base + q0);
+            if (s0 < (uint32_t)m) atomicAnd(&put[s0].x, ~(1u << lane));
+            if (s1 < (uint32_t)m) atomicAnd(&put[s1].y, ~(1u << lane));
+        }
+        __syncwarp();
+        return kept;
+    };
+
+    // This lane's hits, in order: its masks at `mask` (chunk pair k at mask[k * stride]), its
+    // candidates at `seq`.
+    struct Hits {
+        const uint2* mask;
+        const uint32_t* seq;
+        const uint32_t* at;  // the current chunk's candidates
+        int stride, count;
+        uint32_t left, bits;  // chunks with hits still to come, hits of the current chunk
+        __device__ __forceinline__ Hits(const uint32_t* s, uint32_t kept, int r, int m)
+            : mask(reinterpret_cast<const uint2*>(s + ((kept + 1u) & ~1u)) + r), seq(s), at(s),
+              stride(m), count(0), left(0u), bits(0u) {
+            for (uint32_t k = 0; 64 * k < kept; ++k) {
+                const uint2 w = mask[k * stride];
+                count += __popc(w.x) + __popc(w.y);
+                left |= ((w.x ? 1u : 0u) | (w.y ? 2u : 0u)) << (2 * k);
             }
         }
-    }
-    __syncwarp();
-    if (!valid) return;
-    const int total_count = count;
-    count = count < cap ? count : cap;
-    cnt[i] = (uint32_t)count;
-    if (total_count >= cap) atomicOr(flags, 1u);
-    const uint32_t* myrow = rows + lane * kListRow;
-
-    // staged entries -> global tiles (a partial last tile carries unused words)
-    const int staged = min(count, STAGE);
-    const uint4* row4 = reinterpret_cast<const uint4*>(myrow);
-    uint4* out4 = reinterpret_cast<uint4*>(nbr);
-    for (int g = 0; g < (staged + 3) >> 2; ++g) out4[(size_t)g * n + i] = row4[g];
-
-    // first iteration's density and lambda over the finished list, read in uint4 tiles (staged
-    // rows are conflict-free that way)
-    if (density) {
-        DensityLambda2<EXACT> acc;
-        acc.init(xi.w, p);
-        const uint4* tiles = reinterpret_cast<const uint4*>(nbr) + i;
-        for (int g = 0; 4 * g < count; ++g) {
-            const uint4 e = g < STAGE / 4 ? row4[g] : tiles[(size_t)g * n];
-            const int left = count - 4 * g;
-            acc.add2(p, xi, __ldg(ps + e.x), __ldg(ps + (left >= 2 ? e.y : e.x)), left >= 2);
-            if (left > 2)
-                acc.add2(p, xi, __ldg(ps + e.z), __ldg(ps + (left >= 4 ? e.w : e.z)), left >= 4);
+        __device__ __forceinline__ uint32_t next() {  // only called while hits remain
+            if (bits == 0u) {
+                const int k = __ffs(left) - 1;
+                left &= left - 1;
+                bits = reinterpret_cast<const uint32_t*>(mask + (k >> 1) * stride)[k & 1];
+                at = seq + 32 * k;
+            }
+            const uint32_t j = at[__ffs(bits) - 1];
+            bits &= bits - 1;
+            return j;
         }
+    };
+    // Density, lambda and the network's features of this lane's finished list.
+    auto finish = [&](const DensityLambda2<EXACT>& acc, int count) {
         rho_out[i] = acc.rho;
         const float l = acc.lambda(p);
         lam_out[i] = l;
@@ -225,6 +259,147 @@ __global__ void __launch_bounds__(BLOCK)
             write_features(params_for(P, i), acc, l, count, lprev[i], speed[i],
                            feat + (size_t)kFeatures * i);
         }
+    };
+
+    uint2 e_next = lookup(starts);
+    while (starts) {
+        uint32_t used = 0;       // words of the pool in use (even)
+        uint32_t my_seq = 0;     // this lane's run: its candidates' place in the pool,
+        uint32_t my_kept = 0;    // how many they are,
+        int my_q0 = -1;          // its first lane (-1: this lane's run is not in the pool)
+        int my_m = 0;            // and its particles
+        while (starts) {
+            const int q0 = __ffs(starts) - 1;
+            const uint32_t rest = starts & (starts - 1);
+            const int q1 = rest ? __ffs(rest) - 1 : nvalid;
+            const int m = q1 - q0;
+            const uint2 e = e_next;
+            const uint32_t blen = e.y & ~kMixedBucket;
+            uint32_t incl = blen;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(kFullWarp, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const uint32_t off = incl - blen;  // lanes 27..31: the sequence length
+            const uint32_t total = __shfl_sync(kFullWarp, incl, 31);
+            const uint32_t words = ((total + 1u) & ~1u) + 2u * ((total + 63u) >> 6) * m;
+
+            // a dense run: segments of its sequence, the pool to itself
+            if (words > kPool || total > kRunMax) {
+                if (used) break;
+                constexpr uint32_t kSegment = kPool / 2;  // its masks take as much again at most
+                static_assert(kSegment <= kRunMax, "a segment's chunks must fit Hits::left");
+                int count = 0;
+                for (uint32_t s0 = 0; s0 < total; s0 += kSegment) {
+                    // later hits of full lists are neither stored nor needed for the overflow flag
+                    if (__all_sync(kFullWarp, lane < q0 || lane >= q1 || count >= cap)) break;
+                    const uint32_t len = min(kSegment, total - s0);
+                    for (uint32_t c0 = 0; c0 < len; c0 += 32) {
+                        const uint32_t at = s0 + c0 + lane;
+                        int b = 0;  // the last bucket starting at or before `at`
+#pragma unroll
+                        for (int step = 16; step; step >>= 1)
+                            if (__shfl_sync(kFullWarp, off, b + step) <= at) b += step;
+                        const uint32_t bx = __shfl_sync(kFullWarp, e.x, b);
+                        const uint32_t by = __shfl_sync(kFullWarp, e.y, b);
+                        const uint32_t t = bx + (at - __shfl_sync(kFullWarp, off, b));
+                        if (c0 + lane < len)
+                            pool[c0 + lane] = (by & kMixedBucket) ? __ldg(r2i + t) : t;
+                    }
+                    __syncwarp();
+                    const uint32_t kept = test(pool, len, q0, m);
+                    if (lane >= q0 && lane < q1) {
+                        Hits hits(pool, kept, lane - q0, m);
+                        for (int k = 0; k < hits.count && count + k < cap; ++k) {
+                            const int pos = count + k;
+                            nbr[4 * ((size_t)(pos >> 2) * n + i) + (pos & 3)] = hits.next();
+                        }
+                        count += hits.count;
+                    }
+                    __syncwarp();
+                }
+                if (lane >= q0 && lane < q1) {
+                    if (count >= cap) atomicOr(flags, 1u);
+                    count = min(count, cap);
+                    cnt[i] = (uint32_t)count;
+                    if (density) {
+                        DensityLambda2<EXACT> acc;
+                        acc.init(xi.w, p);
+                        for (int g = 0; 4 * g < count; ++g) {
+                            const uint4 t = out4[(size_t)g * n + i];
+                            const int left = count - 4 * g;
+                            acc.template add2<true>(p, xi, __ldg(ps + t.x),
+                                                    __ldg(ps + (left >= 2 ? t.y : t.x)), left >= 2);
+                            if (left > 2)
+                                acc.template add2<true>(p, xi, __ldg(ps + t.z),
+                                                        __ldg(ps + (left >= 4 ? t.w : t.z)),
+                                                        left >= 4);
+                        }
+                        finish(acc, count);
+                    }
+                }
+                if (rest) e_next = lookup(rest);
+                starts = rest;
+                continue;
+            }
+            if (used + words > kPool) break;  // extract first
+            if (rest) e_next = lookup(rest);
+
+            uint32_t* seq = pool + used;
+            const uint32_t longest = __reduce_max_sync(kFullWarp, blen);
+            for (uint32_t k = 0; k < longest; ++k)
+                if (k < blen) seq[off + k] = e.x + k;
+            uint32_t mixed = __ballot_sync(kFullWarp, (e.y & kMixedBucket) != 0u);
+            while (mixed) {  // ranks -> slots
+                const int b = __ffs(mixed) - 1;
+                mixed &= mixed - 1;
+                const uint32_t bx = __shfl_sync(kFullWarp, e.x, b);
+                const uint32_t bl = __shfl_sync(kFullWarp, blen, b);
+                const uint32_t bo = __shfl_sync(kFullWarp, off, b);
+                __syncwarp();
+                for (uint32_t k = lane; k < bl; k += 32) seq[bo + k] = __ldg(r2i + bx + k);
+            }
+            const uint32_t kept = test(seq, total, q0, m);  // synchronises before it reads
+            if (lane >= q0 && lane < q1) {
+                my_seq = used;
+                my_kept = kept;
+                my_q0 = q0;
+                my_m = m;
+            }
+            used += ((kept + 1u) & ~1u) + 2u * ((kept + 63u) >> 6) * m;
+            starts = rest;
+        }
+
+        // extract the lists of the runs in the pool, one lane per particle
+        if (my_q0 >= 0) {
+            Hits hits(pool + my_seq, my_kept, lane - my_q0, my_m);
+            if (hits.count >= cap) atomicOr(flags, 1u);
+            const int count = min(hits.count, cap);
+            cnt[i] = (uint32_t)count;
+            DensityLambda2<EXACT> acc;
+            acc.init(xi.w, p);
+            for (int g = 0; 4 * g < count; ++g) {
+                const int left = count - 4 * g;
+                uint4 t;
+                t.x = hits.next();
+                t.y = t.x;
+                if (left >= 2) t.y = hits.next();
+                t.z = t.y;
+                if (left >= 3) t.z = hits.next();
+                t.w = t.z;
+                if (left >= 4) t.w = hits.next();
+                out4[(size_t)g * n + i] = t;  // a partial last tile repeats its last entry
+                if (density) {
+                    const float4 a = __ldg(ps + t.x), b = __ldg(ps + t.y);
+                    const float4 c = __ldg(ps + t.z), d = __ldg(ps + t.w);
+                    acc.template add2<true>(p, xi, a, b, left >= 2);
+                    if (left > 2) acc.template add2<true>(p, xi, c, d, left >= 4);
+                }
+            }
+            if (density) finish(acc, count);
+        }
+        __syncwarp();
     }
 }
 

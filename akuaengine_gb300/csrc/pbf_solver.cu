@@ -31,6 +31,7 @@ using akua::StepParams;
 
 struct akua_pbf {
     int device = 0;
+    int sms = 1;  // multiprocessors of the device
     int n = 0;
     akua_pbf_config cfg{};
     akua_lambda_corr_params corr{};
@@ -55,7 +56,7 @@ struct akua_pbf {
     float4* dp4 = nullptr;
     // gathered copies and per-step arrays
     float4 *x4g = nullptr, *col4g = nullptr, *ps0 = nullptr, *ps1 = nullptr;
-    float4 *vstar4 = nullptr, *om4 = nullptr, *xv8 = nullptr, *dpg = nullptr, *xref = nullptr;
+    float4 *vstar4 = nullptr, *om4 = nullptr, *xv8 = nullptr, *dpg = nullptr;
     float *sizeg = nullptr, *rhog = nullptr, *lamg = nullptr;
     uint32_t *rrefg = nullptr, *rank_of_import = nullptr, *r2i = nullptr, *order = nullptr;
     // sorts: reference order (A) and Morton order (B)
@@ -148,7 +149,7 @@ cudaError_t dalloc(akua_pbf* s, T** p, size_t count) {
 
 void free_all(akua_pbf* s) {
     void* ptrs[] = {s->d_params, s->x4, s->v4, s->col4, s->size, s->rref, s->rho, s->lam, s->dp4,
-                    s->x4g, s->col4g, s->ps0, s->ps1, s->vstar4, s->om4, s->xv8, s->dpg, s->xref,
+                    s->x4g, s->col4g, s->ps0, s->ps1, s->vstar4, s->om4, s->xv8, s->dpg,
                     s->sizeg, s->rhog, s->lamg, s->rrefg, s->rank_of_import, s->r2i, s->order,
                     s->ka0, s->va0, s->ka1, s->va1, s->kb0, s->vb0, s->kb1, s->vb1,
                     s->sort_scratch, s->sort_scratch_b, s->table, s->nbr, s->cnt, s->flags,
@@ -315,19 +316,24 @@ struct Marker {
     }
 };
 
-// The walk at one tile shape (BLOCK threads, STAGE staged list entries per particle).
+// The walk at one tile shape (BLOCK threads, a pool of 32 x STAGE words per warp).
 template <bool EXACT, int BLOCK, int STAGE>
 void launch_search_shape(akua_pbf* s, cudaStream_t st, int density, float* feat) {
-    akua::k_search<EXACT, BLOCK, STAGE><<<grid_for(s->n, BLOCK), BLOCK,
-                                          akua::search_smem(BLOCK, STAGE), st>>>(
-        s->d_params, s->ps0, s->xref, s->table, s->r2i, s->nbr, s->cnt, s->rho, s->lam,
-        s->flags, density, s->speed, s->lprev, s->lacc, feat, s->psl);
+    constexpr size_t smem = akua::search_smem(BLOCK, STAGE);
+    if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
+        cudaFuncSetAttribute(akua::k_search<EXACT, BLOCK, STAGE>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int per_warp = akua::search_per_warp(s->n, s->sms);
+    akua::k_search<EXACT, BLOCK, STAGE>
+        <<<grid_for(s->n, per_warp * (BLOCK / 32)), BLOCK, smem, st>>>(
+            s->d_params, s->ps0, s->table, s->r2i, s->nbr, s->cnt, s->rho, s->lam, s->flags,
+            density, s->speed, s->lprev, s->lacc, feat, s->psl, per_warp);
 }
 
 template <bool EXACT>
 void launch_search(akua_pbf* s, cudaStream_t st, int density, float* feat) {
     const int b = s->search_block, g = s->search_stage;
-    if (g == 48) {  // 64 or 128 threads (256 x 48 entries would exceed 48 KB of shared memory)
+    if (g == 48) {  // 64 or 128 threads (akua_pbf_set_search_shape refuses 256)
         if (b == 64) launch_search_shape<EXACT, 64, 48>(s, st, density, feat);
         else launch_search_shape<EXACT, 128, 48>(s, st, density, feat);
     } else if (g == 16) {
@@ -429,8 +435,8 @@ void enqueue_body(akua_pbf* s, cudaStream_t st, const char* aos, size_t stride, 
     cudaMemsetAsync(s->mass_bits, 0, sizeof(uint32_t), st);  // "another mass seen" flag
     akua::k_gather<<<ge, akua::kElemBlock, 0, st>>>(
         s->d_params, s->spperm, s->rank_of_import, s->x4, s->v4, s->col4, s->size, s->rref, s->x4g,
-        s->col4g, s->sizeg, s->ps0, s->r2i, s->rrefg, s->xref, s->order, s->rho, s->lam, s->dp4,
-        s->rhog, s->lamg, s->dpg, carry ? 1 : 0, s->lacc, s->lprev,
+        s->col4g, s->sizeg, s->ps0, s->r2i, s->rrefg, s->order, s->rho, s->lam, s->dp4, s->rhog,
+        s->lamg, s->dpg, carry ? 1 : 0, s->lacc, s->lprev,
         learn_mode(s) ? s->speed : nullptr, s->mass_bits);
     mark("k_gather");
     akua::k_table_build<<<ge, akua::kElemBlock, 0, st>>>(s->d_params, s->kr, s->r2i, s->table);
@@ -620,6 +626,7 @@ int create_solver(int32_t n, const akua_pbf_config* cfg, const akua_lambda_corr_
     s->table_size = (uint32_t)((int64_t)cfg->maxNeighbours * n);
     s->table_alloc = s->table_size;
     cudaGetDevice(&s->device);
+    cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device);
     std::vector<uint16_t> sid;
     if (scenes) {
         s->scenes.assign(scenes, scenes + num_scenes);
@@ -650,7 +657,7 @@ int create_solver(int32_t n, const akua_pbf_config* cfg, const akua_lambda_corr_
     chk(dalloc(s, &s->x4g, N)); chk(dalloc(s, &s->col4g, N));
     chk(dalloc(s, &s->ps0, N)); chk(dalloc(s, &s->ps1, N));
     chk(dalloc(s, &s->vstar4, N)); chk(dalloc(s, &s->om4, N)); chk(dalloc(s, &s->xv8, 2 * N));
-    chk(dalloc(s, &s->dpg, N)); chk(dalloc(s, &s->xref, N));
+    chk(dalloc(s, &s->dpg, N));
     chk(dalloc(s, &s->sizeg, N)); chk(dalloc(s, &s->rhog, N)); chk(dalloc(s, &s->lamg, N));
     chk(dalloc(s, &s->rrefg, N)); chk(dalloc(s, &s->rank_of_import, N)); chk(dalloc(s, &s->r2i, N));
     chk(dalloc(s, &s->order, N));
@@ -674,9 +681,6 @@ int create_solver(int32_t n, const akua_pbf_config* cfg, const akua_lambda_corr_
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->side_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming);
-    // every tile shape of the walk fits the default 48 KB of dynamic shared memory
-    static_assert(akua::search_smem(256, 32) <= 48 * 1024 && akua::search_smem(128, 48) <= 48 * 1024,
-                  "walk staging exceeds 48 KB");
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         free_all(s);

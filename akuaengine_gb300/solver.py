@@ -185,7 +185,7 @@ class PBFSolver:
         check(self._lib.akua_pbf_set_pair_blocks(self._h, b), "akua_pbf_set_pair_blocks")
 
     def search_shape(self) -> tuple[int, int]:
-        """The neighbour walk's tile shape: (block size, staged list entries per particle)."""
+        """The neighbour walk's tile shape: (block size, pool words per particle)."""
         b, g = ctypes.c_int32(), ctypes.c_int32()
         check(self._lib.akua_pbf_get_search_shape(self._h, ctypes.byref(b), ctypes.byref(g)),
               "akua_pbf_get_search_shape")

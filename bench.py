@@ -55,8 +55,8 @@ KERNEL_BYTES = {
     "radix_upsweep": lambda L, B: 4,                  # R key (per pass)
     "radix_downsweep": lambda L, B: 16,               # R key, value; W key, value (per pass)
     # R two permutations, x|m, v, colour, size, old rank; W x|m, colour, size, x*|m, rank->slot,
-    # slot->rank, reference-ordered x*|m, order
-    "k_gather": lambda L, B: 8 + 16 + 16 + 16 + 4 + 4 + 16 + 16 + 4 + 16 + 4 + 4 + 16 + 4,
+    # slot->rank, order
+    "k_gather": lambda L, B: 8 + 16 + 16 + 16 + 4 + 4 + 16 + 16 + 4 + 16 + 4 + 4 + 4,
     "k_table_build": lambda L, B: 4 + 4 + 8 * B,      # R keys, slots; W entry
     # R x*|m, 27 bucket entries per cell run; W lists, count, rho, lambda, x*|lambda
     "k_search": lambda L, B: 16 + 27 * 8 * B + L + 4 + 8 + 16,

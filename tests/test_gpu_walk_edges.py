@@ -1,0 +1,70 @@
+"""The neighbour walk where it can go wrong: the particle counts at which it takes another number of
+particles per warp, partial warps, and runs whose candidates do not fit a warp's pool (they go
+through it in segments).  Whole numbers and, with exact math, every record equal the oracle's bit
+for bit."""
+import numpy as np
+import pytest
+
+import akuaengine_gb300 as ak
+from akuaengine_gb300 import LambdaCorrParams, PBFConfig, PBFSolver, scene
+from test_gpu_parity import assert_grid_equal, assert_records_bitexact, run_gpu, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _lib(cuda_lib):
+    return cuda_lib
+
+
+def first_of_block(n, seed):
+    """The first n particles of a lattice block (a ragged last layer) in a box around it."""
+    side = max(2, int(np.ceil(n ** (1.0 / 3.0))))
+    sc = scene.dam_break((side, side, side), (2.0, 1.5, 1.5), seed=seed, jitter_frac=0.1)
+    sc.particles = sc.particles[:n].copy()
+    return sc
+
+
+@pytest.mark.parametrize("where", [9, 31, 33, 65, "8-", "8+", "16-", "16+"])
+def test_particles_per_warp_edges(where):
+    """Counts around a warp and around the lines where the walk goes from 8 to 16 and from 16 to
+    32 particles per warp (8 x 32 and 16 x 32 per multiprocessor)."""
+    if isinstance(where, str):
+        import torch
+
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        n = int(where[:-1]) * 32 * sms + (1 if where.endswith("+") else 0)
+    else:
+        n = where
+    sc = first_of_block(n, seed=n)
+    cfg, corr = PBFConfig(), LambdaCorrParams()
+    g, ge = run_gpu(sc, cfg, corr, 1, ak.OPT_EXACT_MATH)
+    o, oe = run_oracle(sc, cfg, corr, 1)
+    assert_grid_equal(ge, oe, cfg.maxNeighbours)
+    assert_records_bitexact(g, o)
+
+
+@pytest.mark.parametrize("shape", [(64, 16), (64, 32), (128, 48)])
+@pytest.mark.parametrize("kind", ["wide_cell", "cluster", "small_table"])
+def test_runs_longer_than_the_pool(shape, kind):
+    """A walk cell of 2.5 h (sequences of thousands of candidates from buckets that are not the
+    walk's cells), a cluster of 900 particles in a few cells (segments that end inside buckets,
+    lists past the capacity), and the cluster under a table so small that its buckets are mixed
+    and met twice."""
+    sc = first_of_block(3000, seed=5)
+    cfg, corr = PBFConfig(), LambdaCorrParams()
+    if kind == "wide_cell":
+        cfg.spatialHashCellSize = 0.25
+    else:
+        rng = np.random.default_rng(8)
+        sc.particles["position"][:900] = (0.45 + rng.uniform(0.0, 0.17, (900, 3))).astype(np.float32)
+    table = 512 if kind == "small_table" else None
+    o, oe = run_oracle(sc, cfg, corr, 1, table_size=table)
+    p = sc.particles.copy()
+    with PBFSolver(sc.n, cfg, corr, options=ak.OPT_EXACT_MATH, table_size=table) as s:
+        s.set_search_shape(*shape)
+        s.step_host(p, sc.dt, sc.box_min, sc.box_max)
+        ge = {"order": s.read_debug(ak.DEBUG_ORDER), "cnt": s.read_debug(ak.DEBUG_NEIGHBOUR_COUNTS),
+              "nbr": s.read_debug(ak.DEBUG_NEIGHBOURS)}
+    assert_grid_equal(ge, oe, cfg.maxNeighbours)
+    assert_records_bitexact(p, o)
