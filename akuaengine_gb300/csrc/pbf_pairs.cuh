@@ -28,6 +28,21 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// Differences and products with one operand shared, written as two scalar operations: gathered
+// components lie in different registers of their records, and moving them together for a packed
+// operation costs more instructions than it saves.
+__device__ __forceinline__ float2 diff2(float a, float b, float c) {  // (a - b, a - c)
+    return make_float2(a - b, a - c);
+}
+__device__ __forceinline__ float2 rdiff2(float b, float c, float a) {  // (b - a, c - a)
+    return make_float2(b - a, c - a);
+}
+__device__ __forceinline__ float2 scale2(float a, float b, float c) {  // (a b, a c)
+    return make_float2(a * b, a * c);
+}
+__device__ __forceinline__ float2 plus2(float a, float b, float c) {  // (a + b, a + c)
+    return make_float2(a + b, a + c);
+}
 // dot3 of each lane (same contraction as the scalar dot3)
 __device__ __forceinline__ float2 len2_2(float2 x, float2 y, float2 z) {
     return fma2(z, z, fma2(x, x, mul2(y, y)));
@@ -40,6 +55,14 @@ __device__ __forceinline__ float2 poly6_2(const StepParams& p, float2 r2) {
     const float2 w = mul2(f2(p.kp), mul2(mul2(d, d), d));
     if (IN_REACH) return w;
     return make_float2(r2.x > p.h2 ? 0.0f : w.x, r2.y > p.h2 ? 0.0f : w.y);
+}
+
+// 1 / sqrt(x).  Subnormal arguments, which rsqrtf would scale first, only occur below the distance at
+// which spiky2 drops the result.
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
 // Spiky gradient coefficient c with grad W = c * r (per lane).
@@ -56,7 +79,7 @@ __device__ __forceinline__ void spiky2(const StepParams& p, float2 sx, float2 sy
         gy = make_float2(zx ? 0.f : __fdiv_rn(ay.x, rx), zy ? 0.f : __fdiv_rn(ay.y, ry));
         gz = make_float2(zx ? 0.f : __fdiv_rn(az.x, rx), zy ? 0.f : __fdiv_rn(az.y, ry));
     } else {
-        const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+        const float2 ir = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
         const float2 r = mul2(r2, ir);
         const float2 q = sub2(f2(p.h), r);
         float2 c = mul2(mul2(f2(p.ks), mul2(q, q)), ir);
@@ -68,21 +91,49 @@ __device__ __forceinline__ void spiky2(const StepParams& p, float2 sx, float2 sy
     }
 }
 
-// Calls f(j0, j1, two) for consecutive neighbour pairs of one particle in list order; `two` is
-// false only for a trailing single entry, in which case j1 == j0 and must not be accumulated.
-// The next tile of indices is loaded while the current one is processed.
-template <class F>
-__device__ __forceinline__ void for_each_pair(const uint4* __restrict__ col, int n, int c, F&& f) {
+// One tile of four list entries.  A pass reads each list once, so the tile takes no room in the L1
+// that its gathers live on (1M particles: density 69.2 -> 65.8 us, delta 68.4 -> 65.1, XSPH 101 ->
+// 98).
+__device__ __forceinline__ uint4 ld_tile(const uint4* p) {
+    uint4 t;
+    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+        : "=r"(t.x), "=r"(t.y), "=r"(t.z), "=r"(t.w)
+        : "l"(p));
+    return t;
+}
+
+// Calls f(load(j0), load(j1), two) for consecutive neighbour pairs of one particle in list order;
+// `two` is false only for a trailing single entry, in which case j1 == j0 and must not be
+// accumulated.  The next tile of indices is loaded while the current one is processed.  With
+// WHOLE_TILE all four records of a tile are loaded before the first pair is processed: fewer
+// latencies in a row, more registers.  It pays in the density pass (65.8 -> 63.5 us at 1M) and in
+// scenes that do not fill the chip (step of 60,000 particles 188 -> 182 us) and not where the
+// records are wide or the registers short (vorticity 103 -> 107 us, confinement 76 -> 78).
+template <bool WHOLE_TILE, class L, class F>
+__device__ __forceinline__ void for_each_pair(const uint4* __restrict__ col, int n, int c, L&& load,
+                                              F&& f) {
     const int ng = (c + 3) >> 2;
     if (ng == 0) return;
-    uint4 cur = __ldg(col);
+    uint4 cur = ld_tile(col);
     for (int g = 0; g < ng; ++g) {
-        uint4 nxt = make_uint4(0u, 0u, 0u, 0u);
-        if (g + 1 < ng) nxt = __ldg(col + (size_t)(g + 1) * n);
         const int left = c - 4 * g;
-        f(cur.x, left >= 2 ? cur.y : cur.x, left >= 2);
-        if (left > 2) f(cur.z, left >= 4 ? cur.w : cur.z, left >= 4);
-        cur = nxt;
+        if (WHOLE_TILE) {
+            const auto r0 = load(cur.x), r1 = load(left >= 2 ? cur.y : cur.x);
+            auto r2 = r0, r3 = r0;
+            if (left > 2) {
+                r2 = load(cur.z);
+                r3 = load(left >= 4 ? cur.w : cur.z);
+            }
+            if (g + 1 < ng) cur = ld_tile(col + (size_t)(g + 1) * n);
+            f(r0, r1, left >= 2);
+            if (left > 2) f(r2, r3, left >= 4);
+        } else {
+            uint4 nxt = cur;
+            if (g + 1 < ng) nxt = ld_tile(col + (size_t)(g + 1) * n);
+            f(load(cur.x), load(left >= 2 ? cur.y : cur.x), left >= 2);
+            if (left > 2) f(load(cur.z), load(left >= 4 ? cur.w : cur.z), left >= 4);
+            cur = nxt;
+        }
     }
 }
 
@@ -111,14 +162,14 @@ struct DensityLambda2 {
     template <bool IN_REACH = false>
     __device__ __forceinline__ void add2(const StepParams& p, float4 xi, float4 a, float4 b,
                                          bool two) {
-        const float2 sx = sub2(f2(xi.x), make_float2(a.x, b.x));
-        const float2 sy = sub2(f2(xi.y), make_float2(a.y, b.y));
-        const float2 sz = sub2(f2(xi.z), make_float2(a.z, b.z));
+        const float2 sx = diff2(xi.x, a.x, b.x);
+        const float2 sy = diff2(xi.y, a.y, b.y);
+        const float2 sz = diff2(xi.z, a.z, b.z);
         const float2 r2 = len2_2(sx, sy, sz);
         const float2 w = poly6_2<IN_REACH>(p, r2);
         float2 ux, uy, uz;
         spiky2<EXACT, IN_REACH>(p, sx, sy, sz, r2, ux, uy, uz);
-        const float2 s = mul2(f2(-p.inv_rho0), make_float2(a.w, b.w));
+        const float2 s = scale2(-p.inv_rho0, a.w, b.w);
         const float2 l = len2_2(mul2(s, ux), mul2(s, uy), mul2(s, uz));
         rho = __fmaf_rn(a.w, w.x, rho);
         gx = __fmaf_rn(a.w, ux.x, gx);
@@ -155,9 +206,9 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const float4 xi = ps[i];
     DensityLambda2<EXACT> acc;
     acc.init(xi.w, p);
-    for_each_pair(nbr4 + i, n, (int)cnt[i], [&](uint32_t j0, uint32_t j1, bool two) {
-        acc.add2(p, xi, __ldg(ps + j0), __ldg(ps + j1), two);
-    });
+    for_each_pair<true>(
+        nbr4 + i, n, (int)cnt[i], [&](uint32_t j) { return __ldg(ps + j); },
+        [&](float4 a, float4 b, bool two) { acc.add2(p, xi, a, b, two); });
     rho_out[i] = acc.rho;
     const float l = acc.lambda(p);
     lam_out[i] = l;
@@ -166,14 +217,14 @@ __global__ void __launch_bounds__(kMaxPairBlock)
 }
 
 // (W(r2) / W(dq^2))^n of two pairs: the power in s_corr = -k * (...)^n (ConstraintSolverCUDA.cu:124).
-template <bool EXACT>
+template <bool EXACT, bool FOUR>
 __device__ __forceinline__ float2 scorr_pow2(const StepParams& p, float2 r2) {
     const float2 w = poly6_2(p, r2);
     float2 ratio;
     if (EXACT) ratio = make_float2(__fdiv_rn(w.x, p.wdq), __fdiv_rn(w.y, p.wdq));
     else ratio = mul2(w, f2(p.inv_wdq));
     float2 pw;
-    if (p.corr_n_int == 4) {
+    if (FOUR || p.corr_n_int == 4) {
         const float2 q = mul2(ratio, ratio);
         pw = mul2(q, q);
     } else if (p.corr_n_int >= 0) {
@@ -184,6 +235,12 @@ __device__ __forceinline__ float2 scorr_pow2(const StepParams& p, float2 r2) {
     return pw;
 }
 
+// A particle's position and mass with one more value of it.
+struct Rec5 {
+    float4 x;
+    float l;
+};
+
 // Position delta with artificial pressure (ConstraintSolverCUDA.cu:99-130).
 template <bool EXACT>
 __device__ __forceinline__ float3 position_delta(const StepParams& p, int n, float4 xi, float li,
@@ -191,17 +248,18 @@ __device__ __forceinline__ float3 position_delta(const StepParams& p, int n, flo
                                                  const float* __restrict__ lam,
                                                  const uint4* __restrict__ col, int c) {
     float dx = 0.f, dy = 0.f, dz = 0.f;
-    for_each_pair(col, n, c, [&](uint32_t j0, uint32_t j1, bool two) {
-        const float4 a = __ldg(ps + j0), b = __ldg(ps + j1);
-        const float2 lj = make_float2(__ldg(lam + j0), __ldg(lam + j1));
-        const float2 sx = sub2(f2(xi.x), make_float2(a.x, b.x));
-        const float2 sy = sub2(f2(xi.y), make_float2(a.y, b.y));
-        const float2 sz = sub2(f2(xi.z), make_float2(a.z, b.z));
+    auto load = [&](uint32_t j) { return Rec5{__ldg(ps + j), __ldg(lam + j)}; };
+    for_each_pair<false>(col, n, c, load, [&](const Rec5& ra, const Rec5& rb, bool two) {
+        const float4 a = ra.x, b = rb.x;
+        const float2 lj = make_float2(ra.l, rb.l);
+        const float2 sx = diff2(xi.x, a.x, b.x);
+        const float2 sy = diff2(xi.y, a.y, b.y);
+        const float2 sz = diff2(xi.z, a.z, b.z);
         const float2 r2 = len2_2(sx, sy, sz);
         // (lambda_i + lambda_j + s_corr) * m_j with s_corr = -k * pw: the product feeds the sum
         // and is contracted into it, as the CUDA compiler does with the reference's expression
         // (ConstraintSolverCUDA.cu:124-126).
-        const float2 pw = scorr_pow2<EXACT>(p, r2);
+        const float2 pw = scorr_pow2<EXACT, false>(p, r2);
         const float2 bb = mul2(fma2(f2(p.neg_k), pw, add2(f2(li), lj)), make_float2(a.w, b.w));
         float2 gx, gy, gz;
         spiky2<EXACT>(p, sx, sy, sz, r2, gx, gy, gz);
@@ -219,19 +277,21 @@ __device__ __forceinline__ float3 position_delta(const StepParams& p, int n, flo
 
 // The same sum when every particle has mass `m`: positions and lambdas come from one 16-byte
 // gather of psl[j] = (x*_j, lambda_j), and (lambda_i + lambda_j + s_corr) * m is the same product.
-template <bool EXACT>
+// FOUR: the power is 4 (the reference's), known before the loop: without the per-pair branch to
+// powf the parameters stay in registers (1M particles: 75.1 -> 69.9 us).
+template <bool EXACT, bool FOUR>
 __device__ __forceinline__ float3 position_delta_uniform(const StepParams& p, int n, float4 xl,
                                                          const float4* __restrict__ psl, float m,
                                                          const uint4* __restrict__ col, int c) {
     float dx = 0.f, dy = 0.f, dz = 0.f;
-    for_each_pair(col, n, c, [&](uint32_t j0, uint32_t j1, bool two) {
-        const float4 a = __ldg(psl + j0), b = __ldg(psl + j1);
-        const float2 sx = sub2(f2(xl.x), make_float2(a.x, b.x));
-        const float2 sy = sub2(f2(xl.y), make_float2(a.y, b.y));
-        const float2 sz = sub2(f2(xl.z), make_float2(a.z, b.z));
+    auto load = [&](uint32_t j) { return __ldg(psl + j); };
+    for_each_pair<true>(col, n, c, load, [&](float4 a, float4 b, bool two) {
+        const float2 sx = diff2(xl.x, a.x, b.x);
+        const float2 sy = diff2(xl.y, a.y, b.y);
+        const float2 sz = diff2(xl.z, a.z, b.z);
         const float2 r2 = len2_2(sx, sy, sz);
-        const float2 pw = scorr_pow2<EXACT>(p, r2);
-        const float2 bb = mul2(fma2(f2(p.neg_k), pw, add2(f2(xl.w), make_float2(a.w, b.w))), f2(m));
+        const float2 pw = scorr_pow2<EXACT, FOUR>(p, r2);
+        const float2 bb = mul2(fma2(f2(p.neg_k), pw, plus2(xl.w, a.w, b.w)), f2(m));
         float2 gx, gy, gz;
         spiky2<EXACT>(p, sx, sy, sz, r2, gx, gy, gz);
         dx = __fmaf_rn(bb.x, gx.x, dx);
@@ -255,9 +315,12 @@ __device__ __forceinline__ float3 delta_of(const StepParams& p, int i, float4 xi
                                            const float4* __restrict__ psl,
                                            const uint32_t* __restrict__ mass_bits,
                                            const uint4* __restrict__ nbr4, int c) {
-    if (__ldg(mass_bits) == 0u)
-        return position_delta_uniform<EXACT>(p, p.n, psl[i], psl, __uint_as_float(__ldg(mass_bits + 1)),
-                                             nbr4 + i, c);
+    if (__ldg(mass_bits) == 0u) {
+        const float m = __uint_as_float(__ldg(mass_bits + 1));
+        return p.corr_n_int == 4
+                   ? position_delta_uniform<EXACT, true>(p, p.n, psl[i], psl, m, nbr4 + i, c)
+                   : position_delta_uniform<EXACT, false>(p, p.n, psl[i], psl, m, nbr4 + i, c);
+    }
     return position_delta<EXACT>(p, p.n, xi, lam[i], ps_in, lam, nbr4 + i, c);
 }
 
@@ -405,17 +468,17 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     if (i >= n) return;
     const float4 xi = x4[i], vi = v4[i];
     float wx = 0.f, wy = 0.f, wz = 0.f;
-    for_each_pair(nbr4 + i, n, (int)cnt[i], [&](uint32_t j0, uint32_t j1, bool two) {
-        const Rec8 ra = ld_rec8(xv8, j0), rb = ld_rec8(xv8, j1);
+    auto load = [&](uint32_t j) { return ld_rec8(xv8, j); };
+    auto term = [&](const Rec8& ra, const Rec8& rb, bool two) {
         const float4 a = ra.x, b = rb.x, va = ra.v, vb = rb.v;
-        const float2 sx = sub2(f2(xi.x), make_float2(a.x, b.x));
-        const float2 sy = sub2(f2(xi.y), make_float2(a.y, b.y));
-        const float2 sz = sub2(f2(xi.z), make_float2(a.z, b.z));
+        const float2 sx = diff2(xi.x, a.x, b.x);
+        const float2 sy = diff2(xi.y, a.y, b.y);
+        const float2 sz = diff2(xi.z, a.z, b.z);
         float2 gx, gy, gz;
         spiky2<EXACT>(p, sx, sy, sz, len2_2(sx, sy, sz), gx, gy, gz);
-        const float2 ux = sub2(make_float2(va.x, vb.x), f2(vi.x));
-        const float2 uy = sub2(make_float2(va.y, vb.y), f2(vi.y));
-        const float2 uz = sub2(make_float2(va.z, vb.z), f2(vi.z));
+        const float2 ux = rdiff2(va.x, vb.x, vi.x);
+        const float2 uy = rdiff2(va.y, vb.y, vi.y);
+        const float2 uz = rdiff2(va.z, vb.z, vi.z);
         // cross(u, g) contracted as fma(u.y, g.z, -(u.z * g.y)), ...
         const float2 cx = fma2(uy, gz, mul2(f2(-1.0f), mul2(uz, gy)));
         const float2 cy = fma2(uz, gx, mul2(f2(-1.0f), mul2(ux, gz)));
@@ -428,7 +491,8 @@ __global__ void __launch_bounds__(kMaxPairBlock)
             wy = __fmaf_rn(-b.w, cy.y, wy);
             wz = __fmaf_rn(-b.w, cz.y, wz);
         }
-    });
+    };
+    for_each_pair<EXACT>(nbr4 + i, n, (int)cnt[i], load, term);
     const float wn = __fsqrt_rn(len2(wx, wy, wz));
     om4[i] = make_float4(wx, wy, wz, wn);
     xw4[i] = make_float4(xi.x, xi.y, xi.z, wn);  // (x, |omega|) for confinement's single gather
@@ -455,9 +519,9 @@ __global__ void __launch_bounds__(kMaxPairBlock, 5)
     float ex = 0.f, ey = 0.f, ez = 0.f;
     // pair term m_j (|omega_i| - |omega_j|) grad W, given positions, masses and |omega_j|
     auto term = [&](float4 a, float4 b, float2 mj, float2 wj, bool two) {
-        const float2 sx = sub2(f2(xi.x), make_float2(a.x, b.x));
-        const float2 sy = sub2(f2(xi.y), make_float2(a.y, b.y));
-        const float2 sz = sub2(f2(xi.z), make_float2(a.z, b.z));
+        const float2 sx = diff2(xi.x, a.x, b.x);
+        const float2 sy = diff2(xi.y, a.y, b.y);
+        const float2 sz = diff2(xi.z, a.z, b.z);
         float2 gx, gy, gz;
         spiky2<EXACT>(p, sx, sy, sz, len2_2(sx, sy, sz), gx, gy, gz);
         const float2 s = mul2(mj, sub2(f2(wi.w), wj));
@@ -472,15 +536,14 @@ __global__ void __launch_bounds__(kMaxPairBlock, 5)
     };
     if (__ldg(mass_bits) == 0u) {  // one mass: (x, |omega|) in one gather, the same products
         const float m = __uint_as_float(__ldg(mass_bits + 1));
-        for_each_pair(nbr4 + i, n, (int)cnt[i], [&](uint32_t j0, uint32_t j1, bool two) {
-            const float4 a = __ldg(xw4 + j0), b = __ldg(xw4 + j1);
+        auto load = [&](uint32_t j) { return __ldg(xw4 + j); };
+        for_each_pair<false>(nbr4 + i, n, (int)cnt[i], load, [&](float4 a, float4 b, bool two) {
             term(a, b, f2(m), make_float2(a.w, b.w), two);
         });
     } else {
-        for_each_pair(nbr4 + i, n, (int)cnt[i], [&](uint32_t j0, uint32_t j1, bool two) {
-            const float4 a = __ldg(x4 + j0), b = __ldg(x4 + j1);
-            term(a, b, make_float2(a.w, b.w),
-                 make_float2(__ldg(&om4[j0].w), __ldg(&om4[j1].w)), two);
+        auto load = [&](uint32_t j) { return Rec5{__ldg(x4 + j), __ldg(&om4[j].w)}; };
+        for_each_pair<false>(nbr4 + i, n, (int)cnt[i], load, [&](const Rec5& a, const Rec5& b, bool two) {
+            term(a.x, b.x, make_float2(a.x.w, b.x.w), make_float2(a.l, b.l), two);
         });
     }
     const float inv_d = __fdiv_rn(1.0f, rho_i);
@@ -526,17 +589,17 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const Rec8 ri = ld_rec8(xv8, (uint32_t)i);
     const float4 xi = ri.x, vi = ri.v;
     float ax = 0.f, ay = 0.f, az = 0.f;
-    for_each_pair(nbr4 + i, n, (int)cnt[i], [&](uint32_t j0, uint32_t j1, bool two) {
-        const Rec8 ra = ld_rec8(xv8, j0), rb = ld_rec8(xv8, j1);
+    auto load = [&](uint32_t j) { return ld_rec8(xv8, j); };
+    for_each_pair<true>(nbr4 + i, n, (int)cnt[i], load, [&](const Rec8& ra, const Rec8& rb, bool two) {
         const float4 a = ra.x, b = rb.x, va = ra.v, vb = rb.v;
-        const float2 sx = sub2(f2(xi.x), make_float2(a.x, b.x));
-        const float2 sy = sub2(f2(xi.y), make_float2(a.y, b.y));
-        const float2 sz = sub2(f2(xi.z), make_float2(a.z, b.z));
+        const float2 sx = diff2(xi.x, a.x, b.x);
+        const float2 sy = diff2(xi.y, a.y, b.y);
+        const float2 sz = diff2(xi.z, a.z, b.z);
         const float2 w = poly6_2(p, len2_2(sx, sy, sz));
         const float2 s = make_float2(a.w, b.w);  // m_j / rho_j
-        const float2 tx = mul2(s, sub2(make_float2(va.x, vb.x), f2(vi.x)));
-        const float2 ty = mul2(s, sub2(make_float2(va.y, vb.y), f2(vi.y)));
-        const float2 tz = mul2(s, sub2(make_float2(va.z, vb.z), f2(vi.z)));
+        const float2 tx = mul2(s, rdiff2(va.x, vb.x, vi.x));
+        const float2 ty = mul2(s, rdiff2(va.y, vb.y, vi.y));
+        const float2 tz = mul2(s, rdiff2(va.z, vb.z, vi.z));
         ax = __fmaf_rn(tx.x, w.x, ax);
         ay = __fmaf_rn(ty.x, w.x, ay);
         az = __fmaf_rn(tz.x, w.x, az);
