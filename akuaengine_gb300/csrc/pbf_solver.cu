@@ -462,9 +462,14 @@ void invalidate_graph(akua_pbf* s) {
 }
 
 void update_plans(akua_pbf* s, int sp_bits) {
-    s->plan_ref = akua::radix::make_plan(akua::radix::bits_for(s->table_size));
+    // one scene of few particles: a pass is one cluster; a batch holds many scenes' particles
+    const bool small = s->scenes.empty() && s->n <= akua::radix::kClusterMax;
+    auto plan = [&](int bits) {
+        return small ? akua::radix::make_cluster_plan(bits) : akua::radix::make_plan(bits);
+    };
+    s->plan_ref = plan(akua::radix::bits_for(s->table_size));
     s->sp_bits = sp_bits;
-    s->plan_sp = akua::radix::make_plan(3 * sp_bits + s->scene_bits);
+    s->plan_sp = plan(3 * sp_bits + s->scene_bits);
 }
 
 int ensure_graph(akua_pbf* s, const char* aos, size_t stride) {

@@ -97,11 +97,15 @@ extern "C" int akua_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* 
     uint32_t* tmp_vals = scratch + kMaxPairs;
     uint32_t* counts = scratch + 2 * (size_t)kMaxPairs;
     uint32_t* totals = counts + (size_t)akua::radix::MAX_RADIX * akua::radix::num_tiles(n);
-    // the digit totals accumulate atomically and must start at zero on every call
-    e = cudaMemsetAsync(totals, 0,
-                        sizeof(uint32_t) * akua::radix::MAX_PASSES * akua::radix::MAX_RADIX, st);
-    if (e != cudaSuccess) return AKUA_ERR_CUDA;
-    const akua::radix::Plan plan = akua::radix::make_plan(key_bits);
+    const akua::radix::Plan plan = n <= akua::radix::kClusterMax
+                                       ? akua::radix::make_cluster_plan(key_bits)
+                                       : akua::radix::make_plan(key_bits);
+    if (!plan.cluster) {
+        // the digit totals accumulate atomically and must start at zero on every call
+        e = cudaMemsetAsync(totals, 0,
+                            sizeof(uint32_t) * akua::radix::MAX_PASSES * akua::radix::MAX_RADIX, st);
+        if (e != cudaSuccess) return AKUA_ERR_CUDA;
+    }
     NoMark mark;
     // pass p writes to the caller's output when (passes - 1 - p) is even, so the last pass does
     const uint32_t* kin = keys_in;
@@ -114,7 +118,10 @@ extern "C" int akua_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* 
         // the digit covers only this pass's bits, so key bits at and above key_bits never
         // influence the order (a pass narrower than 8 bits still runs the 8-bit kernels)
         const uint32_t mask = (1u << plan.width[p]) - 1u;
-        if (plan.width[p] <= 8)
+        if (plan.cluster)
+            akua::radix::run_cluster_pass<false>(st, kin, vin, kout, vout, n, plan.shift[p], plan.width[p],
+                                          nullptr, mark);
+        else if (plan.width[p] <= 8)
             akua::radix::run_pass<8>(st, kin, vin, kout, vout, counts, tot, n, plan.shift[p],
                                       nullptr, mark, mask);
         else if (plan.width[p] == 9)

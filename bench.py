@@ -54,6 +54,7 @@ KERNEL_BYTES = {
     "k_keys": lambda L, B: 16 + 16 + 4 + 16,
     "radix_upsweep": lambda L, B: 4,                  # R key (per pass)
     "radix_downsweep": lambda L, B: 16,               # R key, value; W key, value (per pass)
+    "radix_cluster_pass": lambda L, B: 16,            # the same, histogram and scan included
     # R two permutations, x|m, v, colour, size, old rank; W x|m, colour, size, x*|m, rank->slot,
     # slot->rank, order
     "k_gather": lambda L, B: 8 + 16 + 16 + 16 + 4 + 4 + 16 + 16 + 4 + 16 + 4 + 4 + 4,
