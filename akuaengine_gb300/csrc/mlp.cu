@@ -43,9 +43,9 @@ int launch_grad(akua_mlp* m, const float* feat, const float* target, int32_t n, 
         attr_set[m->device] = true;
     }
     const int tiles = (n + akua::mlp::kTile - 1) / akua::mlp::kTile;
-    const int grid = std::max(1, std::min(tiles, m->sms));  // one CTA per SM (all of TMEM)
-    akua::mlp::k_mlp_grad<<<grid, akua::mlp::kThreads, akua::mlp::kGradSmem, st>>>(
-        m->params, m->norm, feat, target, n, 1.0f / (float)n, m->grad, m->err);
+    const int grid = std::max(1, std::min(tiles, m->sms));  // one CTA of 16 warps per SM
+    akua::mlp::k_mlp_grad<<<grid, akua::mlp::kGradThreads, akua::mlp::kGradSmem, st>>>(
+        m->params, m->image, m->norm, feat, target, n, 1.0f / (float)n, m->grad, m->err);
     return status_of(cudaGetLastError());
 }
 
@@ -200,14 +200,9 @@ int akua_mlp_adam_step(akua_mlp* m, const float* features, const float* targets,
     const float bc1 = (float)(1.0 - std::pow((double)b1, (double)m->adam_steps));
     const float bc2 = (float)(1.0 - std::pow((double)b2, (double)m->adam_steps));
     const int blocks = (akua::mlp::kParams + 1 + 255) / 256;
-    akua::mlp::k_mlp_adam<<<blocks, 256, 0, st>>>(m->params, m->grad, m->m, m->v, learningRate,
-                                                 b1, b2, 1e-8f, bc1, bc2);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) {  // the forward pass reads the updated weights from their image
-        akua::mlp::k_mlp_image<<<1, akua::mlp::kThreads, 0, st>>>(m->params, m->image);
-        e = cudaGetLastError();
-    }
-    return status_of(e);
+    akua::mlp::k_mlp_adam<<<blocks, 256, 0, st>>>(m->params, m->grad, m->m, m->v, m->image,
+                                                 learningRate, b1, b2, 1e-8f, bc1, bc2);
+    return status_of(cudaGetLastError());
 }
 
 int akua_mlp_synchronize(akua_mlp* m, void* stream) {

@@ -12,13 +12,13 @@
 //   dy = 2 (y - t') / n;  dz3 = bf16(dy w4 silu'(z3));  dz2 = bf16((dz3 W3) silu'(z2));
 //   dz1 = bf16((dz2 W2) silu'(z1));  dW_l = dz_l^T a_{l-1};  db_l = sum dz_l;  dw4 = sum dy a3
 //
-// One CTA of 128 threads per tile of 128 samples (thread t owns sample row t, TMEM lane t).  The
-// forward kernel keeps one 64-column accumulator; the gradient kernel keeps z1..z3, the input
-// gradient and the three weight-gradient accumulators in tensor memory (432 of 512 columns) and
-// accumulates the weight gradients over all tiles it processes before one atomic flush.
-// Weight gradients are MMAs over the batch: dW^T-shaped D[out][in] = A[out][b] B[in][b] with
-// A = dz^T (64 rows, padded to M = 128 with zeros) and B = a^T plus one row of ones, whose column
-// of D is the bias gradient.
+// The forward kernel: one CTA of 128 threads per tile of 128 samples (thread t owns sample row t,
+// TMEM lane t) and one 64-column accumulator.  The gradient kernel: 512 threads per tile, one
+// 64-column accumulator for z and the input gradients in turn and three for the weight gradients,
+// which it accumulates over all tiles it processes before one flush.  Weight gradients are MMAs over
+// the batch, D[out][in] = dz[b][out] a[b][in], with a column of ones beside the activations whose
+// column of D is the bias gradient (64 output features in an M = 128 MMA: the other rows are not
+// read).
 #pragma once
 
 #include <cstddef>
@@ -104,40 +104,27 @@ __device__ __forceinline__ void store_row64(uint8_t* tile, int row, const float*
                    pack_bf16(v[14], v[15]));
 }
 
-// Column `col` of a transposed K-major tile with K = 128 (rows = features, k = sample): 16 values
-// for feature rows r0 .. r0+15 of sample `col`.
-__device__ __forceinline__ void store_col128(uint8_t* tile, int col, const float* v, int r0) {
-#pragma unroll
-    for (int q = 0; q < 16; ++q)
-        *reinterpret_cast<uint16_t*>(tile + tc::kmajor_offset(r0 + q, col, 128)) = bf16_bits(v[q]);
-}
-
-// Stages a [64][K] weight (row-major FP32 [64][kin]) as a BF16 K-major B operand with K = kpad
-// columns (zeros beyond kin); `transposed` stages W^T ([in][out]) instead.
+// Stages a [64][kin] weight (row-major FP32) as a BF16 K-major B operand with K = kpad columns (zeros
+// beyond kin).
 __device__ __forceinline__ void stage_weight(uint8_t* dst, const float* __restrict__ w, int kin,
-                                             int kpad, bool transposed, int t) {
+                                             int kpad, int t) {
     for (int e = t; e < kHid * kpad; e += kThreads) {
-        const int r = e / kpad, k = e - r * kpad;  // operand row r, column k
-        float v = 0.f;
-        if (!transposed) {
-            if (k < kin) v = w[r * kin + k];  // B[out][in] = W[out][in]
-        } else {
-            v = w[k * kin + r];  // B[in][out] = W[out][in]; kin == kpad == 64
-        }
-        *reinterpret_cast<uint16_t*>(dst + tc::kmajor_offset(r, k, kpad)) = bf16_bits(v);
+        const int r = e / kpad, k = e - r * kpad;
+        *reinterpret_cast<uint16_t*>(dst + tc::kmajor_offset(r, k, kpad)) =
+            bf16_bits(k < kin ? w[r * kin + k] : 0.f);
     }
 }
 
-// BF16 operand images of W1, W2, W3 in the forward pass's shared-memory layout, rebuilt by
-// k_mlp_image whenever the parameters change; a forward CTA copies them instead of converting.
+// BF16 operand images of W1, W2, W3 in the kernels' shared-memory layout, built by k_mlp_image when
+// parameters are set and kept up to date by k_mlp_adam; a CTA copies them instead of converting.
 constexpr int kImageBytes = (kHid * kInPad + 2 * kHid * kHid) * 2;
 
 __global__ void __launch_bounds__(kThreads)
     k_mlp_image(const float* __restrict__ params, uint8_t* __restrict__ image) {
     const int t = threadIdx.x;
-    stage_weight(image, params + kW1, kIn, kInPad, false, t);
-    stage_weight(image + kHid * kInPad * 2, params + kW2, kHid, kHid, false, t);
-    stage_weight(image + kHid * kInPad * 2 + kHid * kHid * 2, params + kW3, kHid, kHid, false, t);
+    stage_weight(image, params + kW1, kIn, kInPad, t);
+    stage_weight(image + kHid * kInPad * 2, params + kW2, kHid, kHid, t);
+    stage_weight(image + kHid * kInPad * 2 + kHid * kHid * 2, params + kW3, kHid, kHid, t);
 }
 
 // ------------------------------------------------------------------------------------ forward
@@ -325,31 +312,40 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // ----------------------------------------------------------------------------------- gradient
-// TMEM columns.
-constexpr uint32_t kColZ1 = 0, kColZ2 = 64, kColZ3 = 128, kColDA = 192;
-constexpr uint32_t kColG3 = 256, kColG2 = 336, kColG1 = 416;  // 80, 80, 16 columns
-constexpr uint32_t kGradCols = 512;
-constexpr int kNT = 80;  // rows of a transposed activation operand: 64 features, ones, zeros
+// One CTA per SM, 16 warps: warp w owns rows 32 (w % 4) .. + 31 of the tile and columns
+// 16 (w / 4) .. + 15 of every layer, so a layer's SiLU is spread over 512 threads.  The weight
+// gradients' operands are the forward tiles read along the other axis; the bias gradients are a
+// column of ones beside the activations.  Per tile five dependent MMAs (z1, z2, z3, da2, da1); the
+// weight-gradient MMAs run behind them while the next epilogue works, which is why dz and x have two
+// buffers: an MMA's operands are overwritten only after a later commit of the same issue order.
+//
+// Bound by the chain of a tile (4 us: five MMAs with their epilogues, 33% of the issue slots) and
+// about 8 us of start and flush.  65,536 samples (512 tiles, four rounds of 152 CTAs): 95 -> 23 us
+// against 4 warps per CTA with transposed copies stored two bytes at a time and dw4 reduced by
+// shuffles in every tile; an Adam step, its two kernels together, 110 -> 29 us.
+constexpr int kGradThreads = 512;
+constexpr int kGradCols = 16;  // columns per thread
+constexpr uint32_t kColW = 0;                                // z1, z2, z3, da2, da1 in turn
+constexpr uint32_t kColG3 = 64, kColG2 = 144, kColG1 = 224;  // 80, 80, 16 columns
+constexpr uint32_t kGradTmem = 256;
+constexpr int kNT = 80;  // columns of an activation tile: 64 features, ones, zeros
+constexpr int kDzBytes = kTile * kHid * 2;
+constexpr int kDzPad = 1024;  // rows 64..127 of the M = 128 operand run on past the tile
 
 struct GradSmem {
-    alignas(128) uint8_t w1[kHid * kInPad * 2];      // B: [out][in16]
-    alignas(128) uint8_t w2[kHid * kHid * 2];        // B: [out][in]
+    alignas(128) uint8_t w1[kHid * kInPad * 2];      // [out][in16], K-major: the image's three
+    alignas(128) uint8_t w2[kHid * kHid * 2];        // [out][in]
     alignas(128) uint8_t w3[kHid * kHid * 2];
-    alignas(128) uint8_t w2t[kHid * kHid * 2];       // B: [in][out]
-    alignas(128) uint8_t w3t[kHid * kHid * 2];
-    alignas(128) uint8_t x[kTile * kInPad * 2];      // A: [b][in16]
-    alignas(128) uint8_t a1[kTile * kHid * 2];       // A: [b][64]
-    alignas(128) uint8_t a2[kTile * kHid * 2];
-    alignas(128) uint8_t xT[kInPad * kTile * 2];     // B: [in16][b]: rows 0-7 x, row 8 ones
-    alignas(128) uint8_t a1T[kNT * kTile * 2];       // B: [80][b]: rows 0-63 a1, row 64 ones
-    alignas(128) uint8_t a2T[kNT * kTile * 2];
-    alignas(128) uint8_t dz[kTile * kHid * 2];       // A: [b][64]
-    alignas(128) uint8_t dzT[kTile * kTile * 2];     // A: [128][b]: rows 0-63 dz, rest zero
+    alignas(128) uint8_t x[2][kTile * kInPad * 2];   // [b][16]: 8 features, ones, zeros
+    alignas(128) uint8_t a1[kTile * kNT * 2];        // [b][80]
+    alignas(128) uint8_t a2[kTile * kNT * 2];
+    alignas(128) uint8_t dz[2][kDzBytes + kDzPad];   // [b][64]
     float b1[kHid], b2[kHid], b3[kHid], w4[kHid];
     float norm[kNorm];
     float b4;
-    float gw4[kHid + 1];  // dw4, db4
-    float loss;
+    float y[4][kTile];     // partial outputs of the four column groups
+    float gw4[4][kHid];    // dw4 of the four row quarters
+    float gb4, loss;
     alignas(8) uint64_t bar;
     uint32_t tmem;
 };
@@ -357,297 +353,292 @@ struct GradSmem {
 constexpr size_t kGradSmem = sizeof(GradSmem);
 
 // Accumulates into grad[kParams] (dL/dparams) and grad[kParams] += loss.  Targets are in output
-// units (lambda); the loss is over `n_total` samples (this call may see a slice of them).
-__global__ void __launch_bounds__(kThreads)
-    k_mlp_grad(const float* __restrict__ params, const float* __restrict__ norm,
-               const float* __restrict__ feat, const float* __restrict__ target, int n,
-               float inv_n_total, float* __restrict__ grad, uint32_t* __restrict__ err) {
+// units (lambda); the loss is over `n_total` samples (this call may see a slice of them).  `image`:
+// the BF16 operand images of W1..W3 (k_mlp_image).
+__global__ void __launch_bounds__(kGradThreads, 1)
+    k_mlp_grad(const float* __restrict__ params, const uint8_t* __restrict__ image,
+               const float* __restrict__ norm, const float* __restrict__ feat,
+               const float* __restrict__ target, int n, float inv_n_total,
+               float* __restrict__ grad, uint32_t* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
+    static_assert(offsetof(GradSmem, w2) == sizeof(S.w1) &&
+                      offsetof(GradSmem, w3) == sizeof(S.w1) + sizeof(S.w2),
+                  "the weight image is w1, w2, w3 back to back");
     const int t = threadIdx.x, warp = t >> 5;
-    stage_weight(S.w1, params + kW1, kIn, kInPad, false, t);
-    stage_weight(S.w2, params + kW2, kHid, kHid, false, t);
-    stage_weight(S.w3, params + kW3, kHid, kHid, false, t);
-    stage_weight(S.w2t, params + kW2, kHid, kHid, true, t);
-    stage_weight(S.w3t, params + kW3, kHid, kHid, true, t);
+    const int row = t & (kTile - 1);  // 32 (warp % 4) + lane
+    const int group = t / kTile;      // warp / 4
+    const int c0 = kGradCols * group;
+    for (int k = t; k < kImageBytes / 16; k += kGradThreads)
+        reinterpret_cast<uint4*>(S.w1)[k] = __ldg(reinterpret_cast<const uint4*>(image) + k);
     if (t < kHid) {
         S.b1[t] = params[kB1 + t];
         S.b2[t] = params[kB2 + t];
         S.b3[t] = params[kB3 + t];
         S.w4[t] = params[kW4 + t];
     }
-    if (t <= kHid) S.gw4[t] = 0.f;
     if (t < kNorm) S.norm[t] = norm[t];
     if (t == 0) {
         S.b4 = params[kB4];
+        S.gb4 = 0.f;
         S.loss = 0.f;
         tc::mbar_init(&S.bar, 1);
     }
-    // constant parts of the operand tiles: input padding, ones rows, zero rows
-    {
-        const uint16_t one = bf16_bits(1.0f);
-        *reinterpret_cast<uint4*>(S.x + tc::kmajor_offset(t, 8, kInPad)) = make_uint4(0, 0, 0, 0);
-        for (int r = kIn; r < kInPad; ++r)
-            *reinterpret_cast<uint16_t*>(S.xT + tc::kmajor_offset(r, t, kTile)) =
-                r == kIn ? one : (uint16_t)0;
-        for (int r = kHid; r < kNT; ++r) {
-            const uint16_t v = r == kHid ? one : (uint16_t)0;
-            *reinterpret_cast<uint16_t*>(S.a1T + tc::kmajor_offset(r, t, kTile)) = v;
-            *reinterpret_cast<uint16_t*>(S.a2T + tc::kmajor_offset(r, t, kTile)) = v;
+    {  // constant columns of the operand tiles: a one and zeros
+        const uint4 ones = make_uint4(pack_bf16(1.0f, 0.0f), 0u, 0u, 0u);
+        const uint4 zeros = make_uint4(0u, 0u, 0u, 0u);
+        if (group < 2) {
+            *reinterpret_cast<uint4*>(S.x[group] + tc::kmajor_offset(row, 8, kInPad)) = ones;
+        } else {
+            uint8_t* a = group == 2 ? S.a1 : S.a2;
+            *reinterpret_cast<uint4*>(a + tc::kmajor_offset(row, kHid, kNT)) = ones;
+            *reinterpret_cast<uint4*>(a + tc::kmajor_offset(row, kHid + 8, kNT)) = zeros;
         }
-        for (int r = kHid; r < kTile; ++r)
-            *reinterpret_cast<uint16_t*>(S.dzT + tc::kmajor_offset(r, t, kTile)) = 0;
     }
-    if (warp == 0) tc::tmem_alloc(&S.tmem, kGradCols);
+    if (warp == 0) tc::tmem_alloc(&S.tmem, kGradTmem);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = S.tmem;
-    const uint32_t lane = tmem + ((uint32_t)(warp * 32) << 16);
-    const uint32_t id64 = tc::idesc_bf16(128, 64);
-    const uint32_t id80 = tc::idesc_bf16(128, kNT);
-    const uint32_t id16 = tc::idesc_bf16(128, 16);
-    const uint32_t sx = tc::smem_addr(S.x), sw1 = tc::smem_addr(S.w1);
+    const uint32_t lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    const uint32_t sx = tc::smem_addr(S.x[0]), sw1 = tc::smem_addr(S.w1);
     const uint32_t sa1 = tc::smem_addr(S.a1), sa2 = tc::smem_addr(S.a2);
     const uint32_t sw2 = tc::smem_addr(S.w2), sw3 = tc::smem_addr(S.w3);
-    const uint32_t sw2t = tc::smem_addr(S.w2t), sw3t = tc::smem_addr(S.w3t);
-    const uint32_t sxT = tc::smem_addr(S.xT), sa1T = tc::smem_addr(S.a1T);
-    const uint32_t sa2T = tc::smem_addr(S.a2T), sdz = tc::smem_addr(S.dz);
-    const uint32_t sdzT = tc::smem_addr(S.dzT);
+    const uint32_t sdz = tc::smem_addr(S.dz[0]);
+    constexpr uint32_t kXBytes = kTile * kInPad * 2, kDz = kDzBytes + kDzPad;
     const float inv_scale = 1.0f / S.norm[2 * kIn];
     uint32_t phase = 0;
-    uint32_t acc = 0;  // weight-gradient accumulators hold data
+    uint32_t acc = 0;  // the weight-gradient accumulators hold data
     bool ok = true;
 
-    // issue helpers (thread 0 only)
-    auto gemm_k64 = [&](uint32_t d, uint32_t a, uint32_t b) {  // D = A[128][64] B[64][64]^T
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-            tc::mma_bf16(d, tc::smem_desc(a + 256 * s, 128, kHid * 16),
-                         tc::smem_desc(b + 256 * s, 128, kHid * 16), id64, s > 0);
+    // issue helpers (thread 0 only); every operand's 8-row groups are `sbo` bytes apart
+    auto forward = [&](uint32_t a, uint32_t a_sbo, uint32_t b, int ksteps, uint32_t b_sbo) {
+        constexpr uint32_t id = tc::idesc_bf16(kTile, kHid);
+        for (int s = 0; s < ksteps; ++s)  // W = A B^T
+            tc::mma_bf16(tmem + kColW, tc::smem_desc(a + 256 * s, 128, a_sbo),
+                         tc::smem_desc(b + 256 * s, 128, b_sbo), id, s > 0);
+        tc::mma_commit(&S.bar);
     };
-    auto gemm_batch = [&](uint32_t d, uint32_t b, uint32_t idesc) {  // D += dzT[128][b] B[N][b]^T
+    auto backward = [&](uint32_t dz, uint32_t w) {  // W[b][in] = dz[b][out] w[out][in]
+        constexpr uint32_t id = tc::idesc_bf16(kTile, kHid) | tc::kTransposeB;
+#pragma unroll
+        for (int s = 0; s < kHid / 16; ++s)
+            tc::mma_bf16(tmem + kColW, tc::smem_desc(dz + 256 * s, 128, kHid * 16),
+                         tc::smem_desc(w + 2 * kHid * 16 * s, kHid * 16, 128), id, s > 0);
+        tc::mma_commit(&S.bar);
+    };
+    // G[out][in] += dz[b][out] act[b][in], `cols` columns of the activation tile
+    auto weights = [&](uint32_t g, uint32_t dz, uint32_t act, uint32_t cols) {
+        const uint32_t id = tc::idesc_bf16(kTile, cols) | tc::kTransposeA | tc::kTransposeB;
 #pragma unroll
         for (int s = 0; s < kTile / 16; ++s)
-            tc::mma_bf16(d, tc::smem_desc(sdzT + 256 * s, 128, kTile * 16),
-                         tc::smem_desc(b + 256 * s, 128, kTile * 16), idesc, (acc | s) != 0);
+            tc::mma_bf16(tmem + g, tc::smem_desc(dz + 2 * kHid * 16 * s, kHid * 16, 128),
+                         tc::smem_desc(act + 2 * cols * 16 * s, cols * 16, 128), id, (acc | s) != 0);
     };
-    auto sync_issue = [&]() {
+    auto publish = [&]() {  // this thread's operand stores and tensor-memory reads are done
         tc::fence_async_smem();
         tc::fence_before_sync();
         __syncthreads();
+        if (t == 0) tc::fence_after_sync();
     };
+    // After a wait that ran out nothing waits again; the next tile's check ends the kernel.
     auto wait = [&]() {
-        ok = __syncthreads_and(tc::mbar_wait(&S.bar, phase));
+        if (ok) ok = tc::mbar_wait(&S.bar, phase);
         phase ^= 1;
         tc::fence_after_sync();
-        return ok;
+    };
+    auto put_x = [&](int buf, const float (&f)[kIn]) {  // row t of the tile, threads 0..127
+        float v[kIn];
+#pragma unroll
+        for (int k = 0; k < kIn; ++k) v[k] = (f[k] - S.norm[k]) * S.norm[kIn + k];
+        *reinterpret_cast<uint4*>(S.x[buf] + tc::kmajor_offset(t, 0, kInPad)) =
+            make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
+                       pack_bf16(v[6], v[7]));
+    };
+    auto put16 = [&](uint8_t* tile, int cols, const float (&v)[kGradCols]) {
+        *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(row, c0, cols)) =
+            make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
+                       pack_bf16(v[6], v[7]));
+        *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(row, c0 + 8, cols)) =
+            make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]),
+                       pack_bf16(v[14], v[15]));
+    };
+    // a = silu(z + b) to the activation tile, silu'(z + b) kept
+    auto hidden = [&](const float* bias, uint8_t* tile, float (&d)[kGradCols]) {
+        float v[kGradCols];
+        tc::tmem_ld16(lane + kColW + c0, v);
+#pragma unroll
+        for (int q = 0; q < kGradCols; ++q) {
+            const float z = v[q] + bias[c0 + q];
+            v[q] = silu(z);
+            d[q] = dsilu(z);
+        }
+        put16(tile, kNT, v);
     };
 
     const int tiles = (n + kTile - 1) / kTile;
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const int i = tile * kTile + t;
+    float f[kIn], gw4[kGradCols], gb4 = 0.f, loss = 0.f;
+#pragma unroll
+    for (int q = 0; q < kGradCols; ++q) gw4[q] = 0.f;
+    int buf = 0;
+    if (t < kTile) {
+        load_features(feat, blockIdx.x * kTile + t, n, S.norm, f);
+        put_x(0, f);
+    }
+    publish();
+    if (t == 0) forward(sx, kInPad * 16, sw1, 1, kInPad * 16);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int i = tile * kTile + row;
         const bool valid = i < n;
-        float f[kIn];
-        if (valid) {
-            const float4 a = reinterpret_cast<const float4*>(feat)[2 * (size_t)i];
-            const float4 b = reinterpret_cast<const float4*>(feat)[2 * (size_t)i + 1];
-            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
-            f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-        } else {
-#pragma unroll
-            for (int k = 0; k < kIn; ++k) f[k] = S.norm[k];
-        }
-#pragma unroll
-        for (int k = 0; k < kIn; ++k) f[k] = (f[k] - S.norm[k]) * S.norm[kIn + k];
-        *reinterpret_cast<uint4*>(S.x + tc::kmajor_offset(t, 0, kInPad)) =
-            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
-                       pack_bf16(f[6], f[7]));
-#pragma unroll
-        for (int k = 0; k < kIn; ++k)
-            *reinterpret_cast<uint16_t*>(S.xT + tc::kmajor_offset(k, t, kTile)) = bf16_bits(f[k]);
         const float tgt = valid ? target[i] * inv_scale : 0.f;
-
-        // z1 = x W1^T
-        sync_issue();
-        if (t == 0) {
-            tc::fence_after_sync();
-            tc::mma_bf16(tmem + kColZ1, tc::smem_desc(sx, 128, kInPad * 16),
-                         tc::smem_desc(sw1, 128, kInPad * 16), id64, 0);
-            tc::mma_commit(&S.bar);
-        }
-        if (!wait()) break;
-        // a1 -> A and B^T tiles; z2 = a1 W2^T
-#pragma unroll 1
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(lane + kColZ1 + c0, v);
+        const bool more = tile + (int)gridDim.x < tiles;
+        if (more && t < kTile) load_features(feat, (tile + gridDim.x) * kTile + t, n, S.norm, f);
+        float d1[kGradCols], d2[kGradCols];
+        wait();  // z1
+        hidden(S.b1, S.a1, d1);
+        publish();
+        if (t == 0) forward(sa1, kNT * 16, sw2, kHid / 16, kHid * 16);
+        wait();  // z2
+        hidden(S.b2, S.a2, d2);
+        publish();
+        if (t == 0) forward(sa2, kNT * 16, sw3, kHid / 16, kHid * 16);
+        wait();  // z3
+        float a3[kGradCols], v[kGradCols];
+        tc::tmem_ld16(lane + kColW + c0, v);
+        float part = 0.f;
 #pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = silu(v[q] + S.b1[c0 + q]);
-            store_row64(S.a1, t, v, c0);
-            store_col128(S.a1T, t, v, c0);
+        for (int q = 0; q < kGradCols; ++q) {
+            const float z = v[q] + S.b3[c0 + q];
+            a3[q] = silu(z);
+            v[q] = dsilu(z);
+            part = __fmaf_rn(S.w4[c0 + q], a3[q], part);
         }
-        sync_issue();
-        if (t == 0) {
-            tc::fence_after_sync();
-            gemm_k64(tmem + kColZ2, sa1, sw2);
-            tc::mma_commit(&S.bar);
-        }
-        if (!wait()) break;
-#pragma unroll 1
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(lane + kColZ2 + c0, v);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = silu(v[q] + S.b2[c0 + q]);
-            store_row64(S.a2, t, v, c0);
-            store_col128(S.a2T, t, v, c0);
-        }
-        sync_issue();
-        if (t == 0) {
-            tc::fence_after_sync();
-            gemm_k64(tmem + kColZ3, sa2, sw3);
-            tc::mma_commit(&S.bar);
-        }
-        if (!wait()) break;
-        // output, loss, dy
-        float y = S.b4;
-#pragma unroll 1
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(lane + kColZ3 + c0, v);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) y = __fmaf_rn(S.w4[c0 + q], silu(v[q] + S.b3[c0 + q]), y);
-        }
+        S.y[group][row] = part;
+        ok = __syncthreads_and(ok);
+        if (!ok) break;  // uniform: a wait ran out
+        const float y = S.b4 + ((S.y[0][row] + S.y[1][row]) + (S.y[2][row] + S.y[3][row]));
         const float e = valid ? y - tgt : 0.f;
         const float dy = 2.0f * e * inv_n_total;
-        {
-            float l = e * e * inv_n_total;
-#pragma unroll
-            for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-            if ((t & 31) == 0) atomicAdd(&S.loss, l);
+        if (group == 0) {
+            loss = __fmaf_rn(e * e, inv_n_total, loss);
+            gb4 += dy;
         }
-        // dz3 = dy w4 silu'(z3); dw4 += dy a3; db4 += dy
-#pragma unroll 1
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
-            float v[16], g[16];
-            tc::tmem_ld16(lane + kColZ3 + c0, v);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const float z = v[q] + S.b3[c0 + q];
-                g[q] = dy * silu(z);
-                v[q] = dy * S.w4[c0 + q] * dsilu(z);
-            }
-            store_row64(S.dz, t, v, c0);
-            store_col128(S.dzT, t, v, c0);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                float s = g[q];
-#pragma unroll
-                for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if ((t & 31) == 0) atomicAdd(&S.gw4[c0 + q], s);
-            }
+        for (int q = 0; q < kGradCols; ++q) {
+            gw4[q] = __fmaf_rn(dy, a3[q], gw4[q]);
+            v[q] = dy * S.w4[c0 + q] * v[q];
         }
-        {
-            float s = dy;
-#pragma unroll
-            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if ((t & 31) == 0) atomicAdd(&S.gw4[kHid], s);
-        }
-        // da2 = dz3 W3; dW3|db3 += dz3^T [a2 | 1]
-        sync_issue();
+        put16(S.dz[0], kHid, v);
+        publish();
         if (t == 0) {
-            tc::fence_after_sync();
-            gemm_k64(tmem + kColDA, sdz, sw3t);
-            gemm_batch(tmem + kColG3, sa2T, id80);
-            tc::mma_commit(&S.bar);
+            backward(sdz, sw3);
+            weights(kColG3, sdz, sa2, kNT);
         }
-        if (!wait()) break;
-        // dz2 = da2 silu'(z2)
-#pragma unroll 1
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
-            float d[16], z[16];
-            tc::tmem_ld16(lane + kColDA + c0, d);
-            tc::tmem_ld16(lane + kColZ2 + c0, z);
+        wait();  // da2
+        tc::tmem_ld16(lane + kColW + c0, v);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) d[q] = d[q] * dsilu(z[q] + S.b2[c0 + q]);
-            store_row64(S.dz, t, d, c0);
-            store_col128(S.dzT, t, d, c0);
-        }
-        // da1 = dz2 W2; dW2|db2 += dz2^T [a1 | 1]
-        sync_issue();
+        for (int q = 0; q < kGradCols; ++q) v[q] = v[q] * d2[q];
+        put16(S.dz[1], kHid, v);
+        publish();
         if (t == 0) {
-            tc::fence_after_sync();
-            gemm_k64(tmem + kColDA, sdz, sw2t);
-            gemm_batch(tmem + kColG2, sa1T, id80);
-            tc::mma_commit(&S.bar);
+            backward(sdz + kDz, sw2);
+            weights(kColG2, sdz + kDz, sa1, kNT);
         }
-        if (!wait()) break;
-        // dz1 = da1 silu'(z1); dW1|db1 += dz1^T [x | 1]
-#pragma unroll 1
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
-            float d[16], z[16];
-            tc::tmem_ld16(lane + kColDA + c0, d);
-            tc::tmem_ld16(lane + kColZ1 + c0, z);
+        wait();  // da1, and everything issued before it
+        tc::tmem_ld16(lane + kColW + c0, v);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) d[q] = d[q] * dsilu(z[q] + S.b1[c0 + q]);
-            store_col128(S.dzT, t, d, c0);
-        }
-        sync_issue();
+        for (int q = 0; q < kGradCols; ++q) v[q] = v[q] * d1[q];
+        put16(S.dz[0], kHid, v);
+        if (more && t < kTile) put_x(buf ^ 1, f);
+        publish();
         if (t == 0) {
-            tc::fence_after_sync();
-            gemm_batch(tmem + kColG1, sxT, id16);
-            tc::mma_commit(&S.bar);
+            weights(kColG1, sdz, sx + buf * kXBytes, kInPad);
+            if (more) forward(sx + (buf ^ 1) * kXBytes, kInPad * 16, sw1, 1, kInPad * 16);
+            else tc::mma_commit(&S.bar);
         }
-        if (!wait()) break;
+        buf ^= 1;
         acc = 1;
-        tc::fence_before_sync();
     }
-    __syncthreads();
-    // flush: rows 0..63 of the weight-gradient accumulators live in warps 0 and 1
-    if (ok && acc && warp < 2) {
-        const int o = t;  // output feature
-#pragma unroll 1
-        for (int c0 = 0; c0 < kNT; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(lane + kColG3 + c0, v);
+    if (ok) wait();  // the last weight gradients
+    ok = __syncthreads_and(ok);
+    // flush: rows 0..63 of the weight-gradient accumulators are lanes 0..63
+    if (ok && row < kHid) {
+        const int o = row;  // output feature
+        float v[16];
+        auto row16 = [&](float* g) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const int c = c0 + q;
-                if (c < kHid) atomicAdd(&grad[kW3 + o * kHid + c], v[q]);
-                else if (c == kHid) atomicAdd(&grad[kB3 + o], v[q]);
+            for (int q = 0; q < 16; q += 4) tc::red_add4(g + q, v[q], v[q + 1], v[q + 2], v[q + 3]);
+        };
+        tc::tmem_ld16(lane + kColG3 + c0, v);
+        row16(grad + kW3 + o * kHid + c0);
+        tc::tmem_ld16(lane + kColG2 + c0, v);
+        row16(grad + kW2 + o * kHid + c0);
+        if (group == 0) {
+            tc::tmem_ld16(lane + kColG3 + kHid, v);
+            atomicAdd(&grad[kB3 + o], v[0]);
+        } else if (group == 1) {
+            tc::tmem_ld16(lane + kColG2 + kHid, v);
+            atomicAdd(&grad[kB2 + o], v[0]);
+        } else if (group == 2) {
+            tc::tmem_ld16(lane + kColG1, v);
+            tc::red_add4(grad + kW1 + o * kIn, v[0], v[1], v[2], v[3]);
+            tc::red_add4(grad + kW1 + o * kIn + 4, v[4], v[5], v[6], v[7]);
+            atomicAdd(&grad[kB1 + o], v[kIn]);
+        }
+    }
+    if (ok) {  // dw4, db4 and the loss: sums over the rows
+#pragma unroll
+        for (int q = 0; q < kGradCols; ++q) {
+#pragma unroll
+            for (int o = 16; o; o >>= 1) gw4[q] += __shfl_xor_sync(0xffffffffu, gw4[q], o);
+            if ((t & 31) == 0) S.gw4[warp & 3][c0 + q] = gw4[q];
+        }
+        if (group == 0) {
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+                gb4 += __shfl_xor_sync(0xffffffffu, gb4, o);
+                loss += __shfl_xor_sync(0xffffffffu, loss, o);
             }
-            tc::tmem_ld16(lane + kColG2 + c0, v);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const int c = c0 + q;
-                if (c < kHid) atomicAdd(&grad[kW2 + o * kHid + c], v[q]);
-                else if (c == kHid) atomicAdd(&grad[kB2 + o], v[q]);
+            if ((t & 31) == 0) {
+                atomicAdd(&S.gb4, gb4);
+                atomicAdd(&S.loss, loss);
             }
         }
-        float v[16];
-        tc::tmem_ld16(lane + kColG1, v);
-#pragma unroll
-        for (int q = 0; q < kIn; ++q) atomicAdd(&grad[kW1 + o * kIn + q], v[q]);
-        atomicAdd(&grad[kB1 + o], v[kIn]);
-    }
-    if (ok && acc) {
-        if (t <= kHid) atomicAdd(&grad[kW4 + t], S.gw4[t]);
-        if (t == 0) atomicAdd(&grad[kParams], S.loss);
+        __syncthreads();
+        if (t < kHid)
+            atomicAdd(&grad[kW4 + t],
+                      (S.gw4[0][t] + S.gw4[1][t]) + (S.gw4[2][t] + S.gw4[3][t]));
+        if (t == 0) {
+            atomicAdd(&grad[kB4], S.gb4);
+            atomicAdd(&grad[kParams], S.loss);
+        }
     }
     if (!ok && t == 0) atomicOr(err, (uint32_t)kErrTimeout);
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) {
         tc::fence_after_sync();
-        tc::tmem_free(tmem, kGradCols);
+        tc::tmem_free(tmem, kGradTmem);
     }
 }
 
-// Adam on the FP32 master parameters; clears the gradient (and the loss slot) afterwards.
+// Place of parameter k in the operand images (bytes), or -1 for biases and the output layer.
+__device__ __forceinline__ int image_offset(int k) {
+    if (k < kB1) return (int)tc::kmajor_offset(k / kIn, k % kIn, kInPad);
+    if (k >= kW2 && k < kB2)
+        return kHid * kInPad * 2 + (int)tc::kmajor_offset((k - kW2) / kHid, (k - kW2) % kHid, kHid);
+    if (k >= kW3 && k < kB3)
+        return (kHid * kInPad + kHid * kHid) * 2 +
+               (int)tc::kmajor_offset((k - kW3) / kHid, (k - kW3) % kHid, kHid);
+    return -1;
+}
+
+// Adam on the FP32 master parameters; clears the gradient (and the loss slot) afterwards and keeps
+// the weights' BF16 images up to date (a kernel of its own took 7 us to rebuild them).
 __global__ void k_mlp_adam(float* __restrict__ params, float* __restrict__ grad,
-                           float* __restrict__ m, float* __restrict__ v, float lr, float beta1,
-                           float beta2, float eps, float bc1, float bc2) {
+                           float* __restrict__ m, float* __restrict__ v,
+                           uint8_t* __restrict__ image, float lr, float beta1, float beta2,
+                           float eps, float bc1, float bc2) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > kParams) return;
     if (k == kParams) {
@@ -659,8 +650,11 @@ __global__ void k_mlp_adam(float* __restrict__ params, float* __restrict__ grad,
     const float vk = beta2 * v[k] + (1.0f - beta2) * g * g;
     m[k] = mk;
     v[k] = vk;
-    params[k] -= lr * (mk / bc1) / (sqrtf(vk / bc2) + eps);
+    const float p = params[k] - lr * (mk / bc1) / (sqrtf(vk / bc2) + eps);
+    params[k] = p;
     grad[k] = 0.f;
+    const int at = image_offset(k);
+    if (at >= 0) *reinterpret_cast<uint16_t*>(image + at) = bf16_bits(p);
 }
 
 }  // namespace akua::mlp

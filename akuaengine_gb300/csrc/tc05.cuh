@@ -11,6 +11,8 @@
 // lane m, column n is TMEM column (base + n).  A warp may read only its own 32-lane quarter
 // (warp w % 4 -> lanes 32 (w % 4) .. + 31).
 //
+// An operand may also be read MN-major from the same tile (kTransposeA, kTransposeB).
+//
 // Every wait on an mbarrier is bounded: on timeout the caller gets `false`, records an error
 // and still releases its tensor memory.
 #pragma once
@@ -42,6 +44,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
 __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
+// An operand read along the other axis (bits 15 and 16: A, B is MN-major).  The same tile serves: a
+// core matrix holds 8 rows x 8 contiguous elements either way, the contiguous axis is now M or N
+// (its next 8 elements SBO = 128 bytes on) and the rows are K (the next 8 rows LBO = the tile's
+// row-group stride on), so no transposed copy is stored.
+constexpr uint32_t kTransposeA = 1u << 15;
+constexpr uint32_t kTransposeB = 1u << 16;
 
 // --- tensor memory ------------------------------------------------------------------------------
 // Executed by one full warp.  Writes the allocated base address to *slot (shared memory).
@@ -88,6 +96,14 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
         "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
             smem_addr(bar))
         : "memory");
+}
+
+// --- reductions to global memory ------------------------------------------------------------------
+// p[0..3] += v, one 16-byte reduction (p 16-byte aligned).
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
+                 "f"(d)
+                 : "memory");
 }
 
 // --- mbarrier -----------------------------------------------------------------------------------
