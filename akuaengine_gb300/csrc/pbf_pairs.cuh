@@ -137,6 +137,95 @@ __device__ __forceinline__ void for_each_pair(const uint4* __restrict__ col, int
     }
 }
 
+// What a pair of neighbours adds to a particle's sums: N values of each.
+template <int N>
+struct Terms {
+    float2 v[N];
+};
+
+// Calls add(t, k) with the N terms t[] of each neighbour of particle i, in list order: load(j)
+// gathers a neighbour's record, term(a, b) evaluates two of them.  With LANES = 1 a thread works
+// through its particle's list by itself.  With 2 or 4 lanes per particle each lane gathers and
+// evaluates its own pair of every 4 or 8 entries, the next one's records in flight, and the lanes
+// hand their terms round by shuffles, so that every lane adds all of them in list order (the sums are
+// the same bit for bit) and a list takes a half or a quarter of the steps.  All lanes of a warp call
+// it (c = 0 for lanes without a particle).
+template <int LANES, bool WHOLE_TILE, int N, class L, class T, class A>
+__device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr4, int n, int i, int c,
+                                                   L&& load, T&& term, A&& add) {
+    if constexpr (LANES == 1) {
+        for_each_pair<WHOLE_TILE>(nbr4 + i, n, c, load, [&](auto a, auto b, bool two) {
+            const Terms<N> t = term(a, b);
+            float one[N];
+#pragma unroll
+            for (int q = 0; q < N; ++q) one[q] = t.v[q].x;
+            add(one);
+            if (two) {
+#pragma unroll
+                for (int q = 0; q < N; ++q) one[q] = t.v[q].y;
+                add(one);
+            }
+        });
+    } else {
+        constexpr int E = 2 * LANES;  // entries per step
+        const int role = threadIdx.x & (LANES - 1);
+        const int group = (threadIdx.x & 31) & ~(LANES - 1);
+        const int steps = __reduce_max_sync(0xffffffffu, (unsigned)((c + E - 1) / E));
+        auto pair = [&](int s, uint32_t& j0, uint32_t& j1) {  // this lane's entries of step s
+            const int e = E * s + 2 * role;
+            j0 = j1 = (uint32_t)i;
+            if (e < c) {
+                const uint2* at = reinterpret_cast<const uint2*>(nbr4 + (size_t)(e >> 2) * n + i);
+                const uint2 t = __ldg(at + ((e >> 1) & 1));
+                j0 = t.x;
+                j1 = e + 1 < c ? t.y : t.x;
+            }
+        };
+        uint32_t j0, j1;
+        pair(0, j0, j1);
+        auto ra = load(j0), rb = load(j1);
+        pair(1, j0, j1);
+        for (int s = 0; s < steps; ++s) {
+            const Terms<N> t = term(ra, rb);
+            if (s + 1 < steps) {
+                ra = load(j0);
+                rb = load(j1);
+                pair(s + 2, j0, j1);
+            }
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                float one[N];
+#pragma unroll
+                for (int q = 0; q < N; ++q)
+                    one[q] = __shfl_sync(0xffffffffu, (k & 1) ? t.v[q].y : t.v[q].x, group + (k >> 1));
+                if (E * s + k < c) add(one);
+            }
+        }
+    }
+}
+
+// Lanes per particle of the pair kernels.  A scene too small to fill the chip is as slow as the chain
+// of gathers of one list, which more lanes shorten, until the shuffles cost more issue slots than the
+// chain costs time: about 16 warps per SM with 4 lanes (24 with exact math, whose terms are longer)
+// and 18 with 2.  Steps in us with 1 / 2 / 4 lanes: 1,000 particles 95 / 95 / 84, 8,000 121 / 108 /
+// 96, 27,000 139 / 128 / 132 (exact 207 / 181 / 160), 40,000 156 / 151 / 176 (exact 226 / 205 / 216),
+// 60,000 167 / 176 / 208.
+inline int pair_lanes(int n, int sms, bool exact) {
+    const long long warps = 32ll * sms;  // threads of one warp per SM
+    if (4ll * n <= (exact ? 24 : 16) * warps) return 4;
+    return 2ll * n <= 18 * warps ? 2 : 1;
+}
+
+// sum += s * (x, y, z) of each neighbour's terms (s, x, y, z), one rounding per component.
+struct Sum3 {
+    float x = 0.f, y = 0.f, z = 0.f;
+    __device__ __forceinline__ void operator()(const float (&t)[4]) {
+        x = __fmaf_rn(t[0], t[1], x);
+        y = __fmaf_rn(t[0], t[2], y);
+        z = __fmaf_rn(t[0], t[3], z);
+    }
+};
+
 // A particle's two-float4 record (x.xyz, w0 | v.xyz, w1) read in one 256-bit load (32-byte
 // aligned: record j starts at float4 2j of a cudaMalloc'd array).
 struct Rec8 {
@@ -151,7 +240,8 @@ __device__ __forceinline__ Rec8 ld_rec8(const float4* __restrict__ rec, uint32_t
     return r;
 }
 
-// Density and lambda accumulators (ConstraintSolverCUDA.cu:16-97), two neighbours per call.
+// Density and lambda accumulators (ConstraintSolverCUDA.cu:16-97) and the terms of two neighbours:
+// mass, poly6, the spiky gradient, |grad_j C_i|^2.
 template <bool EXACT>
 struct DensityLambda2 {
     float rho, gx, gy, gz, sum;
@@ -160,29 +250,33 @@ struct DensityLambda2 {
         gx = gy = gz = sum = 0.f;
     }
     template <bool IN_REACH = false>
-    __device__ __forceinline__ void add2(const StepParams& p, float4 xi, float4 a, float4 b,
-                                         bool two) {
+    static __device__ __forceinline__ Terms<6> terms(const StepParams& p, float4 xi, float4 a,
+                                                     float4 b) {
         const float2 sx = diff2(xi.x, a.x, b.x);
         const float2 sy = diff2(xi.y, a.y, b.y);
         const float2 sz = diff2(xi.z, a.z, b.z);
         const float2 r2 = len2_2(sx, sy, sz);
-        const float2 w = poly6_2<IN_REACH>(p, r2);
-        float2 ux, uy, uz;
-        spiky2<EXACT, IN_REACH>(p, sx, sy, sz, r2, ux, uy, uz);
+        Terms<6> t;
+        t.v[0] = make_float2(a.w, b.w);
+        t.v[1] = poly6_2<IN_REACH>(p, r2);
+        spiky2<EXACT, IN_REACH>(p, sx, sy, sz, r2, t.v[2], t.v[3], t.v[4]);
         const float2 s = scale2(-p.inv_rho0, a.w, b.w);
-        const float2 l = len2_2(mul2(s, ux), mul2(s, uy), mul2(s, uz));
-        rho = __fmaf_rn(a.w, w.x, rho);
-        gx = __fmaf_rn(a.w, ux.x, gx);
-        gy = __fmaf_rn(a.w, uy.x, gy);
-        gz = __fmaf_rn(a.w, uz.x, gz);
-        sum = sum + l.x;
-        if (two) {
-            rho = __fmaf_rn(b.w, w.y, rho);
-            gx = __fmaf_rn(b.w, ux.y, gx);
-            gy = __fmaf_rn(b.w, uy.y, gy);
-            gz = __fmaf_rn(b.w, uz.y, gz);
-            sum = sum + l.y;
-        }
+        t.v[5] = len2_2(mul2(s, t.v[2]), mul2(s, t.v[3]), mul2(s, t.v[4]));
+        return t;
+    }
+    __device__ __forceinline__ void operator()(const float (&t)[6]) {
+        rho = __fmaf_rn(t[0], t[1], rho);
+        gx = __fmaf_rn(t[0], t[2], gx);
+        gy = __fmaf_rn(t[0], t[3], gy);
+        gz = __fmaf_rn(t[0], t[4], gz);
+        sum = sum + t[5];
+    }
+    template <bool IN_REACH = false>
+    __device__ __forceinline__ void add2(const StepParams& p, float4 xi, float4 a, float4 b,
+                                         bool two) {
+        const Terms<6> t = terms<IN_REACH>(p, xi, a, b);
+        (*this)({t.v[0].x, t.v[1].x, t.v[2].x, t.v[3].x, t.v[4].x, t.v[5].x});
+        if (two) (*this)({t.v[0].y, t.v[1].y, t.v[2].y, t.v[3].y, t.v[4].y, t.v[5].y});
     }
     __device__ __forceinline__ float lambda(const StepParams& p) const {
         const float ax = gx * p.inv_rho0, ay = gy * p.inv_rho0, az = gz * p.inv_rho0;
@@ -192,23 +286,39 @@ struct DensityLambda2 {
     }
 };
 
-template <bool EXACT>
+// The particle of this thread (LANES threads each) and whether there is one; threads beyond the last
+// particle leave, except where their warp's lanes work together.
+template <int LANES>
+__device__ __forceinline__ bool particle_of_thread(int n, int& i) {
+    i = (int)((blockIdx.x * blockDim.x + threadIdx.x) / LANES);
+    const bool live = i < n;
+    if (LANES > 1 && !live) i = n - 1;
+    return live;
+}
+// Whether this thread writes its particle's results.
+template <int LANES>
+__device__ __forceinline__ bool writes(bool live) {
+    return live && (threadIdx.x & (LANES - 1)) == 0;
+}
+
+template <bool EXACT, int LANES>
 __global__ void __launch_bounds__(kMaxPairBlock)
     k_density_lambda(const StepParams* __restrict__ P, const float4* __restrict__ ps,
                      const uint4* __restrict__ nbr4, const uint32_t* __restrict__ cnt,
                      float* __restrict__ rho_out, float* __restrict__ lam_out,
                      float* __restrict__ lacc, float4* __restrict__ psl) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P->n) return;
+    const int n = P->n;
+    int i;
+    const bool live = particle_of_thread<LANES>(n, i);
+    if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    const int n = p.n;
-    if (i >= n) return;
     const float4 xi = ps[i];
     DensityLambda2<EXACT> acc;
     acc.init(xi.w, p);
-    for_each_pair<true>(
-        nbr4 + i, n, (int)cnt[i], [&](uint32_t j) { return __ldg(ps + j); },
-        [&](float4 a, float4 b, bool two) { acc.add2(p, xi, a, b, two); });
+    for_each_neighbour<LANES, true, 6>(
+        nbr4, n, i, live ? (int)cnt[i] : 0, [&](uint32_t j) { return __ldg(ps + j); },
+        [&](float4 a, float4 b) { return DensityLambda2<EXACT>::terms(p, xi, a, b); }, acc);
+    if (!writes<LANES>(live)) return;
     rho_out[i] = acc.rho;
     const float l = acc.lambda(p);
     lam_out[i] = l;
@@ -242,14 +352,14 @@ struct Rec5 {
 };
 
 // Position delta with artificial pressure (ConstraintSolverCUDA.cu:99-130).
-template <bool EXACT>
-__device__ __forceinline__ float3 position_delta(const StepParams& p, int n, float4 xi, float li,
+template <bool EXACT, int LANES>
+__device__ __forceinline__ float3 position_delta(const StepParams& p, float4 xi, float li,
                                                  const float4* __restrict__ ps,
                                                  const float* __restrict__ lam,
-                                                 const uint4* __restrict__ col, int c) {
-    float dx = 0.f, dy = 0.f, dz = 0.f;
+                                                 const uint4* __restrict__ nbr4, int i, int c) {
+    Sum3 d;
     auto load = [&](uint32_t j) { return Rec5{__ldg(ps + j), __ldg(lam + j)}; };
-    for_each_pair<false>(col, n, c, load, [&](const Rec5& ra, const Rec5& rb, bool two) {
+    auto term = [&](const Rec5& ra, const Rec5& rb) {
         const float4 a = ra.x, b = rb.x;
         const float2 lj = make_float2(ra.l, rb.l);
         const float2 sx = diff2(xi.x, a.x, b.x);
@@ -260,55 +370,45 @@ __device__ __forceinline__ float3 position_delta(const StepParams& p, int n, flo
         // and is contracted into it, as the CUDA compiler does with the reference's expression
         // (ConstraintSolverCUDA.cu:124-126).
         const float2 pw = scorr_pow2<EXACT, false>(p, r2);
-        const float2 bb = mul2(fma2(f2(p.neg_k), pw, add2(f2(li), lj)), make_float2(a.w, b.w));
-        float2 gx, gy, gz;
-        spiky2<EXACT>(p, sx, sy, sz, r2, gx, gy, gz);
-        dx = __fmaf_rn(bb.x, gx.x, dx);
-        dy = __fmaf_rn(bb.x, gy.x, dy);
-        dz = __fmaf_rn(bb.x, gz.x, dz);
-        if (two) {
-            dx = __fmaf_rn(bb.y, gx.y, dx);
-            dy = __fmaf_rn(bb.y, gy.y, dy);
-            dz = __fmaf_rn(bb.y, gz.y, dz);
-        }
-    });
-    return make_float3(dx * p.inv_rho0, dy * p.inv_rho0, dz * p.inv_rho0);
+        Terms<4> t;
+        t.v[0] = mul2(fma2(f2(p.neg_k), pw, add2(f2(li), lj)), make_float2(a.w, b.w));
+        spiky2<EXACT>(p, sx, sy, sz, r2, t.v[1], t.v[2], t.v[3]);
+        return t;
+    };
+    for_each_neighbour<LANES, false, 4>(nbr4, p.n, i, c, load, term, d);
+    return make_float3(d.x * p.inv_rho0, d.y * p.inv_rho0, d.z * p.inv_rho0);
 }
 
 // The same sum when every particle has mass `m`: positions and lambdas come from one 16-byte
 // gather of psl[j] = (x*_j, lambda_j), and (lambda_i + lambda_j + s_corr) * m is the same product.
 // FOUR: the power is 4 (the reference's), known before the loop: without the per-pair branch to
 // powf the parameters stay in registers (1M particles: 75.1 -> 69.9 us).
-template <bool EXACT, bool FOUR>
-__device__ __forceinline__ float3 position_delta_uniform(const StepParams& p, int n, float4 xl,
+template <bool EXACT, bool FOUR, int LANES>
+__device__ __forceinline__ float3 position_delta_uniform(const StepParams& p,
                                                          const float4* __restrict__ psl, float m,
-                                                         const uint4* __restrict__ col, int c) {
-    float dx = 0.f, dy = 0.f, dz = 0.f;
+                                                         const uint4* __restrict__ nbr4, int i,
+                                                         int c) {
+    const float4 xl = psl[i];
+    Sum3 d;
     auto load = [&](uint32_t j) { return __ldg(psl + j); };
-    for_each_pair<true>(col, n, c, load, [&](float4 a, float4 b, bool two) {
+    auto term = [&](float4 a, float4 b) {
         const float2 sx = diff2(xl.x, a.x, b.x);
         const float2 sy = diff2(xl.y, a.y, b.y);
         const float2 sz = diff2(xl.z, a.z, b.z);
         const float2 r2 = len2_2(sx, sy, sz);
         const float2 pw = scorr_pow2<EXACT, FOUR>(p, r2);
-        const float2 bb = mul2(fma2(f2(p.neg_k), pw, plus2(xl.w, a.w, b.w)), f2(m));
-        float2 gx, gy, gz;
-        spiky2<EXACT>(p, sx, sy, sz, r2, gx, gy, gz);
-        dx = __fmaf_rn(bb.x, gx.x, dx);
-        dy = __fmaf_rn(bb.x, gy.x, dy);
-        dz = __fmaf_rn(bb.x, gz.x, dz);
-        if (two) {
-            dx = __fmaf_rn(bb.y, gx.y, dx);
-            dy = __fmaf_rn(bb.y, gy.y, dy);
-            dz = __fmaf_rn(bb.y, gz.y, dz);
-        }
-    });
-    return make_float3(dx * p.inv_rho0, dy * p.inv_rho0, dz * p.inv_rho0);
+        Terms<4> t;
+        t.v[0] = mul2(fma2(f2(p.neg_k), pw, plus2(xl.w, a.w, b.w)), f2(m));
+        spiky2<EXACT>(p, sx, sy, sz, r2, t.v[1], t.v[2], t.v[3]);
+        return t;
+    };
+    for_each_neighbour<LANES, true, 4>(nbr4, p.n, i, c, load, term, d);
+    return make_float3(d.x * p.inv_rho0, d.y * p.inv_rho0, d.z * p.inv_rho0);
 }
 
 // Delta of particle i: the single-gather form when the step's masses all have one bit pattern
 // (mass_bits = {0 when they do, that pattern}, from k_gather), else the general one.
-template <bool EXACT>
+template <bool EXACT, int LANES>
 __device__ __forceinline__ float3 delta_of(const StepParams& p, int i, float4 xi,
                                            const float4* __restrict__ ps_in,
                                            const float* __restrict__ lam,
@@ -318,10 +418,10 @@ __device__ __forceinline__ float3 delta_of(const StepParams& p, int i, float4 xi
     if (__ldg(mass_bits) == 0u) {
         const float m = __uint_as_float(__ldg(mass_bits + 1));
         return p.corr_n_int == 4
-                   ? position_delta_uniform<EXACT, true>(p, p.n, psl[i], psl, m, nbr4 + i, c)
-                   : position_delta_uniform<EXACT, false>(p, p.n, psl[i], psl, m, nbr4 + i, c);
+                   ? position_delta_uniform<EXACT, true, LANES>(p, psl, m, nbr4, i, c)
+                   : position_delta_uniform<EXACT, false, LANES>(p, psl, m, nbr4, i, c);
     }
-    return position_delta<EXACT>(p, p.n, xi, lam[i], ps_in, lam, nbr4 + i, c);
+    return position_delta<EXACT, LANES>(p, xi, lam[i], ps_in, lam, nbr4, i, c);
 }
 
 // Soft box clamp of one coordinate (ConstraintSolverCUDA.cu:136-157).
@@ -333,19 +433,21 @@ __device__ __forceinline__ float clamp_axis(float x, float lo_wall, float hi_wal
     return x + c;
 }
 
-template <bool EXACT>
+template <bool EXACT, int LANES>
 __global__ void __launch_bounds__(kMaxPairBlock)
     k_delta_correct(const StepParams* __restrict__ P, const float4* __restrict__ ps_in,
                     const float* __restrict__ lam, const uint4* __restrict__ nbr4,
                     const uint32_t* __restrict__ cnt, float4* __restrict__ ps_out,
                     float4* __restrict__ dp4, const float4* __restrict__ psl,
                     const uint32_t* __restrict__ mass_bits) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P->n) return;
+    int i;
+    const bool live = particle_of_thread<LANES>(P->n, i);
+    if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    if (i >= p.n) return;
     const float4 xi = ps_in[i];
-    const float3 d = delta_of<EXACT>(p, i, xi, ps_in, lam, psl, mass_bits, nbr4, (int)cnt[i]);
+    const float3 d = delta_of<EXACT, LANES>(p, i, xi, ps_in, lam, psl, mass_bits, nbr4,
+                                            live ? (int)cnt[i] : 0);
+    if (!writes<LANES>(live)) return;
     dp4[i] = make_float4(d.x, d.y, d.z, 0.f);
     float nx = clamp_axis(xi.x + d.x, p.box_min[0], p.box_max[0]);
     float ny = clamp_axis(xi.y + d.y, p.box_min[1], p.box_max[1]);
@@ -380,7 +482,7 @@ __device__ __forceinline__ void damp_plane(const StepParams& p, float px, float 
 // (IntegrationCUDA.cu:75-102).  With `has_delta == 0` (zero iterations) the predicted positions
 // go straight to the update and the carried density/lambda/delta move into the state.  Also moves
 // the gathered colour, size and reference rank into the state arrays.
-template <bool EXACT>
+template <bool EXACT, int LANES>
 __global__ void __launch_bounds__(kMaxPairBlock)
     k_delta_final(const StepParams* __restrict__ P, const float4* __restrict__ ps_in,
                   const float* __restrict__ lam, const uint4* __restrict__ nbr4,
@@ -394,14 +496,18 @@ __global__ void __launch_bounds__(kMaxPairBlock)
                   float* __restrict__ rho, float* __restrict__ lam_out, int has_delta,
                   const float4* __restrict__ psl, const uint32_t* __restrict__ mass_bits,
                   float4* __restrict__ xv8) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P->n) return;
+    int i;
+    const bool live = particle_of_thread<LANES>(P->n, i);
+    if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    if (i >= p.n) return;
     const float4 xi = ps_in[i];
     float nx = xi.x, ny = xi.y, nz = xi.z;
+    float3 d = make_float3(0.f, 0.f, 0.f);
+    if (has_delta)
+        d = delta_of<EXACT, LANES>(p, i, xi, ps_in, lam, psl, mass_bits, nbr4,
+                                   live ? (int)cnt[i] : 0);
+    if (!writes<LANES>(live)) return;
     if (has_delta) {
-        const float3 d = delta_of<EXACT>(p, i, xi, ps_in, lam, psl, mass_bits, nbr4, (int)cnt[i]);
         dp4[i] = make_float4(d.x, d.y, d.z, 0.f);
         nx = clamp_axis(xi.x + d.x, p.box_min[0], p.box_max[0]);
         ny = clamp_axis(xi.y + d.y, p.box_min[1], p.box_max[1]);
@@ -455,21 +561,21 @@ __global__ void __launch_bounds__(kMaxPairBlock)
 
 // omega_i = sum_j -m_j (v_j - v_i) x grad W(x_i - x_j)  (IntegrationCUDA.cu:104-128).
 // om4.w = |omega_i| for the confinement pass.
-template <bool EXACT>
+template <bool EXACT, int LANES>
 __global__ void __launch_bounds__(kMaxPairBlock)
     k_vorticity(const StepParams* __restrict__ P, const float4* __restrict__ x4,
                 const float4* __restrict__ v4, const float4* __restrict__ xv8,
                 const uint4* __restrict__ nbr4, const uint32_t* __restrict__ cnt,
                 float4* __restrict__ om4, float4* __restrict__ xw4) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P->n) return;
+    const int n = P->n;
+    int i;
+    const bool live = particle_of_thread<LANES>(n, i);
+    if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    const int n = p.n;
-    if (i >= n) return;
     const float4 xi = x4[i], vi = v4[i];
-    float wx = 0.f, wy = 0.f, wz = 0.f;
+    Sum3 w;
     auto load = [&](uint32_t j) { return ld_rec8(xv8, j); };
-    auto term = [&](const Rec8& ra, const Rec8& rb, bool two) {
+    auto term = [&](const Rec8& ra, const Rec8& rb) {
         const float4 a = ra.x, b = rb.x, va = ra.v, vb = rb.v;
         const float2 sx = diff2(xi.x, a.x, b.x);
         const float2 sy = diff2(xi.y, a.y, b.y);
@@ -480,19 +586,16 @@ __global__ void __launch_bounds__(kMaxPairBlock)
         const float2 uy = rdiff2(va.y, vb.y, vi.y);
         const float2 uz = rdiff2(va.z, vb.z, vi.z);
         // cross(u, g) contracted as fma(u.y, g.z, -(u.z * g.y)), ...
-        const float2 cx = fma2(uy, gz, mul2(f2(-1.0f), mul2(uz, gy)));
-        const float2 cy = fma2(uz, gx, mul2(f2(-1.0f), mul2(ux, gz)));
-        const float2 cz = fma2(ux, gy, mul2(f2(-1.0f), mul2(uy, gx)));
-        wx = __fmaf_rn(-a.w, cx.x, wx);
-        wy = __fmaf_rn(-a.w, cy.x, wy);
-        wz = __fmaf_rn(-a.w, cz.x, wz);
-        if (two) {
-            wx = __fmaf_rn(-b.w, cx.y, wx);
-            wy = __fmaf_rn(-b.w, cy.y, wy);
-            wz = __fmaf_rn(-b.w, cz.y, wz);
-        }
+        Terms<4> t;
+        t.v[0] = make_float2(-a.w, -b.w);
+        t.v[1] = fma2(uy, gz, mul2(f2(-1.0f), mul2(uz, gy)));
+        t.v[2] = fma2(uz, gx, mul2(f2(-1.0f), mul2(ux, gz)));
+        t.v[3] = fma2(ux, gy, mul2(f2(-1.0f), mul2(uy, gx)));
+        return t;
     };
-    for_each_pair<EXACT>(nbr4 + i, n, (int)cnt[i], load, term);
+    for_each_neighbour<LANES, EXACT, 4>(nbr4, n, i, live ? (int)cnt[i] : 0, load, term, w);
+    if (!writes<LANES>(live)) return;
+    const float wx = w.x, wy = w.y, wz = w.z;
     const float wn = __fsqrt_rn(len2(wx, wy, wz));
     om4[i] = make_float4(wx, wy, wz, wn);
     xw4[i] = make_float4(xi.x, xi.y, xi.z, wn);  // (x, |omega|) for confinement's single gather
@@ -502,50 +605,46 @@ __global__ void __launch_bounds__(kMaxPairBlock)
 // particle records (x, m_i / rho_i | v) for the XSPH pass.
 // Capped at 48 registers (five 256-thread blocks per SM): 80 µs against 84 at 60 registers on the
 // 1M scene, although 36 bytes spill; the same cap slowed vorticity and the last delta pass.
-template <bool EXACT>
-__global__ void __launch_bounds__(kMaxPairBlock, 5)
+template <bool EXACT, int LANES>
+__global__ void __launch_bounds__(kMaxPairBlock, LANES == 1 ? 5 : 1)
     k_confine(const StepParams* __restrict__ P, const float4* __restrict__ x4,
               const float4* __restrict__ v4, const float4* __restrict__ om4,
               const float* __restrict__ rho, const uint4* __restrict__ nbr4,
               const uint32_t* __restrict__ cnt, float4* __restrict__ xv8,
               const float4* __restrict__ xw4, const uint32_t* __restrict__ mass_bits) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P->n) return;
+    const int n = P->n;
+    int i;
+    const bool live = particle_of_thread<LANES>(n, i);
+    if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    const int n = p.n;
-    if (i >= n) return;
     const float4 xi = x4[i], vi = v4[i], wi = om4[i];
     const float rho_i = rho[i];
-    float ex = 0.f, ey = 0.f, ez = 0.f;
-    // pair term m_j (|omega_i| - |omega_j|) grad W, given positions, masses and |omega_j|
-    auto term = [&](float4 a, float4 b, float2 mj, float2 wj, bool two) {
+    const int c = live ? (int)cnt[i] : 0;
+    Sum3 eta;
+    // m_j (|omega_i| - |omega_j|) and grad W, given positions, masses and |omega_j|
+    auto pair = [&](float4 a, float4 b, float2 mj, float2 wj) {
         const float2 sx = diff2(xi.x, a.x, b.x);
         const float2 sy = diff2(xi.y, a.y, b.y);
         const float2 sz = diff2(xi.z, a.z, b.z);
-        float2 gx, gy, gz;
-        spiky2<EXACT>(p, sx, sy, sz, len2_2(sx, sy, sz), gx, gy, gz);
-        const float2 s = mul2(mj, sub2(f2(wi.w), wj));
-        ex = __fmaf_rn(s.x, gx.x, ex);
-        ey = __fmaf_rn(s.x, gy.x, ey);
-        ez = __fmaf_rn(s.x, gz.x, ez);
-        if (two) {
-            ex = __fmaf_rn(s.y, gx.y, ex);
-            ey = __fmaf_rn(s.y, gy.y, ey);
-            ez = __fmaf_rn(s.y, gz.y, ez);
-        }
+        Terms<4> t;
+        spiky2<EXACT>(p, sx, sy, sz, len2_2(sx, sy, sz), t.v[1], t.v[2], t.v[3]);
+        t.v[0] = mul2(mj, sub2(f2(wi.w), wj));
+        return t;
     };
     if (__ldg(mass_bits) == 0u) {  // one mass: (x, |omega|) in one gather, the same products
         const float m = __uint_as_float(__ldg(mass_bits + 1));
         auto load = [&](uint32_t j) { return __ldg(xw4 + j); };
-        for_each_pair<false>(nbr4 + i, n, (int)cnt[i], load, [&](float4 a, float4 b, bool two) {
-            term(a, b, f2(m), make_float2(a.w, b.w), two);
-        });
+        auto term = [&](float4 a, float4 b) { return pair(a, b, f2(m), make_float2(a.w, b.w)); };
+        for_each_neighbour<LANES, false, 4>(nbr4, n, i, c, load, term, eta);
     } else {
         auto load = [&](uint32_t j) { return Rec5{__ldg(x4 + j), __ldg(&om4[j].w)}; };
-        for_each_pair<false>(nbr4 + i, n, (int)cnt[i], load, [&](const Rec5& a, const Rec5& b, bool two) {
-            term(a.x, b.x, make_float2(a.x.w, b.x.w), make_float2(a.l, b.l), two);
-        });
+        auto term = [&](const Rec5& a, const Rec5& b) {
+            return pair(a.x, b.x, make_float2(a.x.w, b.x.w), make_float2(a.l, b.l));
+        };
+        for_each_neighbour<LANES, false, 4>(nbr4, n, i, c, load, term, eta);
     }
+    if (!writes<LANES>(live)) return;
+    float ex = eta.x, ey = eta.y, ez = eta.z;
     const float inv_d = __fdiv_rn(1.0f, rho_i);
     ex = ex * inv_d;
     ey = ey * inv_d;
@@ -573,42 +672,42 @@ __global__ void __launch_bounds__(kMaxPairBlock, 5)
 
 // XSPH viscosity (IntegrationCUDA.cu:167-195) from the confined-velocity snapshot in the records
 // (x, m / rho | v).  Also leaves the bucket table all-empty for the next step.
+template <int LANES>
 __global__ void __launch_bounds__(kMaxPairBlock)
     k_xsph(const StepParams* __restrict__ P, const float4* __restrict__ xv8,
            const uint4* __restrict__ nbr4, const uint32_t* __restrict__ cnt,
            float4* __restrict__ v4, const uint32_t* __restrict__ kr, uint2* __restrict__ table) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P->n) return;
-    {  // the walk is done: empty this step's bucket entries (thread i: the bucket starting at rank i)
+    const int n = P->n;
+    int i;
+    const bool live = particle_of_thread<LANES>(n, i);
+    if (LANES == 1 && !live) return;
+    if (writes<LANES>(live)) {
+        // the walk is done: empty this step's bucket entries (particle i: the bucket starting at
+        // rank i)
         const uint32_t k = kr[i];
         if (i == 0 || kr[i - 1] != k) table[k] = make_uint2(0u, 0u);
     }
     const StepParams& p = params_for(P, i);
-    const int n = p.n;
-    if (i >= n) return;
     const Rec8 ri = ld_rec8(xv8, (uint32_t)i);
     const float4 xi = ri.x, vi = ri.v;
-    float ax = 0.f, ay = 0.f, az = 0.f;
+    Sum3 sum;
     auto load = [&](uint32_t j) { return ld_rec8(xv8, j); };
-    for_each_pair<true>(nbr4 + i, n, (int)cnt[i], load, [&](const Rec8& ra, const Rec8& rb, bool two) {
+    auto term = [&](const Rec8& ra, const Rec8& rb) {
         const float4 a = ra.x, b = rb.x, va = ra.v, vb = rb.v;
         const float2 sx = diff2(xi.x, a.x, b.x);
         const float2 sy = diff2(xi.y, a.y, b.y);
         const float2 sz = diff2(xi.z, a.z, b.z);
-        const float2 w = poly6_2(p, len2_2(sx, sy, sz));
         const float2 s = make_float2(a.w, b.w);  // m_j / rho_j
-        const float2 tx = mul2(s, rdiff2(va.x, vb.x, vi.x));
-        const float2 ty = mul2(s, rdiff2(va.y, vb.y, vi.y));
-        const float2 tz = mul2(s, rdiff2(va.z, vb.z, vi.z));
-        ax = __fmaf_rn(tx.x, w.x, ax);
-        ay = __fmaf_rn(ty.x, w.x, ay);
-        az = __fmaf_rn(tz.x, w.x, az);
-        if (two) {
-            ax = __fmaf_rn(tx.y, w.y, ax);
-            ay = __fmaf_rn(ty.y, w.y, ay);
-            az = __fmaf_rn(tz.y, w.y, az);
-        }
-    });
+        Terms<4> t;
+        t.v[0] = poly6_2(p, len2_2(sx, sy, sz));
+        t.v[1] = mul2(s, rdiff2(va.x, vb.x, vi.x));
+        t.v[2] = mul2(s, rdiff2(va.y, vb.y, vi.y));
+        t.v[3] = mul2(s, rdiff2(va.z, vb.z, vi.z));
+        return t;
+    };
+    for_each_neighbour<LANES, true, 4>(nbr4, n, i, live ? (int)cnt[i] : 0, load, term, sum);
+    if (!writes<LANES>(live)) return;
+    const float ax = sum.x, ay = sum.y, az = sum.z;
     v4[i] = make_float4(__fmaf_rn(p.visc, ax, vi.x), __fmaf_rn(p.visc, ay, vi.y),
                         __fmaf_rn(p.visc, az, vi.z), 0.f);
 }

@@ -347,11 +347,11 @@ void launch_search(akua_pbf* s, cudaStream_t st, int density, float* feat) {
     }
 }
 
-template <bool EXACT>
+template <bool EXACT, int LANES>
 void enqueue_pairs(akua_pbf* s, cudaStream_t st, Marker& mark) {
     const int n = s->n;
     const int* pb = s->pair_block;  // per kernel: density, delta, last delta, vort., conf., XSPH
-    auto gp = [&](int k) { return grid_for(n, pb[k]); };
+    auto gp = [&](int k) { return grid_for(n, pb[k] / LANES); };
     const int iters = s->cfg.solverIterations;
     float4* ps[2] = {s->ps0, s->ps1};
     const uint4* nbr4 = reinterpret_cast<const uint4*>(s->nbr);
@@ -366,17 +366,17 @@ void enqueue_pairs(akua_pbf* s, cudaStream_t st, Marker& mark) {
         float4* cur = ps[it & 1];
         float4* nxt = ps[(it + 1) & 1];
         if (it > 0) {
-            akua::k_density_lambda<EXACT><<<gp(0), pb[0], 0, st>>>(
+            akua::k_density_lambda<EXACT, LANES><<<gp(0), pb[0], 0, st>>>(
                 s->d_params, cur, nbr4, s->cnt, s->rho, s->lam,
                 learn == 1 ? s->lacc : nullptr, s->psl);  // warm: the network's estimate is the sum
             mark("k_density_lambda");
         }
         if (it + 1 < iters) {
-            akua::k_delta_correct<EXACT><<<gp(1), pb[1], 0, st>>>(
+            akua::k_delta_correct<EXACT, LANES><<<gp(1), pb[1], 0, st>>>(
                 s->d_params, cur, s->lam, nbr4, s->cnt, nxt, s->dp4, s->psl, s->mass_bits);
             mark("k_delta_correct");
         } else {
-            akua::k_delta_final<EXACT><<<gp(2), pb[2], 0, st>>>(
+            akua::k_delta_final<EXACT, LANES><<<gp(2), pb[2], 0, st>>>(
                 s->d_params, cur, s->lam, nbr4, s->cnt, s->x4g, s->x4, s->v4, s->vstar4, s->dp4,
                 s->col4g, s->sizeg, s->col4, s->size, s->rrefg, s->rref, s->rhog, s->lamg, s->dpg,
                 s->rho, nullptr, 1, s->psl, s->mass_bits, s->xv8);  // lam_out: zero iterations only
@@ -384,21 +384,21 @@ void enqueue_pairs(akua_pbf* s, cudaStream_t st, Marker& mark) {
         }
     }
     if (iters == 0) {
-        akua::k_delta_final<EXACT><<<gp(2), pb[2], 0, st>>>(
+        akua::k_delta_final<EXACT, LANES><<<gp(2), pb[2], 0, st>>>(
             s->d_params, s->ps0, nullptr, nbr4, s->cnt, s->x4g, s->x4, s->v4, s->vstar4, s->dp4,
             s->col4g, s->sizeg, s->col4, s->size, s->rrefg, s->rref, s->rhog, s->lamg, s->dpg,
             s->rho, s->lam, 0, s->psl, s->mass_bits, s->xv8);  // no delta: lambda is not read
         mark("k_delta_final");
     }
     // psl is free after the last delta: it carries (x, |omega|) to confinement
-    akua::k_vorticity<EXACT><<<gp(3), pb[3], 0, st>>>(s->d_params, s->x4, s->v4, s->xv8, nbr4,
+    akua::k_vorticity<EXACT, LANES><<<gp(3), pb[3], 0, st>>>(s->d_params, s->x4, s->v4, s->xv8, nbr4,
                                                       s->cnt, s->om4, s->psl);
     mark("k_vorticity");
-    akua::k_confine<EXACT><<<gp(4), pb[4], 0, st>>>(s->d_params, s->x4, s->v4, s->om4,
+    akua::k_confine<EXACT, LANES><<<gp(4), pb[4], 0, st>>>(s->d_params, s->x4, s->v4, s->om4,
                                                     s->rho, nbr4, s->cnt, s->xv8, s->psl,
                                                     s->mass_bits);
     mark("k_confine");
-    akua::k_xsph<<<gp(5), pb[5], 0, st>>>(s->d_params, s->xv8, nbr4, s->cnt, s->v4,
+    akua::k_xsph<LANES><<<gp(5), pb[5], 0, st>>>(s->d_params, s->xv8, nbr4, s->cnt, s->v4,
                                           s->kr, s->table);
     mark("k_xsph");
 }
@@ -441,8 +441,17 @@ void enqueue_body(akua_pbf* s, cudaStream_t st, const char* aos, size_t stride, 
     mark("k_gather");
     akua::k_table_build<<<ge, akua::kElemBlock, 0, st>>>(s->d_params, s->kr, s->r2i, s->table);
     mark("k_table_build");
-    if (s->options & AKUA_PBF_OPT_EXACT_MATH) enqueue_pairs<true>(s, st, mark);
-    else enqueue_pairs<false>(s, st, mark);
+    const bool exact = (s->options & AKUA_PBF_OPT_EXACT_MATH) != 0;
+    switch (akua::pair_lanes(n, s->sms, exact)) {
+        case 4:
+            exact ? enqueue_pairs<true, 4>(s, st, mark) : enqueue_pairs<false, 4>(s, st, mark);
+            break;
+        case 2:
+            exact ? enqueue_pairs<true, 2>(s, st, mark) : enqueue_pairs<false, 2>(s, st, mark);
+            break;
+        default:
+            exact ? enqueue_pairs<true, 1>(s, st, mark) : enqueue_pairs<false, 1>(s, st, mark);
+    }
     if (aos) {
         akua::k_export<<<grid_for(n, akua::kIoBlock), akua::kIoBlock, 0, st>>>(
             s->d_params, const_cast<char*>(aos), stride, n, s->r2i, s->kr, s->x4, s->v4, s->vstar4, s->dp4,

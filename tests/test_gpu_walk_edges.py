@@ -68,3 +68,40 @@ def test_runs_longer_than_the_pool(shape, kind):
               "nbr": s.read_debug(ak.DEBUG_NEIGHBOURS)}
     assert_grid_equal(ge, oe, cfg.maxNeighbours)
     assert_records_bitexact(p, o)
+
+
+@pytest.mark.parametrize("exact", [True, False], ids=["exact", "fast"])
+@pytest.mark.parametrize("where", ["4-", "4+", "2-", "2+"])
+def test_lanes_per_particle_edges(where, exact):
+    """Both sides of the lines where the pair kernels go from 4 to 2 and from 2 to 1 lanes per particle,
+    with two masses.  Exact math: the oracle's records; fast math: those of the same particles
+    stepped in a scene beyond every line (a far-away block makes up the number), whose kernels
+    use one lane."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    per = {"4": (24 if exact else 16) * 32 * sms // 4, "2": 18 * 32 * sms // 2}[where[0]]
+    n = per + (1 if where.endswith("+") else 0)
+    sc = first_of_block(n, seed=7)
+    sc.particles["mass"][::3] = 0.8
+    cfg, corr = PBFConfig(), LambdaCorrParams()
+    if exact:
+        g, ge = run_gpu(sc, cfg, corr, 1, ak.OPT_EXACT_MATH)
+        o, oe = run_oracle(sc, cfg, corr, 1)
+        assert_grid_equal(ge, oe, cfg.maxNeighbours)
+        assert_records_bitexact(g, o)
+        return
+    # one table size, so the shared particles hash alike; the filler is out of everyone's reach
+    table, extra = 1 << 24, 18 * 32 * sms
+    fill = first_of_block(extra, seed=8).particles
+    fill["position"][:, 0] += sc.box_max[0] + 5.0
+    box_max = (sc.box_max[0] + 40.0,) + tuple(sc.box_max[1:])
+    sc.particles["color"][:, 0] = np.arange(n) / np.float32(n)  # tell particles apart
+    out = []
+    for p in (sc.particles, np.concatenate([sc.particles, fill])):
+        wide = scene.Scene(p.copy(), sc.box_min, box_max, sc.dt, "lanes")
+        g, _ = run_gpu(wide, cfg, corr, 1, 0, table_size=table)
+        own = g[g["position"][:, 0] < sc.box_max[0] + 2.0]
+        out.append(own[np.lexsort((own["color"][:, 0],))])
+    assert len(out[0]) == n == len(out[1])
+    assert_records_bitexact(out[1], out[0])
