@@ -14,7 +14,7 @@
 namespace akua {
 
 // Everything a kernel of one step reads besides the particle arrays.  Lives in device memory and is
-// rewritten by a one-thread kernel at the start of every step, so a captured step graph replays
+// rewritten by the first kernel of every step, so a captured step graph replays
 // with new dt / box / gravity without re-capture.
 // Solid obstacles as signed distance functions (SDF boundary; the reference's clamp is a stand-in
 // for a boundary of this kind, ConstraintSolverCUDA.cu:131-134).  type: 1 sphere (centre a,

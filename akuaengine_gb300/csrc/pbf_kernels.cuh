@@ -70,10 +70,6 @@ __device__ __forceinline__ void copy_words(float* __restrict__ dst, const float*
     for (int w = done + threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
 }
 
-__global__ void k_set_params(StepParams p, StepParams* __restrict__ dst) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *dst = p;
-}
-
 // Per-scene parameters of a batch, uploaded in chunks passed by value (kernel parameters are
 // captured at launch, so the host copy may change right after).
 constexpr int kParamChunk = 16;  // 16 x 168 bytes: under the classic 4 KB parameter limit
@@ -129,17 +125,36 @@ __device__ __forceinline__ void write_keys(const StepParams& p, float4 x, float4
     bval[r] = i;
 }
 
+// The first kernel of a step (k_import or k_keys) also begins it: a single scene's parameters come by
+// value and are left in device memory for the kernels that follow (a batch's are uploaded before,
+// k_set_params_chunk), and the mass flag of k_gather is cleared.
+struct StepStart {
+    StepParams value;    // SINGLE only
+    StepParams* device;
+    uint32_t* mass_bits;
+};
+template <bool SINGLE>
+__device__ __forceinline__ const StepParams& begin_step(const StepStart& b, int i) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (SINGLE) *b.device = b.value;
+        b.mass_bits[0] = 0u;
+    }
+    return SINGLE ? b.value : params_for(b.device, i);
+}
+
 // Cell hash and Morton key of the walk cell of each predicted position, both scattered into the
 // previous reference order (so both stable sorts tie like the reference's), each with the import
 // index as payload.  Steps that import the records compute them in k_import instead.
+template <bool SINGLE>
 __global__ void __launch_bounds__(kElemBlock)
-    k_keys(const StepParams* __restrict__ P, const float4* __restrict__ x4,
+    k_keys(const __grid_constant__ StepStart begin, int n, const float4* __restrict__ x4,
            const float4* __restrict__ v4, const uint32_t* __restrict__ rref,
            uint32_t* __restrict__ akey, uint32_t* __restrict__ aval, uint32_t* __restrict__ bkey,
            uint32_t* __restrict__ bval) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P->n) return;
-    write_keys(params_for(P, i), x4[i], v4[i], rref[i], (uint32_t)i, akey, aval, bkey, bval);
+    if (i >= n) return;
+    write_keys(begin_step<SINGLE>(begin, i), x4[i], v4[i], rref[i], (uint32_t)i, akey, aval, bkey,
+               bval);
 }
 
 // Reads the attached records (buffer order = previous reference order) into the state, and writes
@@ -147,10 +162,12 @@ __global__ void __launch_bounds__(kElemBlock)
 // stages its records through shared memory so global reads are coalesced when records are packed.
 // With `carry`, density, lambda and position_delta are read too: with zero solver iterations the
 // reference leaves them as they were.
+template <bool SINGLE>
 __global__ void __launch_bounds__(kIoBlock)
-    k_import(const StepParams* __restrict__ P, const char* __restrict__ aos, uint64_t stride,
+    k_import(const __grid_constant__ StepStart begin, const char* __restrict__ aos, uint64_t stride,
              int n, float4* __restrict__ x4, float4* __restrict__ v4, float4* __restrict__ col4,
-             float* __restrict__ size, uint32_t* __restrict__ rref, float* __restrict__ rho,
+             float* __restrict__ size, uint32_t* __restrict__ origin, uint32_t* __restrict__ rref,
+             float* __restrict__ rho,
              float* __restrict__ lam, float4* __restrict__ dp4, int carry,
              uint32_t* __restrict__ akey, uint32_t* __restrict__ aval, uint32_t* __restrict__ bkey,
              uint32_t* __restrict__ bval) {
@@ -175,9 +192,11 @@ __global__ void __launch_bounds__(kIoBlock)
     const float4 v = make_float4(r[kVel], r[kVel + 1], r[kVel + 2], 0.f);
     x4[i] = x;
     v4[i] = v;
-    write_keys(params_for(P, i), x, v, (uint32_t)i, (uint32_t)i, akey, aval, bkey, bval);
+    write_keys(begin_step<SINGLE>(begin, i), x, v, (uint32_t)i, (uint32_t)i, akey, aval, bkey,
+               bval);
     col4[i] = make_float4(r[kColor], r[kColor + 1], r[kColor + 2], r[kColor + 3]);
     size[i] = r[kSize];
+    origin[i] = (uint32_t)i;
     rref[i] = (uint32_t)i;
     if (carry) {
         rho[i] = r[kDensity];
@@ -189,14 +208,15 @@ __global__ void __launch_bounds__(kIoBlock)
 
 // Moves the state into the new internal order (slot s holds the particle of import index
 // sp_import[s], reference rank rank_of_import[...]) and writes the predicted positions, both maps
-// between ranks and slots and the debug order (pre-sort record index per rank).
+// between ranks and slots and the debug order (pre-sort record index per rank).  Colour and size
+// stay where the import put them: a slot carries the index of its own (origin), which the export
+// follows, instead of 20 bytes that every step would move twice.
 __global__ void __launch_bounds__(kElemBlock)
     k_gather(const StepParams* __restrict__ P, const uint32_t* __restrict__ sp_import,
              const uint32_t* __restrict__ rank_of_import, const float4* __restrict__ x4,
-             const float4* __restrict__ v4, const float4* __restrict__ col4,
-             const float* __restrict__ size, const uint32_t* __restrict__ rref_old,
-             float4* __restrict__ x4g, float4* __restrict__ col4g, float* __restrict__ sizeg,
-             float4* __restrict__ ps0, uint32_t* __restrict__ r2i, uint32_t* __restrict__ rank_of,
+             const float4* __restrict__ v4, const uint32_t* __restrict__ origin,
+             const uint32_t* __restrict__ rref_old, float4* __restrict__ x4g,
+             uint32_t* __restrict__ origing, float4* __restrict__ ps0, uint32_t* __restrict__ r2i, uint32_t* __restrict__ rank_of,
              uint32_t* __restrict__ order_out,
              const float* __restrict__ rho_in, const float* __restrict__ lam_in,
              const float4* __restrict__ dp_in, float* __restrict__ rho_out,
@@ -224,8 +244,7 @@ __global__ void __launch_bounds__(kElemBlock)
         }
         const float4 q = make_float4(xs.x, xs.y, xs.z, x.w);
         x4g[s] = x;
-        col4g[s] = col4[o];
-        sizeg[s] = size[o];
+        origing[s] = origin[o];
         ps0[s] = q;
         r2i[r] = (uint32_t)s;
         rank_of[s] = r;
@@ -285,7 +304,8 @@ __global__ void __launch_bounds__(kIoBlock)
              const float4* __restrict__ dp4, const float4* __restrict__ om4,
              const float* __restrict__ rho, const float* __restrict__ lam,
              const float4* __restrict__ col4, const float* __restrict__ size,
-             const float* __restrict__ lacc, float* __restrict__ lacc_ref) {
+             const uint32_t* __restrict__ origin, const float* __restrict__ lacc,
+             float* __restrict__ lacc_ref) {
     __shared__ __align__(16) float rec[kIoBlock * kRecWords];
     const int r0 = blockIdx.x * kIoBlock;
     const int cnt = min(kIoBlock, n - r0);
@@ -294,7 +314,8 @@ __global__ void __launch_bounds__(kIoBlock)
         const int r = r0 + t;
         const uint32_t s = r2i[r];
         if (lacc_ref) lacc_ref[r] = lacc[s];
-        const float4 x = x4[s], v = v4[s], vs = vstar4[s], d = dp4[s], w = om4[s], c = col4[s];
+        const uint32_t from = origin[s];
+        const float4 x = x4[s], v = v4[s], vs = vstar4[s], d = dp4[s], w = om4[s], c = col4[from];
         float* o = rec + t * kRecWords;
         o[kPos] = x.x; o[kPos + 1] = x.y; o[kPos + 2] = x.z;
         o[kVel] = v.x; o[kVel + 1] = v.y; o[kVel + 2] = v.z;
@@ -307,7 +328,7 @@ __global__ void __launch_bounds__(kIoBlock)
         o[kLambda] = lam[s];
         o[kHash] = __uint_as_float(kr[r] - params_for(P, r).table_offset);  // the scene's own hash
         o[kColor] = c.x; o[kColor + 1] = c.y; o[kColor + 2] = c.z; o[kColor + 3] = c.w;
-        o[kSize] = size[s];
+        o[kSize] = size[from];
     }
     __syncthreads();
     if (stride == kRecWords * 4) {

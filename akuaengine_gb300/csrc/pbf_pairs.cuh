@@ -481,16 +481,15 @@ __device__ __forceinline__ void damp_plane(const StepParams& p, float px, float 
 // Last Jacobi iteration fused with update (IntegrationCUDA.cu:38-49) and boundary damping
 // (IntegrationCUDA.cu:75-102).  With `has_delta == 0` (zero iterations) the predicted positions
 // go straight to the update and the carried density/lambda/delta move into the state.  Also moves
-// the gathered colour, size and reference rank into the state arrays.
+// the gathered origin and reference rank into the state arrays.
 template <bool EXACT, int LANES>
 __global__ void __launch_bounds__(kMaxPairBlock)
     k_delta_final(const StepParams* __restrict__ P, const float4* __restrict__ ps_in,
                   const float* __restrict__ lam, const uint4* __restrict__ nbr4,
                   const uint32_t* __restrict__ cnt, const float4* __restrict__ x_old,
                   float4* __restrict__ x4, float4* __restrict__ v4, float4* __restrict__ vstar4,
-                  float4* __restrict__ dp4, const float4* __restrict__ col4g,
-                  const float* __restrict__ sizeg, float4* __restrict__ col4,
-                  float* __restrict__ size, const uint32_t* __restrict__ rref_new,
+                  float4* __restrict__ dp4, const uint32_t* __restrict__ origing,
+                  uint32_t* __restrict__ origin, const uint32_t* __restrict__ rref_new,
                   uint32_t* __restrict__ rref, const float* __restrict__ rho_c,
                   const float* __restrict__ lam_c, const float4* __restrict__ dp_c,
                   float* __restrict__ rho, float* __restrict__ lam_out, int has_delta,
@@ -554,8 +553,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     v4[i] = vn;
     xv8[2 * (size_t)i] = xn;  // (x, m | v) for vorticity's single gather
     xv8[2 * (size_t)i + 1] = vn;
-    col4[i] = col4g[i];
-    size[i] = sizeg[i];
+    origin[i] = origing[i];
     rref[i] = rref_new[i];
 }
 

@@ -1,8 +1,8 @@
 // Host side of the GB300 PBF step: device memory, the per-step launch sequence, CUDA-graph
 // capture and the C ABI declared in include/akua_pbf.h.
 //
-// One handle = one particle set on one device.  A step is [params] [import + sort keys, or the
-// keys alone when the state stayed on the device] and then the captured body: radix sort by
+// One handle = one particle set on one device.  A step is [a batch's params] [import + sort keys, or
+// the keys alone when the state stayed on the device] and then the captured body: radix sort by
 // (hash, previous reference rank) beside radix sort by Morton cell -> gather into the new internal
 // order -> bucket table -> neighbour walk (+ iteration 1 density/lambda) -> (delta+correct,
 // density+lambda) x iterations -> delta+update+damping -> vorticity -> confinement -> XSPH (which
@@ -55,9 +55,10 @@ struct akua_pbf {
     float *rho = nullptr, *lam = nullptr;
     float4* dp4 = nullptr;
     // gathered copies and per-step arrays
-    float4 *x4g = nullptr, *col4g = nullptr, *ps0 = nullptr, *ps1 = nullptr;
+    float4 *x4g = nullptr, *ps0 = nullptr, *ps1 = nullptr;
+    uint32_t *origin = nullptr, *origing = nullptr;  // a slot's colour and size: their import index
     float4 *vstar4 = nullptr, *om4 = nullptr, *xv8 = nullptr, *dpg = nullptr;
-    float *sizeg = nullptr, *rhog = nullptr, *lamg = nullptr;
+    float *rhog = nullptr, *lamg = nullptr;
     uint32_t *rrefg = nullptr, *rank_of_import = nullptr, *r2i = nullptr, *order = nullptr;
     // sorts: reference order (A) and Morton order (B)
     uint32_t *ka0 = nullptr, *va0 = nullptr, *ka1 = nullptr, *va1 = nullptr;
@@ -149,8 +150,8 @@ cudaError_t dalloc(akua_pbf* s, T** p, size_t count) {
 
 void free_all(akua_pbf* s) {
     void* ptrs[] = {s->d_params, s->x4, s->v4, s->col4, s->size, s->rref, s->rho, s->lam, s->dp4,
-                    s->x4g, s->col4g, s->ps0, s->ps1, s->vstar4, s->om4, s->xv8, s->dpg,
-                    s->sizeg, s->rhog, s->lamg, s->rrefg, s->rank_of_import, s->r2i, s->order,
+                    s->x4g, s->origin, s->origing, s->ps0, s->ps1, s->vstar4, s->om4, s->xv8, s->dpg,
+                    s->rhog, s->lamg, s->rrefg, s->rank_of_import, s->r2i, s->order,
                     s->ka0, s->va0, s->ka1, s->va1, s->kb0, s->vb0, s->kb1, s->vb1,
                     s->sort_scratch, s->sort_scratch_b, s->table, s->nbr, s->cnt, s->flags,
                     s->staging,
@@ -378,7 +379,7 @@ void enqueue_pairs(akua_pbf* s, cudaStream_t st, Marker& mark) {
         } else {
             akua::k_delta_final<EXACT, LANES><<<gp(2), pb[2], 0, st>>>(
                 s->d_params, cur, s->lam, nbr4, s->cnt, s->x4g, s->x4, s->v4, s->vstar4, s->dp4,
-                s->col4g, s->sizeg, s->col4, s->size, s->rrefg, s->rref, s->rhog, s->lamg, s->dpg,
+                s->origing, s->origin, s->rrefg, s->rref, s->rhog, s->lamg, s->dpg,
                 s->rho, nullptr, 1, s->psl, s->mass_bits, s->xv8);  // lam_out: zero iterations only
             mark("k_delta_final");
         }
@@ -386,7 +387,7 @@ void enqueue_pairs(akua_pbf* s, cudaStream_t st, Marker& mark) {
     if (iters == 0) {
         akua::k_delta_final<EXACT, LANES><<<gp(2), pb[2], 0, st>>>(
             s->d_params, s->ps0, nullptr, nbr4, s->cnt, s->x4g, s->x4, s->v4, s->vstar4, s->dp4,
-            s->col4g, s->sizeg, s->col4, s->size, s->rrefg, s->rref, s->rhog, s->lamg, s->dpg,
+            s->origing, s->origin, s->rrefg, s->rref, s->rhog, s->lamg, s->dpg,
             s->rho, s->lam, 0, s->psl, s->mass_bits, s->xv8);  // no delta: lambda is not read
         mark("k_delta_final");
     }
@@ -432,10 +433,9 @@ void enqueue_body(akua_pbf* s, cudaStream_t st, const char* aos, size_t stride, 
         cudaStreamWaitEvent(st, s->ev_join, 0);
         mark.launches += mark_b.launches;
     }
-    cudaMemsetAsync(s->mass_bits, 0, sizeof(uint32_t), st);  // "another mass seen" flag
     akua::k_gather<<<ge, akua::kElemBlock, 0, st>>>(
-        s->d_params, s->spperm, s->rank_of_import, s->x4, s->v4, s->col4, s->size, s->rref, s->x4g,
-        s->col4g, s->sizeg, s->ps0, s->r2i, s->rrefg, s->order, s->rho, s->lam, s->dp4, s->rhog,
+        s->d_params, s->spperm, s->rank_of_import, s->x4, s->v4, s->origin, s->rref, s->x4g,
+        s->origing, s->ps0, s->r2i, s->rrefg, s->order, s->rho, s->lam, s->dp4, s->rhog,
         s->lamg, s->dpg, carry ? 1 : 0, s->lacc, s->lprev,
         learn_mode(s) ? s->speed : nullptr, s->mass_bits);
     mark("k_gather");
@@ -455,7 +455,7 @@ void enqueue_body(akua_pbf* s, cudaStream_t st, const char* aos, size_t stride, 
     if (aos) {
         akua::k_export<<<grid_for(n, akua::kIoBlock), akua::kIoBlock, 0, st>>>(
             s->d_params, const_cast<char*>(aos), stride, n, s->r2i, s->kr, s->x4, s->v4, s->vstar4, s->dp4,
-            s->om4, s->rho, s->lam, s->col4, s->size, s->lacc,
+            s->om4, s->rho, s->lam, s->col4, s->size, s->origin, s->lacc,
             learn_mode(s) ? s->lacc_ref : nullptr);
         mark("k_export");
     }
@@ -530,21 +530,21 @@ int do_step(akua_pbf* s, const char* aos, size_t stride, bool force_import, floa
             s->prof_names[s->prof_next++] = nullptr;
         }
     }
-    if (!batch) {
-        akua::k_set_params<<<1, 32, 0, st>>>(p, s->d_params);
-    } else {
+    if (batch) {
         for (size_t k0 = 0; k0 < ps.size(); k0 += akua::kParamChunk) {
             akua::ParamChunk c;
             c.count = (int)std::min(ps.size() - k0, (size_t)akua::kParamChunk);
             for (int k = 0; k < c.count; ++k) c.p[k] = ps[k0 + k];
             akua::k_set_params_chunk<<<1, akua::kParamChunk, 0, st>>>(c, s->d_params + k0);
         }
+        mark("k_set_params");
     }
-    mark("k_set_params");
+    const akua::StepStart begin{p, s->d_params, s->mass_bits};
     const bool import = force_import || !(s->options & AKUA_PBF_OPT_RESIDENT) || !s->state_valid;
     if (import) {
-        akua::k_import<<<grid_for(s->n, akua::kIoBlock), akua::kIoBlock, 0, st>>>(
-            s->d_params, aos, stride, s->n, s->x4, s->v4, s->col4, s->size, s->rref, s->rho,
+        const auto kernel = batch ? akua::k_import<false> : akua::k_import<true>;
+        kernel<<<grid_for(s->n, akua::kIoBlock), akua::kIoBlock, 0, st>>>(
+            begin, aos, stride, s->n, s->x4, s->v4, s->col4, s->size, s->origin, s->rref, s->rho,
             s->lam, s->dp4, s->cfg.solverIterations == 0 ? 1 : 0, s->ka0, s->va0, s->kb0, s->vb0);
         mark("k_import");
         if (learn_mode(s)) {  // the previous step's lambda sums, in the records' order
@@ -554,8 +554,9 @@ int do_step(akua_pbf* s, const char* aos, size_t stride, bool force_import, floa
         }
     }
     if (!import) {  // the state is already on the device: only the sort keys
-        akua::k_keys<<<grid_for(s->n, akua::kElemBlock), akua::kElemBlock, 0, st>>>(
-            s->d_params, s->x4, s->v4, s->rref, s->ka0, s->va0, s->kb0, s->vb0);
+        const auto kernel = batch ? akua::k_keys<false> : akua::k_keys<true>;
+        kernel<<<grid_for(s->n, akua::kElemBlock), akua::kElemBlock, 0, st>>>(
+            begin, s->n, s->x4, s->v4, s->rref, s->ka0, s->va0, s->kb0, s->vb0);
         mark("k_keys");
     }
     cudaError_t e = cudaGetLastError();
@@ -668,11 +669,11 @@ int create_solver(int32_t n, const akua_pbf_config* cfg, const akua_lambda_corr_
     chk(dalloc(s, &s->x4, N)); chk(dalloc(s, &s->v4, N)); chk(dalloc(s, &s->col4, N));
     chk(dalloc(s, &s->size, N)); chk(dalloc(s, &s->rref, N));
     chk(dalloc(s, &s->rho, N)); chk(dalloc(s, &s->lam, N)); chk(dalloc(s, &s->dp4, N));
-    chk(dalloc(s, &s->x4g, N)); chk(dalloc(s, &s->col4g, N));
+    chk(dalloc(s, &s->x4g, N)); chk(dalloc(s, &s->origin, N)); chk(dalloc(s, &s->origing, N));
     chk(dalloc(s, &s->ps0, N)); chk(dalloc(s, &s->ps1, N));
     chk(dalloc(s, &s->vstar4, N)); chk(dalloc(s, &s->om4, N)); chk(dalloc(s, &s->xv8, 2 * N));
     chk(dalloc(s, &s->dpg, N));
-    chk(dalloc(s, &s->sizeg, N)); chk(dalloc(s, &s->rhog, N)); chk(dalloc(s, &s->lamg, N));
+    chk(dalloc(s, &s->rhog, N)); chk(dalloc(s, &s->lamg, N));
     chk(dalloc(s, &s->rrefg, N)); chk(dalloc(s, &s->rank_of_import, N)); chk(dalloc(s, &s->r2i, N));
     chk(dalloc(s, &s->order, N));
     chk(dalloc(s, &s->ka0, N)); chk(dalloc(s, &s->va0, N));
@@ -945,7 +946,7 @@ int akua_pbf_read_debug(akua_pbf* s, int32_t what, void* dst, size_t bytes) {
         }
         akua::k_export<<<grid_for(s->n, akua::kIoBlock), akua::kIoBlock, 0, s->stream>>>(
             s->d_params, tmp, sizeof(akua_particle), s->n, s->r2i, s->kr, s->x4, s->v4, s->vstar4, s->dp4,
-            s->om4, s->rho, s->lam, s->col4, s->size, nullptr, nullptr);
+            s->om4, s->rho, s->lam, s->col4, s->size, s->origin, nullptr, nullptr);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(dst, tmp, need, cudaMemcpyDeviceToHost, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
@@ -979,9 +980,8 @@ int akua_pbf_read_debug(akua_pbf* s, int32_t what, void* dst, size_t bytes) {
 int akua_pbf_kernels_per_step(akua_pbf* s) {
     if (!s) return AKUA_ERR_INVALID_ARGUMENT;
     if (s->body_launches == 0) return AKUA_ERR_INVALID_ARGUMENT;  // no step issued yet
-    // parameter upload (one launch per chunk of scenes) + import or the sort keys + the body
-    const int uploads =
-        s->scenes.empty() ? 1 : (int)((s->scenes.size() + akua::kParamChunk - 1) / akua::kParamChunk);
+    // a batch's parameter upload (one launch per chunk of scenes) + import or the sort keys + body
+    const int uploads = (int)((s->scenes.size() + akua::kParamChunk - 1) / akua::kParamChunk);
     return uploads + 1 + s->body_launches;
 }
 

@@ -48,16 +48,15 @@ WORKLOAD = "dam_break_1m"
 # the mean bytes of one particle's list tiles (16 * ceil(count / 4)), `B` the mean number of bucket
 # table entries per particle (one 8-byte entry per occupied bucket), both taken from the run.
 KERNEL_BYTES = {
-    # R record 108; W x|m, v, colour, size, rank, hash key and Morton key with their payloads
-    "k_import": lambda L, B: 108 + 16 + 16 + 16 + 4 + 4 + 16,
+    # R record 108; W x|m, v, colour, size, origin, rank, hash key and Morton key with their payloads
+    "k_import": lambda L, B: 108 + 16 + 16 + 16 + 4 + 4 + 4 + 16,
     # R x|m, v, rank; W hash key, index, Morton key
     "k_keys": lambda L, B: 16 + 16 + 4 + 16,
     "radix_upsweep": lambda L, B: 4,                  # R key (per pass)
     "radix_downsweep": lambda L, B: 16,               # R key, value; W key, value (per pass)
     "radix_cluster_pass": lambda L, B: 16,            # the same, histogram and scan included
-    # R two permutations, x|m, v, colour, size, old rank; W x|m, colour, size, x*|m, rank->slot,
-    # slot->rank, order
-    "k_gather": lambda L, B: 8 + 16 + 16 + 16 + 4 + 4 + 16 + 16 + 4 + 16 + 4 + 4 + 4,
+    # R two permutations, x|m, v, origin, old rank; W x|m, origin, x*|m, rank->slot, slot->rank, order
+    "k_gather": lambda L, B: 8 + 16 + 16 + 4 + 4 + 16 + 4 + 16 + 4 + 4 + 4,
     "k_table_build": lambda L, B: 4 + 4 + 8 * B,      # R keys, slots; W entry
     # R x*|m, 27 bucket entries per cell run; W lists, count, rho, lambda, x*|lambda
     "k_search": lambda L, B: 16 + 27 * 8 * B + L + 4 + 8 + 16,
@@ -65,16 +64,16 @@ KERNEL_BYTES = {
     "k_density_lambda": lambda L, B: 16 + 4 + L + 8 + 16,
     # R x*|m, lambda, count, lists; W x*|m, delta
     "k_delta_correct": lambda L, B: 16 + 4 + 4 + L + 16 + 16,
-    # R x*|m, lambda, count, lists, x|m, colour, size, rank; W x, v, v*, delta, colour, size, rank,
+    # R x*|m, lambda, count, lists, x|m, origin, rank; W x, v, v*, delta, origin, rank,
     # record (x|m, v)
-    "k_delta_final": lambda L, B: 16 + 4 + 4 + L + 16 + 16 + 4 + 4 + 16 * 4 + 16 + 4 + 4 + 32,
+    "k_delta_final": lambda L, B: 16 + 4 + 4 + L + 16 + 4 + 4 + 16 * 4 + 4 + 4 + 32,
     "k_vorticity": lambda L, B: 16 + 16 + 4 + L + 16 + 16,   # R x, v, count, lists; W omega, x|omega
     # R x, v, omega, rho, count, lists; W record (x|m/rho, v)
     "k_confine": lambda L, B: 16 + 16 + 16 + 4 + 4 + L + 32,
     # R record, count, lists, keys; W v, emptied bucket entries
     "k_xsph": lambda L, B: 32 + 4 + L + 16 + 4 + 8 * B,
-    # R slot, key, x, v, v*, delta, omega, colour, rho, lambda, size; W record 108
-    "k_export": lambda L, B: 4 + 4 + 16 * 6 + 4 + 4 + 4 + 108,
+    # R slot, key, origin, x, v, v*, delta, omega, colour, rho, lambda, size; W record 108
+    "k_export": lambda L, B: 4 + 4 + 4 + 16 * 6 + 4 + 4 + 4 + 108,
 }
 
 
