@@ -474,7 +474,10 @@ void update_plans(akua_pbf* s, int sp_bits) {
     // one scene of few particles: a pass is one cluster; a batch holds many scenes' particles
     const bool small = s->scenes.empty() && s->n <= akua::radix::kClusterMax;
     auto plan = [&](int bits) {
-        return small ? akua::radix::make_cluster_plan(bits) : akua::radix::make_plan(bits);
+        if (small) return akua::radix::make_cluster_plan(bits);
+        akua::radix::Plan p = akua::radix::make_plan(bits);
+        p.fused = s->scenes.empty() && akua::radix::num_tiles(s->n) <= akua::radix::kFusedTiles;
+        return p;
     };
     s->plan_ref = plan(akua::radix::bits_for(s->table_size));
     s->sp_bits = sp_bits;

@@ -7,8 +7,8 @@
 // the reference's merge sort yields for equal hashes.
 //
 // A sort of `bits`-bit keys runs ceil(bits / 10) passes of equal digit width (8..10 bits).  Each
-// pass: per-tile digit counts (also accumulated into per-digit totals), one block per digit that
-// turns its row of the (digit, tile) count matrix into global offsets, and a stable scatter in
+// pass: per-tile digit counts, a scan of the (tile, digit) count matrix over the tiles (for inputs of
+// few tiles in the scatter itself), and a stable scatter in
 // which warps rank their keys by ballots and per-warp running digit counters, order the tile in
 // shared memory and store it in runs.  Inputs of at most kClusterMax pairs take one launch per pass.
 #pragma once
@@ -26,14 +26,17 @@ constexpr int WARPS = BLOCK / 32;
 constexpr int ROUNDS = 16;                // keys per lane
 constexpr int WARP_ITEMS = ROUNDS * 32;   // 512
 constexpr int TILE = WARPS * WARP_ITEMS;  // 4096 keys per tile
-constexpr int SCAN_BLOCK = 256;
 constexpr int MAX_PASSES = 4;
+// Tiles up to which the scatters add up the counts themselves.  Three passes in us without and with
+// the scan's launch: 100,000 keys 27 / 32, 262,144 (64 tiles) 33 / 37, 300,000 40 / 36.
+constexpr int kFusedTiles = 64;
 
 inline int num_tiles(int n) { return (n + TILE - 1) / TILE; }
 
 // Digit width per pass for keys of `bits` significant bits.
 struct Plan {
     bool cluster = false;  // passes of one cluster each (make_cluster_plan)
+    bool fused = false;    // the scatters scan the counts themselves (at most kFusedTiles tiles)
     int passes = 0;
     int width[MAX_PASSES] = {0, 0, 0, 0};
     int shift[MAX_PASSES] = {0, 0, 0, 0};
@@ -78,12 +81,14 @@ __device__ __forceinline__ uint32_t same_digit(uint32_t digit, bool live) {
     return peers;
 }
 
-// counts[d * tiles + tile] = keys of `tile` with digit d; totals[d] += the same.  A key's digit
-// is (key >> shift) & digit_mask; digit_mask < RADIX narrows a pass to fewer bits than BITS.
+// counts[tile * RADIX + d] = keys of `tile` with digit d.  A key's digit is (key >> shift) &
+// digit_mask; digit_mask < RADIX narrows a pass to fewer bits than BITS.  (One row per tile: stores
+// and the scatter's reads are contiguous.  One row per digit, with the digits' totals added up by
+// atomics, cost 26 us against 12 over 8M keys and 54 against 48 for three passes over 2^20.)
 template <int BITS>
 __global__ void __launch_bounds__(BLOCK) upsweep(const uint32_t* __restrict__ keys, int n, int shift,
-                                                 uint32_t digit_mask, uint32_t* __restrict__ counts,
-                                                 uint32_t* __restrict__ totals, int tiles) {
+                                                 uint32_t digit_mask,
+                                                 uint32_t* __restrict__ counts) {
     constexpr int RADIX = 1 << BITS;
     __shared__ uint32_t hist[WARPS][RADIX];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -104,51 +109,50 @@ __global__ void __launch_bounds__(BLOCK) upsweep(const uint32_t* __restrict__ ke
         uint32_t s = 0;
 #pragma unroll
         for (int w = 0; w < WARPS; ++w) s += hist[w][d];
-        counts[(size_t)d * tiles + blockIdx.x] = s;
-        if (s) atomicAdd(&totals[d], s);
+        counts[(size_t)blockIdx.x * RADIX + d] = s;
     }
 }
 
-// Block d: offsets[d][t] = sum of totals[0..d) + sum of counts[d][0..t).
-__global__ void __launch_bounds__(SCAN_BLOCK) scan_rows(uint32_t* __restrict__ counts,
-                                                        const uint32_t* __restrict__ totals,
-                                                        int tiles) {
-    __shared__ uint32_t red[SCAN_BLOCK / 32];
-    __shared__ uint32_t carry_s;
-    const int d = blockIdx.x;
+// counts[t][d] becomes the sum of counts[0..t)[d], totals[d] the sum over all tiles.  A block takes 8
+// digits (one 32-byte sector of a row), its warps a run of tiles each, a quarter of the run per lane.
+constexpr int SCAN_WARPS = 32;
+constexpr int SCAN_DIGITS = 8;
+template <int BITS>
+__global__ void __launch_bounds__(32 * SCAN_WARPS)
+    scan_tiles(uint32_t* __restrict__ counts, uint32_t* __restrict__ totals, int tiles) {
+    constexpr int RADIX = 1 << BITS;
+    constexpr int PARTS = 32 / SCAN_DIGITS;
+    __shared__ uint32_t sums[SCAN_WARPS][SCAN_DIGITS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t part = 0;
-    for (int k = threadIdx.x; k < d; k += SCAN_BLOCK) part += totals[k];
+    const int digit = lane % SCAN_DIGITS, part = lane / SCAN_DIGITS;
+    const int per = (tiles + SCAN_WARPS * PARTS - 1) / (SCAN_WARPS * PARTS);
+    const int t0 = min((warp * PARTS + part) * per, tiles), t1 = min(t0 + per, tiles);
+    uint32_t* col = counts + blockIdx.x * SCAN_DIGITS + digit;
+    uint32_t sum = 0;
+#pragma unroll 8
+    for (int t = t0; t < t1; ++t) sum += col[(size_t)t * RADIX];
+    uint32_t run = 0, warp_sum = 0;  // the lower parts of this warp's run, and all of it
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) red[warp] = part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t b = 0;
-        for (int w = 0; w < SCAN_BLOCK / 32; ++w) b += red[w];
-        carry_s = b;
+    for (int q = 0; q < PARTS; ++q) {
+        const uint32_t c = __shfl_sync(0xffffffffu, sum, q * SCAN_DIGITS + digit);
+        run += q < part ? c : 0u;
+        warp_sum += c;
     }
+    if (part == 0) sums[warp][digit] = warp_sum;
     __syncthreads();
-    uint32_t* row = counts + (size_t)d * tiles;
-    for (int chunk = 0; chunk < tiles; chunk += SCAN_BLOCK) {
-        const int t = chunk + threadIdx.x;
-        const uint32_t v = t < tiles ? row[t] : 0u;
-        uint32_t incl = v;
+    uint32_t all = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        __syncthreads();  // red[] reuse
-        if (lane == 31) red[warp] = incl;
-        __syncthreads();
-        uint32_t wpre = 0;
-        for (int w = 0; w < warp; ++w) wpre += red[w];
-        const uint32_t carry = carry_s;
-        if (t < tiles) row[t] = carry + wpre + incl - v;
-        __syncthreads();
-        if (threadIdx.x == SCAN_BLOCK - 1) carry_s = carry + wpre + incl;
-        __syncthreads();
+    for (int w = 0; w < SCAN_WARPS; ++w) {
+        const uint32_t c = sums[w][digit];
+        run += w < warp ? c : 0u;
+        all += c;
+    }
+    if (warp == 0 && part == 0) totals[blockIdx.x * SCAN_DIGITS + digit] = all;
+#pragma unroll 8
+    for (int t = t0; t < t1; ++t) {
+        const uint32_t c = col[(size_t)t * RADIX];
+        col[(size_t)t * RADIX] = run;
+        run += c;
     }
 }
 
@@ -184,14 +188,17 @@ __host__ __device__ constexpr size_t scatter_smem(int warps, int radix, int pair
 // consecutive addresses: an SM issues one 32-byte sector per two cycles, and pairs stored straight
 // from their input order touch one each.
 // 2^20 random pairs of 27 bits, three passes: 92 -> 54 us (with the upsweep's loads and the ballots,
-// 73 without the ordering); a pass over 8M particles' keys 73 -> 58 us, over 1M 13.3 -> 13.5 (their
+// 73 without the ordering); a pass over 8M particles' keys 73 -> 53 us, over 1M 13.3 -> 13.5 (their
 // runs of equal keys make short runs of stores by themselves).
-template <int BITS>
-__global__ void __launch_bounds__(BLOCK)
+// FUSED: `counts` holds the tiles' counts themselves and every block adds up what it needs; there are
+// then few blocks, and all the registers they ask for are theirs (three blocks per SM otherwise: a
+// pass over 8M particles' keys 53 us, with two 58, with one 88).
+template <int BITS, bool FUSED>
+__global__ void __launch_bounds__(BLOCK, FUSED ? 1 : 3)
     downsweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
               uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n, int shift,
-              uint32_t digit_mask, const uint32_t* __restrict__ offsets, int tiles,
-              uint32_t* __restrict__ rank_out) {
+              uint32_t digit_mask, const uint32_t* __restrict__ counts,
+              const uint32_t* __restrict__ totals, int tiles, uint32_t* __restrict__ rank_out) {
     constexpr int RADIX = 1 << BITS;
     constexpr int PER = RADIX / BLOCK;  // digits per thread in the scan
     static_assert(RADIX % BLOCK == 0, "the scan gives every thread the same number of digits");
@@ -215,10 +222,26 @@ __global__ void __launch_bounds__(BLOCK)
         key[r] = valid ? keys_in[idx] : 0u;
         val[r] = valid ? (vals_in ? vals_in[idx] : (uint32_t)idx) : 0u;
     }
-    uint32_t first[PER];  // this thread's digits: output position of the tile's first key
+    // this thread's digits: the keys of the tiles before this one, and of all
+    uint32_t first[PER], all[PER];
+    if (FUSED) {
 #pragma unroll
-    for (int k = 0; k < PER; ++k)
-        first[k] = offsets[(size_t)(threadIdx.x * PER + k) * tiles + blockIdx.x];
+        for (int k = 0; k < PER; ++k) first[k] = all[k] = 0u;
+#pragma unroll 8
+        for (int t = 0; t < tiles; ++t)
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const uint32_t c = counts[(size_t)t * RADIX + threadIdx.x * PER + k];
+                first[k] += t < (int)blockIdx.x ? c : 0u;
+                all[k] += c;
+            }
+    } else {
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            first[k] = counts[(size_t)blockIdx.x * RADIX + threadIdx.x * PER + k];
+            all[k] = totals[threadIdx.x * PER + k];
+        }
+    }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
@@ -247,12 +270,18 @@ __global__ void __launch_bounds__(BLOCK)
         mine[k] = run;
         total += run;
     }
+    uint32_t below = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) below += all[k];
     uint32_t at = block_exclusive<WARPS>(total, sums);
+    __syncthreads();  // `sums` again
+    below = block_exclusive<WARPS>(below, sums);  // the keys of all lower digits
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
         start[threadIdx.x * PER + k] = at;
-        to[threadIdx.x * PER + k] = first[k] - at;
+        to[threadIdx.x * PER + k] = below + first[k] - at;
         at += mine[k];
+        below += all[k];
     }
     __syncthreads();
 #pragma unroll
@@ -280,19 +309,27 @@ __global__ void __launch_bounds__(BLOCK)
 }
 
 // One pass over the digit (key >> shift) & digit_mask; digit_mask defaults to all BITS bits.
+// `fused`: no scan launch, for inputs of few tiles (the scatters then read tiles x tiles rows).
 template <int BITS, class Mark>
 inline void run_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                      uint32_t* vout, uint32_t* counts, uint32_t* totals, int n, int shift,
-                     uint32_t* rank_out, Mark& mark, uint32_t digit_mask = (1u << BITS) - 1u) {
+                     uint32_t* rank_out, Mark& mark, bool fused,
+                     uint32_t digit_mask = (1u << BITS) - 1u) {
     const int tiles = num_tiles(n);
     constexpr int RADIX = 1 << BITS;
+    constexpr size_t smem = scatter_smem(WARPS, RADIX, TILE);
     digit_mask &= RADIX - 1;  // the kernels' shared-memory tables hold RADIX digits
-    upsweep<BITS><<<tiles, BLOCK, 0, s>>>(kin, n, shift, digit_mask, counts, totals, tiles);
+    upsweep<BITS><<<tiles, BLOCK, 0, s>>>(kin, n, shift, digit_mask, counts);
     mark("radix_upsweep");
-    scan_rows<<<RADIX, SCAN_BLOCK, 0, s>>>(counts, totals, tiles);
-    mark("radix_scan");
-    downsweep<BITS><<<tiles, BLOCK, scatter_smem(WARPS, RADIX, TILE), s>>>(
-        kin, vin, kout, vout, n, shift, digit_mask, counts, tiles, rank_out);
+    if (!fused) {
+        scan_tiles<BITS><<<RADIX / SCAN_DIGITS, 32 * SCAN_WARPS, 0, s>>>(counts, totals, tiles);
+        mark("radix_scan");
+        downsweep<BITS, false><<<tiles, BLOCK, smem, s>>>(kin, vin, kout, vout, n, shift, digit_mask,
+                                                          counts, totals, tiles, rank_out);
+    } else {
+        downsweep<BITS, true><<<tiles, BLOCK, smem, s>>>(kin, vin, kout, vout, n, shift, digit_mask,
+                                                         counts, nullptr, tiles, rank_out);
+    }
     mark("radix_downsweep");
 }
 
@@ -460,9 +497,9 @@ inline void run_cluster_pass(cudaStream_t s, const uint32_t* kin, const uint32_t
     mark("radix_cluster_pass");
 }
 
-// Scratch words the sort needs for n keys: the count matrix plus per-pass digit totals.
+// Scratch words the sort needs for n keys: the count matrix and a pass's digit totals.
 inline size_t scratch_words(int n) {
-    return (size_t)MAX_RADIX * num_tiles(n) + (size_t)MAX_PASSES * MAX_RADIX;
+    return (size_t)MAX_RADIX * num_tiles(n) + MAX_RADIX;
 }
 
 // Sorts (k0, v0) by the low plan bits (a cluster plan: n <= kClusterMax), ping-ponging with (k1, v1); all four buffers hold n words.
@@ -476,13 +513,11 @@ inline void sort_pairs(cudaStream_t s, const Plan& plan, uint32_t* k0, uint32_t*
                        uint32_t* rank_out = nullptr) {
     uint32_t* counts = scratch;
     uint32_t* totals = scratch + (size_t)MAX_RADIX * num_tiles(n);
-    if (!plan.cluster) cudaMemsetAsync(totals, 0, sizeof(uint32_t) * MAX_PASSES * MAX_RADIX, s);
     const uint32_t* kin = k0;
     const uint32_t* vin = index_payload ? nullptr : v0;
     uint32_t* kout = k1;
     uint32_t* vout = v1;
     for (int p = 0; p < plan.passes; ++p) {
-        uint32_t* tot = totals + (size_t)p * MAX_RADIX;
         const bool last = p + 1 == plan.passes;
         // a digit narrower than 8 bits only occurs in the last pass, where the key's higher
         // bits are zero, so the 8-bit kernel sorts it correctly
@@ -490,11 +525,14 @@ inline void sort_pairs(cudaStream_t s, const Plan& plan, uint32_t* k0, uint32_t*
             run_cluster_pass<true>(s, kin, vin, kout, vout, n, plan.shift[p], plan.width[p],
                              last ? rank_out : nullptr, mark);
         else if (plan.width[p] <= 8)
-            run_pass<8>(s, kin, vin, kout, vout, counts, tot, n, plan.shift[p], last ? rank_out : nullptr, mark);
+            run_pass<8>(s, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
+                        last ? rank_out : nullptr, mark, plan.fused);
         else if (plan.width[p] == 9)
-            run_pass<9>(s, kin, vin, kout, vout, counts, tot, n, plan.shift[p], last ? rank_out : nullptr, mark);
+            run_pass<9>(s, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
+                        last ? rank_out : nullptr, mark, plan.fused);
         else
-            run_pass<10>(s, kin, vin, kout, vout, counts, tot, n, plan.shift[p], last ? rank_out : nullptr, mark);
+            run_pass<10>(s, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
+                        last ? rank_out : nullptr, mark, plan.fused);
         if (kout == k1) {
             kin = k1; vin = v1; kout = k0; vout = v0;
         } else {

@@ -27,9 +27,9 @@ namespace {
 
 constexpr int kMaxPairs = AKUA_SORT_NOALLOC_MAX_PAIRS;
 constexpr size_t kTiles = ((size_t)kMaxPairs + akua::radix::TILE - 1) / akua::radix::TILE;
-// one ping-pong buffer of keys and values, the (digit, tile) count matrix, per-pass digit totals
+// one ping-pong buffer of keys and values, the (tile, digit) count matrix, a pass's digit totals
 constexpr size_t kCountWords =
-    (size_t)akua::radix::MAX_RADIX * kTiles + (size_t)akua::radix::MAX_PASSES * akua::radix::MAX_RADIX;
+    (size_t)akua::radix::MAX_RADIX * kTiles + akua::radix::MAX_RADIX;
 constexpr size_t kScratchWords = 2 * (size_t)kMaxPairs + kCountWords;
 
 struct NoMark {
@@ -100,12 +100,7 @@ extern "C" int akua_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* 
     const akua::radix::Plan plan = n <= akua::radix::kClusterMax
                                        ? akua::radix::make_cluster_plan(key_bits)
                                        : akua::radix::make_plan(key_bits);
-    if (!plan.cluster) {
-        // the digit totals accumulate atomically and must start at zero on every call
-        e = cudaMemsetAsync(totals, 0,
-                            sizeof(uint32_t) * akua::radix::MAX_PASSES * akua::radix::MAX_RADIX, st);
-        if (e != cudaSuccess) return AKUA_ERR_CUDA;
-    }
+    const bool fused = akua::radix::num_tiles(n) <= akua::radix::kFusedTiles;
     NoMark mark;
     // pass p writes to the caller's output when (passes - 1 - p) is even, so the last pass does
     const uint32_t* kin = keys_in;
@@ -114,7 +109,6 @@ extern "C" int akua_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* 
         const bool to_out = ((plan.passes - 1 - p) & 1) == 0;
         uint32_t* kout = to_out ? keys_out : tmp_keys;
         uint32_t* vout = to_out ? vals_out : tmp_vals;
-        uint32_t* tot = totals + (size_t)p * akua::radix::MAX_RADIX;
         // the digit covers only this pass's bits, so key bits at and above key_bits never
         // influence the order (a pass narrower than 8 bits still runs the 8-bit kernels)
         const uint32_t mask = (1u << plan.width[p]) - 1u;
@@ -122,14 +116,14 @@ extern "C" int akua_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* 
             akua::radix::run_cluster_pass<false>(st, kin, vin, kout, vout, n, plan.shift[p], plan.width[p],
                                           nullptr, mark);
         else if (plan.width[p] <= 8)
-            akua::radix::run_pass<8>(st, kin, vin, kout, vout, counts, tot, n, plan.shift[p],
-                                      nullptr, mark, mask);
+            akua::radix::run_pass<8>(st, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
+                                      nullptr, mark, fused, mask);
         else if (plan.width[p] == 9)
-            akua::radix::run_pass<9>(st, kin, vin, kout, vout, counts, tot, n, plan.shift[p],
-                                      nullptr, mark, mask);
+            akua::radix::run_pass<9>(st, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
+                                      nullptr, mark, fused, mask);
         else
-            akua::radix::run_pass<10>(st, kin, vin, kout, vout, counts, tot, n, plan.shift[p],
-                                      nullptr, mark, mask);
+            akua::radix::run_pass<10>(st, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
+                                      nullptr, mark, fused, mask);
         kin = kout;
         vin = vout;
     }
