@@ -76,6 +76,12 @@ struct StepParams {
     float sdf_stiffness;
 };
 
+// Programmatic dependent launch: the step's kernels are set up while the one before them ends, and
+// wait here for its stores.
+__device__ __forceinline__ void after_previous_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // The parameters of the scene particle (or reference rank, or internal slot) i belongs to.
 __device__ __forceinline__ const StepParams& params_for(const StepParams* P, int i) {
     const uint16_t* sid = P->scene_of;

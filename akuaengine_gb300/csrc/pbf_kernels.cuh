@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(kElemBlock)
                   const uint32_t* __restrict__ r2i, uint2* __restrict__ table) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = P->n;
+    after_previous_kernel();
     if (r >= n) return;
     const uint32_t k = kr[r];
     if (r > 0 && kr[r - 1] == k) return;
@@ -310,6 +311,7 @@ __global__ void __launch_bounds__(kIoBlock)
     const int r0 = blockIdx.x * kIoBlock;
     const int cnt = min(kIoBlock, n - r0);
     const int t = threadIdx.x;
+    after_previous_kernel();
     if (t < cnt) {
         const int r = r0 + t;
         const uint32_t s = r2i[r];

@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
+    after_previous_kernel();
     const float4 xi = ps[i];
     DensityLambda2<EXACT> acc;
     acc.init(xi.w, p);
@@ -444,6 +445,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(P->n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
+    after_previous_kernel();
     const float4 xi = ps_in[i];
     const float3 d = delta_of<EXACT, LANES>(p, i, xi, ps_in, lam, psl, mass_bits, nbr4,
                                             live ? (int)cnt[i] : 0);
@@ -499,6 +501,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(P->n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
+    after_previous_kernel();
     const float4 xi = ps_in[i];
     float nx = xi.x, ny = xi.y, nz = xi.z;
     float3 d = make_float3(0.f, 0.f, 0.f);
@@ -570,6 +573,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
+    after_previous_kernel();
     const float4 xi = x4[i], vi = v4[i];
     Sum3 w;
     auto load = [&](uint32_t j) { return ld_rec8(xv8, j); };
@@ -615,6 +619,7 @@ __global__ void __launch_bounds__(kMaxPairBlock, LANES == 1 ? 5 : 1)
     const bool live = particle_of_thread<LANES>(n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
+    after_previous_kernel();
     const float4 xi = x4[i], vi = v4[i], wi = om4[i];
     const float rho_i = rho[i];
     const int c = live ? (int)cnt[i] : 0;
@@ -679,13 +684,14 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     int i;
     const bool live = particle_of_thread<LANES>(n, i);
     if (LANES == 1 && !live) return;
+    const StepParams& p = params_for(P, i);
+    after_previous_kernel();
     if (writes<LANES>(live)) {
         // the walk is done: empty this step's bucket entries (particle i: the bucket starting at
         // rank i)
         const uint32_t k = kr[i];
         if (i == 0 || kr[i - 1] != k) table[k] = make_uint2(0u, 0u);
     }
-    const StepParams& p = params_for(P, i);
     const Rec8 ri = ld_rec8(xv8, (uint32_t)i);
     const float4 xi = ri.x, vi = ri.v;
     Sum3 sum;

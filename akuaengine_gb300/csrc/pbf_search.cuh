@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
     const float4* pair_xy = reinterpret_cast<const float4*>(pairs);  // (xa, xb, ya, yb)
     const float2* pair_z = reinterpret_cast<const float2*>(pairs + 64);
 
+    after_previous_kernel();
     const float4 xi = valid ? ps[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int cx = cell_coord(xi.x, p.search_cell);
     const int cy = cell_coord(xi.y, p.search_cell);

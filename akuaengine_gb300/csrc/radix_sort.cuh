@@ -81,6 +81,29 @@ __device__ __forceinline__ uint32_t same_digit(uint32_t digit, bool live) {
     return peers;
 }
 
+// Programmatic dependent launch: a kernel launched with `after` is set up while the stream's previous
+// kernel ends, and waits here for its stores.  No kernel lets the next one start before its own
+// blocks are done: blocks that wait take the room of blocks that work (2^20 pairs launched one by
+// one: 68 us without, 58 with an early start, 47 like this; replayed from a graph 48, 55, 46).
+__device__ __forceinline__ void wait_for_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... Params, class... Args>
+inline void launch(bool after, void (*kernel)(Params...), int grid, int block, size_t smem,
+                   cudaStream_t st, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = after ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // counts[tile * RADIX + d] = keys of `tile` with digit d.  A key's digit is (key >> shift) &
 // digit_mask; digit_mask < RADIX narrows a pass to fewer bits than BITS.  (One row per tile: stores
 // and the scatter's reads are contiguous.  One row per digit, with the digits' totals added up by
@@ -94,6 +117,7 @@ __global__ void __launch_bounds__(BLOCK) upsweep(const uint32_t* __restrict__ ke
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int t = threadIdx.x; t < WARPS * RADIX; t += BLOCK) (&hist[0][0])[t] = 0;
     __syncthreads();
+    wait_for_previous();
     const int base = blockIdx.x * TILE + warp * WARP_ITEMS + lane;
     uint32_t key[ROUNDS];  // all loads in flight at once: 14.4 -> 8.8 us at 1M, launch included
 #pragma unroll
@@ -128,6 +152,7 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS)
     const int per = (tiles + SCAN_WARPS * PARTS - 1) / (SCAN_WARPS * PARTS);
     const int t0 = min((warp * PARTS + part) * per, tiles), t1 = min(t0 + per, tiles);
     uint32_t* col = counts + blockIdx.x * SCAN_DIGITS + digit;
+    wait_for_previous();
     uint32_t sum = 0;
 #pragma unroll 8
     for (int t = t0; t < t1; ++t) sum += col[(size_t)t * RADIX];
@@ -213,6 +238,7 @@ __global__ void __launch_bounds__(BLOCK, FUSED ? 1 : 3)
     for (int t = threadIdx.x; t < WARPS * RADIX; t += BLOCK) (&count[0][0])[t] = 0;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const int tile0 = blockIdx.x * TILE;
+    wait_for_previous();
     const int base = tile0 + warp * WARP_ITEMS + lane;
     uint32_t key[ROUNDS], val[ROUNDS], pos[ROUNDS];
 #pragma unroll
@@ -309,25 +335,25 @@ __global__ void __launch_bounds__(BLOCK, FUSED ? 1 : 3)
 }
 
 // One pass over the digit (key >> shift) & digit_mask; digit_mask defaults to all BITS bits.
-// `fused`: no scan launch, for inputs of few tiles (the scatters then read tiles x tiles rows).
+// `after`: the stream's previous kernel is this sort's previous pass.  `fused`: no scan launch, for inputs of few tiles (the scatters then read tiles x tiles rows).
 template <int BITS, class Mark>
 inline void run_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                      uint32_t* vout, uint32_t* counts, uint32_t* totals, int n, int shift,
-                     uint32_t* rank_out, Mark& mark, bool fused,
+                     uint32_t* rank_out, Mark& mark, bool fused, bool after,
                      uint32_t digit_mask = (1u << BITS) - 1u) {
     const int tiles = num_tiles(n);
     constexpr int RADIX = 1 << BITS;
     constexpr size_t smem = scatter_smem(WARPS, RADIX, TILE);
     digit_mask &= RADIX - 1;  // the kernels' shared-memory tables hold RADIX digits
-    upsweep<BITS><<<tiles, BLOCK, 0, s>>>(kin, n, shift, digit_mask, counts);
+    launch(after, upsweep<BITS>, tiles, BLOCK, 0, s, kin, n, shift, digit_mask, counts);
     mark("radix_upsweep");
     if (!fused) {
-        scan_tiles<BITS><<<RADIX / SCAN_DIGITS, 32 * SCAN_WARPS, 0, s>>>(counts, totals, tiles);
+        launch(true, scan_tiles<BITS>, RADIX / SCAN_DIGITS, 32 * SCAN_WARPS, 0, s, counts, totals, tiles);
         mark("radix_scan");
-        downsweep<BITS, false><<<tiles, BLOCK, smem, s>>>(kin, vin, kout, vout, n, shift, digit_mask,
+        launch(true, downsweep<BITS, false>, tiles, BLOCK, smem, s, kin, vin, kout, vout, n, shift, digit_mask,
                                                           counts, totals, tiles, rank_out);
     } else {
-        downsweep<BITS, true><<<tiles, BLOCK, smem, s>>>(kin, vin, kout, vout, n, shift, digit_mask,
+        launch(true, downsweep<BITS, true>, tiles, BLOCK, smem, s, kin, vin, kout, vout, n, shift, digit_mask,
                                                          counts, nullptr, tiles, rank_out);
     }
     mark("radix_downsweep");
@@ -398,6 +424,7 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kCluste
     const int first = (int)rank * kPer + warp * (32 * ROUNDS) + lane;
     const uint32_t below = (1u << lane) - 1u;
     uint32_t key[ROUNDS], val[ROUNDS], pos[ROUNDS];
+    wait_for_previous();
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
         const int at = first + 32 * r;
@@ -479,15 +506,15 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kCluste
 template <bool RUNS, class Mark>
 inline void run_cluster_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                              uint32_t* vout, int n, int shift, int width, uint32_t* rank_out,
-                             Mark& mark) {
+                             Mark& mark, bool after) {
     constexpr int kRound = kClusterBlocks * kClusterThreads;
     const uint32_t mask = (1u << width) - 1u;
     auto go = [&](auto kernel, int rounds) {
         const size_t smem = scatter_smem(kClusterWarps, kClusterRadix, kClusterThreads * rounds);
         if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kernel<<<kClusterBlocks, kClusterThreads, smem, s>>>(kin, vin, kout, vout, n, shift, mask,
-                                                             rank_out);
+        launch(after, kernel, kClusterBlocks, kClusterThreads, smem, s, kin, vin, kout, vout, n, shift,
+               mask, rank_out);
     };
     if (n <= kRound) go(cluster_pass<1, RUNS>, 1);
     else if (n <= 2 * kRound) go(cluster_pass<2, RUNS>, 2);
@@ -523,16 +550,16 @@ inline void sort_pairs(cudaStream_t s, const Plan& plan, uint32_t* k0, uint32_t*
         // bits are zero, so the 8-bit kernel sorts it correctly
         if (plan.cluster)
             run_cluster_pass<true>(s, kin, vin, kout, vout, n, plan.shift[p], plan.width[p],
-                             last ? rank_out : nullptr, mark);
+                             last ? rank_out : nullptr, mark, p > 0);
         else if (plan.width[p] <= 8)
             run_pass<8>(s, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
-                        last ? rank_out : nullptr, mark, plan.fused);
+                        last ? rank_out : nullptr, mark, plan.fused, p > 0);
         else if (plan.width[p] == 9)
             run_pass<9>(s, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
-                        last ? rank_out : nullptr, mark, plan.fused);
+                        last ? rank_out : nullptr, mark, plan.fused, p > 0);
         else
             run_pass<10>(s, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
-                        last ? rank_out : nullptr, mark, plan.fused);
+                        last ? rank_out : nullptr, mark, plan.fused, p > 0);
         if (kout == k1) {
             kin = k1; vin = v1; kout = k0; vout = v0;
         } else {

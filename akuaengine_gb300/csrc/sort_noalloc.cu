@@ -114,16 +114,16 @@ extern "C" int akua_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* 
         const uint32_t mask = (1u << plan.width[p]) - 1u;
         if (plan.cluster)
             akua::radix::run_cluster_pass<false>(st, kin, vin, kout, vout, n, plan.shift[p], plan.width[p],
-                                          nullptr, mark);
+                                          nullptr, mark, p > 0);
         else if (plan.width[p] <= 8)
             akua::radix::run_pass<8>(st, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
-                                      nullptr, mark, fused, mask);
+                                      nullptr, mark, fused, p > 0, mask);
         else if (plan.width[p] == 9)
             akua::radix::run_pass<9>(st, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
-                                      nullptr, mark, fused, mask);
+                                      nullptr, mark, fused, p > 0, mask);
         else
             akua::radix::run_pass<10>(st, kin, vin, kout, vout, counts, totals, n, plan.shift[p],
-                                      nullptr, mark, fused, mask);
+                                      nullptr, mark, fused, p > 0, mask);
         kin = kout;
         vin = vout;
     }
