@@ -33,6 +33,23 @@ struct Guard {
     }
 };
 
+// A launch that is set up while the stream's previous kernel ends (the kernel waits for its stores).
+template <class... Params, class... Args>
+void launch_after(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st,
+                  Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 int launch_grad(akua_mlp* m, const float* feat, const float* target, int32_t n, cudaStream_t st) {
     static bool attr_set[64] = {};
     if (m->device < 64 && !attr_set[m->device]) {
@@ -44,8 +61,8 @@ int launch_grad(akua_mlp* m, const float* feat, const float* target, int32_t n, 
     }
     const int tiles = (n + akua::mlp::kTile - 1) / akua::mlp::kTile;
     const int grid = std::max(1, std::min(tiles, m->sms));  // one CTA of 16 warps per SM
-    akua::mlp::k_mlp_grad<<<grid, akua::mlp::kGradThreads, akua::mlp::kGradSmem, st>>>(
-        m->params, m->image, m->norm, feat, target, n, 1.0f / (float)n, m->grad, m->err);
+    launch_after(akua::mlp::k_mlp_grad, grid, akua::mlp::kGradThreads, akua::mlp::kGradSmem, st,
+                 m->params, m->image, m->norm, feat, target, n, 1.0f / (float)n, m->grad, m->err);
     return status_of(cudaGetLastError());
 }
 
@@ -200,8 +217,8 @@ int akua_mlp_adam_step(akua_mlp* m, const float* features, const float* targets,
     const float bc1 = (float)(1.0 - std::pow((double)b1, (double)m->adam_steps));
     const float bc2 = (float)(1.0 - std::pow((double)b2, (double)m->adam_steps));
     const int blocks = (akua::mlp::kParams + 1 + 255) / 256;
-    akua::mlp::k_mlp_adam<<<blocks, 256, 0, st>>>(m->params, m->grad, m->m, m->v, m->image,
-                                                 learningRate, b1, b2, 1e-8f, bc1, bc2);
+    launch_after(akua::mlp::k_mlp_adam, blocks, 256, 0, st, m->params, m->grad, m->m, m->v, m->image,
+                 learningRate, b1, b2, 1e-8f, bc1, bc2);
     return status_of(cudaGetLastError());
 }
 
