@@ -73,9 +73,9 @@ namespace akua::mlp {
 int enqueue_forward(const akua_mlp* m, const float* feat, int n, float* out, float* out2,
                     float* out4, cudaStream_t st) {
     const int tiles = (n + kTile - 1) / kTile;
-    const int grid = std::max(1, std::min(tiles, 5 * m->sms));  // 5 x 40 KB of shared memory
-    k_mlp_forward<<<grid, kThreads, 0, st>>>(m->params, m->image, m->norm, feat, n, out, out2,
-                                             out4, m->err);
+    const int grid = std::max(1, std::min(tiles, 2 * m->sms));
+    launch_after(k_mlp_forward, grid, kFwdThreads, kFwdSmem, st, m->params, m->image, m->norm, feat, n,
+                 out, out2, out4, m->err);
     return status_of(cudaGetLastError());
 }
 }  // namespace akua::mlp
@@ -90,6 +90,9 @@ int akua_mlp_create(akua_mlp** out) {
     cudaError_t e = cudaGetDevice(&m->device);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(akua::mlp::k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)akua::mlp::kFwdSmem);
     const size_t pb = sizeof(float) * akua::mlp::kParams;
     if (e == cudaSuccess) e = cudaMalloc(&m->params, pb);
     if (e == cudaSuccess) e = cudaMalloc(&m->grad, pb + sizeof(float));

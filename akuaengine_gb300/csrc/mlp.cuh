@@ -12,8 +12,8 @@
 //   dy = 2 (y - t') / n;  dz3 = bf16(dy w4 silu'(z3));  dz2 = bf16((dz3 W3) silu'(z2));
 //   dz1 = bf16((dz2 W2) silu'(z1));  dW_l = dz_l^T a_{l-1};  db_l = sum dz_l;  dw4 = sum dy a3
 //
-// The forward kernel: one CTA of 128 threads per tile of 128 samples (thread t owns sample row t,
-// TMEM lane t) and one 64-column accumulator.  The gradient kernel: 512 threads per tile, one
+// The forward kernel: a warpgroup per tile of 128 samples (thread t owns sample row t, TMEM lane t) and
+// one 64-column accumulator.  The gradient kernel: 512 threads per tile, one
 // 64-column accumulator for z and the input gradients in turn and three for the weight gradients,
 // which it accumulates over all tiles it processes before one flush.  Weight gradients are MMAs over
 // the batch, D[out][in] = dz[b][out] a[b][in], with a column of ones beside the activations whose
@@ -66,15 +66,16 @@ __device__ __forceinline__ float silu(float z) { return z * sigmoid(z); }
 // Inference: silu of two values, the tanh evaluated on an FP16 pair (tanh.approx.f16x2: one
 // multi-function operation for two activations; its error, about 2^-11 relative, is below the
 // BF16 rounding the hidden activations get next).
-__device__ __forceinline__ float2 silu2(float z0, float z1) {
-    const __half2 hz = __floats2half2_rn(0.5f * z0, 0.5f * z1);
+__device__ __forceinline__ float2 silu2(float2 z) {
+    const float2 half = make_float2(0.5f, 0.5f);
+    const float2 hz = __fmul2_rn(half, z);
+    const __half2 h = __floats2half2_rn(hz.x, hz.y);
     uint32_t in, out;
-    memcpy(&in, &hz, 4);
+    memcpy(&in, &h, 4);
     asm("tanh.approx.f16x2 %0, %1;" : "=r"(out) : "r"(in));
     __half2 ht;
     memcpy(&ht, &out, 4);
-    const float2 t = __half22float2(ht);
-    return make_float2(z0 * __fmaf_rn(0.5f, t.x, 0.5f), z1 * __fmaf_rn(0.5f, t.y, 0.5f));
+    return __fmul2_rn(z, __ffma2_rn(half, __half22float2(ht), half));
 }
 __device__ __forceinline__ float dsilu(float z) {
     const float s = sigmoid(z);
@@ -91,17 +92,6 @@ __device__ __forceinline__ uint16_t bf16_bits(float a) {
 }
 __device__ __forceinline__ float bf16_round(float a) {
     return __bfloat162float(__float2bfloat16_rn(a));
-}
-
-// Row `row` of a K-major tile with K = 64: 64 values as eight 16-byte core-matrix rows.
-__device__ __forceinline__ void store_row64(uint8_t* tile, int row, const float* v, int c0) {
-    // v holds 16 values for columns c0 .. c0+15
-    *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(row, c0, 64)) =
-        make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
-                   pack_bf16(v[6], v[7]));
-    *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(row, c0 + 8, 64)) =
-        make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]),
-                   pack_bf16(v[14], v[15]));
 }
 
 // Stages a [64][kin] weight (row-major FP32) as a BF16 K-major B operand with K = kpad columns (zeros
@@ -128,61 +118,65 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // ------------------------------------------------------------------------------------ forward
+// Four tiles of 128 samples per CTA, a warpgroup each with its own accumulator, operand tiles and
+// barriers; the weights are staged once for all four.
+constexpr int kFwdGroups = 4;
+constexpr int kFwdThreads = kFwdGroups * kTile;
 struct FwdSmem {
     alignas(128) uint8_t w1[kHid * kInPad * 2];
     alignas(128) uint8_t w2[kHid * kHid * 2];
     alignas(128) uint8_t w3[kHid * kHid * 2];
-    alignas(128) uint8_t x[kTile * kInPad * 2];
-    alignas(128) uint8_t h[kTile * kHid * 2];
-    float b1[kHid], b2[kHid], b3[kHid], w4[kHid];
+    alignas(128) uint8_t x[kFwdGroups][kTile * kInPad * 2];
+    alignas(128) uint8_t h[kFwdGroups][kTile * kHid * 2];
+    alignas(16) float b1[kHid], b2[kHid], b3[kHid], w4[kHid];
     float norm[kNorm];
     float b4;
-    alignas(8) uint64_t bar;
+    alignas(8) uint64_t bar[kFwdGroups];
     uint32_t tmem;
 };
+constexpr size_t kFwdSmem = sizeof(FwdSmem);
+
+// SiLU of 32 columns of this thread's TMEM row plus their biases, two at a time: f(column, values).
+template <class F>
+__device__ __forceinline__ void silu_columns(uint32_t taddr, const float* b, F&& f) {
+    uint32_t r[2][16];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) tc::tmem_ld16_async(taddr + 16 * c, r[c]);
+    tc::tmem_wait_ld();
+#pragma unroll
+    for (int c = 0; c < 2; ++c) tc::tmem_after_wait(r[c]);
+#pragma unroll
+    for (int q = 0; q < 32; q += 2) {
+        const float2 z = make_float2(__uint_as_float(r[q / 16][q % 16]),
+                                     __uint_as_float(r[q / 16][q % 16 + 1]));
+        f(q, silu2(__fadd2_rn(z, *reinterpret_cast<const float2*>(b + q))));
+    }
+}
 
 // Epilogue of a hidden layer: TMEM columns [col, col+64) of this thread's row -> bias, SiLU,
 // BF16 -> row t of the next layer's A tile.
 __device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float* b, uint8_t* h, int t) {
-    uint32_t r[4][16];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) tc::tmem_ld16_async(taddr + 16 * c, r[c]);
-    tc::tmem_wait_ld();
+    for (int c0 = 0; c0 < kHid; c0 += 32) {
+        uint32_t v[16];
+        silu_columns(taddr + c0, b + c0, [&](int q, float2 a) { v[q / 2] = pack_bf16(a.x, a.y); });
 #pragma unroll
-    for (int c = 0; c < 4; ++c) tc::tmem_after_wait(r[c]);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        float v[16];
-#pragma unroll
-        for (int q = 0; q < 16; q += 2) {
-            const float2 a = silu2(__uint_as_float(r[c][q]) + b[16 * c + q],
-                                   __uint_as_float(r[c][q + 1]) + b[16 * c + q + 1]);
-            v[q] = a.x;
-            v[q + 1] = a.y;
-        }
-        store_row64(h, t, v, 16 * c);
+        for (int q = 0; q < 16; q += 4)
+            *reinterpret_cast<uint4*>(h + tc::kmajor_offset(t, c0 + 2 * q, 64)) =
+                make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]);
     }
 }
 
 // Output layer on the FP32 pipe: b4 + sum_c w4[c] silu(z3[c] + b3[c]).
 __device__ __forceinline__ float output_layer(uint32_t taddr, const float* b3, const float* w4,
                                               float b4) {
-    uint32_t r[4][16];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) tc::tmem_ld16_async(taddr + 16 * c, r[c]);
-    tc::tmem_wait_ld();
-#pragma unroll
-    for (int c = 0; c < 4; ++c) tc::tmem_after_wait(r[c]);
     float y = b4;
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int q = 0; q < 16; q += 2) {
-            const float2 a = silu2(__uint_as_float(r[c][q]) + b3[16 * c + q],
-                                   __uint_as_float(r[c][q + 1]) + b3[16 * c + q + 1]);
-            y = __fmaf_rn(w4[16 * c + q], a.x, y);
-            y = __fmaf_rn(w4[16 * c + q + 1], a.y, y);
-        }
+    for (int c0 = 0; c0 < kHid; c0 += 32)
+        silu_columns(taddr + c0, b3 + c0, [&](int q, float2 a) {
+            y = __fmaf_rn(w4[c0 + q], a.x, y);
+            y = __fmaf_rn(w4[c0 + q + 1], a.y, y);
+        });
     return y;
 }
 
@@ -202,112 +196,120 @@ __device__ __forceinline__ void load_features(const float* __restrict__ feat, in
 // Features (n x 8, FP32) -> out2[i] = the network's estimate p_i (output * out_scale) and
 // out[i] = lambda0_i + blend * (p_i - lambda0_i), lambda0 = feature 3 (blend 1: out = p); the
 // latter also into out4[4 i] when given.
-__global__ void __launch_bounds__(kThreads)
+//
+// Bound by the SiLU epilogues' issue slots and by a tile's chain of three MMAs, which the other
+// warpgroups' epilogues fill: two CTAs of four warpgroups per SM (64 registers a thread).
+// 1M samples: 72 -> 67 us against five CTAs of one warpgroup with scalar epilogues, 155,648: 20.5 ->
+// 16.4 (the hardware tanh of 192 activations a sample alone takes about 40 at 1M).
+__global__ void __launch_bounds__(kFwdThreads, 2)
     k_mlp_forward(const float* __restrict__ params, const uint8_t* __restrict__ image,
                   const float* __restrict__ norm, const float* __restrict__ feat, int n,
                   float* __restrict__ out, float* __restrict__ out2, float* __restrict__ out4,
                   uint32_t* __restrict__ err) {
-    __shared__ FwdSmem S;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    FwdSmem& S = *reinterpret_cast<FwdSmem*>(smem_raw);
     static_assert(offsetof(FwdSmem, w2) == offsetof(FwdSmem, w1) + sizeof(S.w1) &&
                       offsetof(FwdSmem, w3) == offsetof(FwdSmem, w2) + sizeof(S.w2) &&
                       sizeof(S.w1) + sizeof(S.w2) + sizeof(S.w3) == kImageBytes,
                   "the weight image is w1, w2, w3 back to back");
-    const int t = threadIdx.x, warp = t >> 5;
+    const int group = threadIdx.x / kTile, t = threadIdx.x % kTile, warp = t >> 5;
+    if (t == 0) tc::mbar_init(&S.bar[group], 1);
+    uint8_t* x = S.x[group];
+    uint8_t* h = S.h[group];
+    // columns 8..15 of the input tile stay zero
+    *reinterpret_cast<uint4*>(x + tc::kmajor_offset(t, 8, kInPad)) = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x < 32) tc::tmem_alloc(&S.tmem, kFwdGroups * kHid);
+    tc::wait_for_previous();
     {
         const uint4* src = reinterpret_cast<const uint4*>(image);
         uint4* dst = reinterpret_cast<uint4*>(S.w1);
-        for (int k = t; k < kImageBytes / 16; k += kThreads) dst[k] = __ldg(src + k);
+        for (int k = threadIdx.x; k < kImageBytes / 16; k += kFwdThreads) dst[k] = __ldg(src + k);
     }
-    if (t < kHid) {
+    if (threadIdx.x < kHid) {
         S.b1[t] = params[kB1 + t];
         S.b2[t] = params[kB2 + t];
         S.b3[t] = params[kB3 + t];
         S.w4[t] = params[kW4 + t];
     }
-    if (t < kNorm) S.norm[t] = norm[t];
-    if (t == 0) {
-        S.b4 = params[kB4];
-        tc::mbar_init(&S.bar, 1);
-    }
-    // columns 8..15 of the input tile stay zero
-    *reinterpret_cast<uint4*>(S.x + tc::kmajor_offset(t, 8, kInPad)) = make_uint4(0, 0, 0, 0);
-    if (warp == 0) tc::tmem_alloc(&S.tmem, 64);
+    if (threadIdx.x < kNorm) S.norm[t] = norm[t];
+    if (threadIdx.x == 0) S.b4 = params[kB4];
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem = S.tmem;
+    const uint32_t tmem = S.tmem + kHid * group;
     const uint32_t lane = tmem + ((uint32_t)(warp * 32) << 16);
-    const uint32_t idesc = tc::idesc_bf16(128, 64);
-    const uint64_t dx = tc::smem_desc(tc::smem_addr(S.x), 128, kInPad * 16);
+    constexpr uint32_t idesc = tc::idesc_bf16(128, 64);
+    const uint64_t dx = tc::smem_desc(tc::smem_addr(x), 128, kInPad * 16);
     const uint64_t dw1 = tc::smem_desc(tc::smem_addr(S.w1), 128, kInPad * 16);
-    const uint32_t sh = tc::smem_addr(S.h), sw2 = tc::smem_addr(S.w2), sw3 = tc::smem_addr(S.w3);
+    const uint32_t sh = tc::smem_addr(h), sw2 = tc::smem_addr(S.w2), sw3 = tc::smem_addr(S.w3);
     uint32_t phase = 0;
     bool ok = true;
+    auto publish = [&]() {  // this warpgroup's operand stores and tensor-memory reads are done
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kTile) : "memory");
+        if (t == 0) tc::fence_after_sync();
+    };
+    // after a wait that ran out nothing waits again and nothing is written
+    auto wait = [&]() {
+        if (ok) ok = tc::mbar_wait(&S.bar[group], phase);
+        phase ^= 1;
+        tc::fence_after_sync();
+    };
+    auto layer = [&](uint32_t sw) {
+        if (t == 0) {
+#pragma unroll
+            for (int s = 0; s < kHid / 16; ++s)
+                tc::mma_bf16(tmem, tc::smem_desc(sh + 256 * s, 128, kHid * 16),
+                             tc::smem_desc(sw + 256 * s, 128, kHid * 16), idesc, s > 0);
+            tc::mma_commit(&S.bar[group]);
+        }
+        wait();
+    };
     const int tiles = (n + kTile - 1) / kTile;
+    // tiles in an order that gives every CTA one before any gets a second
+    const int first = blockIdx.x + gridDim.x * group, step = gridDim.x * kFwdGroups;
     float fnext[kIn];
-    load_features(feat, blockIdx.x * kTile + t, n, S.norm, fnext);
+    load_features(feat, first * kTile + t, n, S.norm, fnext);
     const float blend = S.norm[2 * kIn + 1];
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+    for (int tile = first; tile < tiles; tile += step) {
         const int i = tile * kTile + t;
         const float lam0 = fnext[kLam0];
         float f[kIn];
 #pragma unroll
         for (int k = 0; k < kIn; ++k) f[k] = (fnext[k] - S.norm[k]) * S.norm[kIn + k];
-        if (tile + (int)gridDim.x < tiles)  // the next tile's features, in flight meanwhile
-            load_features(feat, (tile + gridDim.x) * kTile + t, n, S.norm, fnext);
-        *reinterpret_cast<uint4*>(S.x + tc::kmajor_offset(t, 0, kInPad)) =
+        if (tile + step < tiles)  // the next tile's features, in flight meanwhile
+            load_features(feat, (tile + step) * kTile + t, n, S.norm, fnext);
+        *reinterpret_cast<uint4*>(x + tc::kmajor_offset(t, 0, kInPad)) =
             make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
                        pack_bf16(f[6], f[7]));
-        // layer 1
-        tc::fence_async_smem();
-        tc::fence_before_sync();
-        __syncthreads();
+        publish();
         if (t == 0) {
-            tc::fence_after_sync();
             tc::mma_bf16(tmem, dx, dw1, idesc, 0);
-            tc::mma_commit(&S.bar);
+            tc::mma_commit(&S.bar[group]);
         }
-        ok = __syncthreads_and(tc::mbar_wait(&S.bar, phase));
-        phase ^= 1;
-        if (!ok) break;
-        tc::fence_after_sync();
-        hidden_epilogue(lane, S.b1, S.h, t);
-        // layers 2 and 3
-        for (int layer = 0; layer < 2 && ok; ++layer) {
-            tc::fence_async_smem();
-            tc::fence_before_sync();
-            __syncthreads();
-            if (t == 0) {
-                tc::fence_after_sync();
-                const uint32_t sw = layer == 0 ? sw2 : sw3;
-#pragma unroll
-                for (int s = 0; s < kHid / 16; ++s)
-                    tc::mma_bf16(tmem, tc::smem_desc(sh + 256 * s, 128, kHid * 16),
-                                 tc::smem_desc(sw + 256 * s, 128, kHid * 16), idesc, s > 0);
-                tc::mma_commit(&S.bar);
-            }
-            ok = __syncthreads_and(tc::mbar_wait(&S.bar, phase));
-            phase ^= 1;
-            if (!ok) break;
-            tc::fence_after_sync();
-            if (layer == 0) hidden_epilogue(lane, S.b2, S.h, t);
-        }
-        if (!ok) break;
+        wait();
+        hidden_epilogue(lane, S.b1, h, t);
+        publish();
+        layer(sw2);
+        hidden_epilogue(lane, S.b2, h, t);
+        publish();
+        layer(sw3);
         const float y = output_layer(lane, S.b3, S.w4, S.b4);
-        if (i < n) {
+        if (ok && i < n) {
             const float o = y * S.norm[2 * kIn];
             const float used = blend == 1.0f ? o : __fmaf_rn(blend, o - lam0, lam0);
             out[i] = used;
             if (out2) out2[i] = o;
             if (out4) out4[4 * (size_t)i] = used;  // a float4 array's 4th component
         }
-        tc::fence_before_sync();
     }
-    if (!ok && t == 0) atomicOr(err, (uint32_t)kErrTimeout);
+    if (!ok) atomicOr(err, (uint32_t)kErrTimeout);
+    tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) {
+    if (threadIdx.x < 32) {
         tc::fence_after_sync();
-        tc::tmem_free(tmem, 64);
+        tc::tmem_free(S.tmem, kFwdGroups * kHid);
     }
 }
 

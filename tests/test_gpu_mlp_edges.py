@@ -60,3 +60,20 @@ def test_images_follow_adam_steps(net):  # noqa: F811
         assert fresh.gradient(f, t)[1] == pytest.approx(net.gradient(f, t)[1], rel=1e-5)
     finally:
         fresh.close()
+
+
+@pytest.mark.parametrize("rounds", [1, 4, 5])
+def test_forward_grid_edges(net, rounds):  # noqa: F811
+    """Counts around a tile for every block (two per multiprocessor), for every warpgroup of them, and
+    beyond: a sample's output does not depend on the others, so it equals that of a small call bit
+    for bit."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    params, mean, inv_std, scale, feat, _ = _problem(6, 128 * 2 * sms * rounds + 1)
+    net.set_params(params)
+    net.set_normalization(mean, inv_std, scale)
+    f = torch.from_numpy(feat).cuda()
+    for n in (len(feat), len(feat) - 2):
+        want = torch.cat([net.forward(f[k:min(k + 8000, n)]) for k in range(0, n, 8000)])
+        assert torch.equal(net.forward(f[:n]), want)
