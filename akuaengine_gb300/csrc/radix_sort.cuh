@@ -89,19 +89,26 @@ __device__ __forceinline__ void wait_for_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class... Params, class... Args>
-inline void launch(bool after, void (*kernel)(Params...), int grid, int block, size_t smem,
-                   cudaStream_t st, Args... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t launch(bool after, void (*kernel)(Params...), int grid, int block, size_t smem,
+                          cudaStream_t st, int cluster, Args... args) {
+    cudaLaunchAttribute attr[2] = {};
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = after ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    cfg.attrs = attr;
+    if (after) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
 // counts[tile * RADIX + d] = keys of `tile` with digit d.  A key's digit is (key >> shift) &
@@ -345,35 +352,34 @@ inline void run_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, u
     constexpr int RADIX = 1 << BITS;
     constexpr size_t smem = scatter_smem(WARPS, RADIX, TILE);
     digit_mask &= RADIX - 1;  // the kernels' shared-memory tables hold RADIX digits
-    launch(after, upsweep<BITS>, tiles, BLOCK, 0, s, kin, n, shift, digit_mask, counts);
+    launch(after, upsweep<BITS>, tiles, BLOCK, 0, s, 1, kin, n, shift, digit_mask, counts);
     mark("radix_upsweep");
     if (!fused) {
-        launch(true, scan_tiles<BITS>, RADIX / SCAN_DIGITS, 32 * SCAN_WARPS, 0, s, counts, totals, tiles);
+        launch(true, scan_tiles<BITS>, RADIX / SCAN_DIGITS, 32 * SCAN_WARPS, 0, s, 1, counts, totals, tiles);
         mark("radix_scan");
-        launch(true, downsweep<BITS, false>, tiles, BLOCK, smem, s, kin, vin, kout, vout, n, shift, digit_mask,
+        launch(true, downsweep<BITS, false>, tiles, BLOCK, smem, s, 1, kin, vin, kout, vout, n, shift, digit_mask,
                                                           counts, totals, tiles, rank_out);
     } else {
-        launch(true, downsweep<BITS, true>, tiles, BLOCK, smem, s, kin, vin, kout, vout, n, shift, digit_mask,
+        launch(true, downsweep<BITS, true>, tiles, BLOCK, smem, s, 1, kin, vin, kout, vout, n, shift, digit_mask,
                                                          counts, nullptr, tiles, rank_out);
     }
     mark("radix_downsweep");
 }
 
-// ---- Sorts of up to kClusterMax pairs: a pass in one kernel, on one cluster of 8 blocks.
+// ---- Sorts of up to kClusterMax pairs: a pass in one kernel, on one cluster of blocks.
 //
 // A tiled pass over a small input is three launches, each a few microseconds of latency for next to
 // no work.  Here one cluster holds all pairs in registers: a block ranks its own (match.any and
 // per-warp digit counters, as downsweep does), reads the other blocks' digit totals through
 // distributed shared memory, scans them and scatters to global memory.
-// Three passes over 27,000 random keys: 56 -> 22 us, 4,096: 39 -> 8; at 65,536 32 us, where the tiled
-// passes take 34 (eight SMs against sixteen).  The step of 27,000 particles: 158 -> 133 us.
-constexpr int kClusterBlocks = 8;
+// Sorts of random keys in three passes: 27,000 pairs 56 -> 18 us, 65,536 34 -> 24; in two, 4,096: 39 -> 8.
+// The step of 27,000 particles: 158 -> 131 us.
 constexpr int kClusterThreads = 512;  // one thread per digit in the scans
 constexpr int kClusterWarps = kClusterThreads / 32;
 constexpr int kClusterBits = 9;
 constexpr int kClusterRadix = 1 << kClusterBits;
-constexpr int kClusterMaxRounds = 16;
-constexpr int kClusterMax = kClusterBlocks * kClusterThreads * kClusterMaxRounds;  // 65,536 pairs
+constexpr int kClusterMax = 16 * kClusterThreads * 8;         // 65,536: eight rounds of 16 blocks
+constexpr int kClusterPortableMax = 8 * kClusterThreads * 4;  // 16,384: four rounds of 8 blocks
 static_assert(kClusterRadix == kClusterThreads, "thread d scans digit d");
 
 inline Plan make_cluster_plan(int bits) {
@@ -404,8 +410,8 @@ __device__ __forceinline__ void cluster_wait() {
 
 // One pass over the digit (key >> shift) & digit_mask, digit_mask < kClusterRadix.  Block b holds
 // the pairs from b * 512 * ROUNDS on; warp w of it 32 * ROUNDS of them, in rounds of 32.
-template <int ROUNDS, bool RUNS>
-__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kClusterThreads)
+template <int BLOCKS, int ROUNDS, bool RUNS>
+__global__ void __launch_bounds__(kClusterThreads)
     cluster_pass(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                  uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n, int shift,
                  uint32_t digit_mask, uint32_t* __restrict__ rank_out) {
@@ -463,7 +469,7 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kCluste
     // digit t: the pairs of all blocks, and of the blocks before this one
     uint32_t all = 0, before = 0;
 #pragma unroll
-    for (uint32_t b = 0; b < kClusterBlocks; ++b) {
+    for (uint32_t b = 0; b < BLOCKS; ++b) {
         const uint32_t c = ld_remote(&total[t], b);
         all += c;
         before += b < rank ? c : 0u;
@@ -507,21 +513,49 @@ template <bool RUNS, class Mark>
 inline void run_cluster_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                              uint32_t* vout, int n, int shift, int width, uint32_t* rank_out,
                              Mark& mark, bool after) {
-    constexpr int kRound = kClusterBlocks * kClusterThreads;
+    constexpr int kRound = 8 * kClusterThreads;
     const uint32_t mask = (1u << width) - 1u;
-    auto go = [&](auto kernel, int rounds) {
+    auto go = [&](auto kernel, int blocks, int rounds) {
         const size_t smem = scatter_smem(kClusterWarps, kClusterRadix, kClusterThreads * rounds);
-        if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch(after, kernel, kClusterBlocks, kClusterThreads, smem, s, kin, vin, kout, vout, n, shift,
+        launch(after, kernel, blocks, kClusterThreads, smem, s, blocks, kin, vin, kout, vout, n, shift,
                mask, rank_out);
     };
-    if (n <= kRound) go(cluster_pass<1, RUNS>, 1);
-    else if (n <= 2 * kRound) go(cluster_pass<2, RUNS>, 2);
-    else if (n <= 4 * kRound) go(cluster_pass<4, RUNS>, 4);
-    else if (n <= 8 * kRound) go(cluster_pass<8, RUNS>, 8);
-    else go(cluster_pass<16, RUNS>, 16);
+    // 8 blocks wait for one another sooner, 16 spread the pairs and their scattered stores over more
+    // SMs.  A step with 8 and with 16: 6,000 particles 85.3 and 86.3 us, 12,000 91.1 and 91.8, 27,000
+    // 115.5 and 113.9, 40,000 136.3 and 132.1, 60,000 151.5 and 147.0.
+    if (n <= kRound) go(cluster_pass<8, 1, RUNS>, 8, 1);
+    else if (n <= 2 * kRound) go(cluster_pass<8, 2, RUNS>, 8, 2);
+    else if (n <= 4 * kRound) go(cluster_pass<8, 4, RUNS>, 8, 4);
+    else if (n <= 8 * kRound) go(cluster_pass<16, 4, RUNS>, 16, 4);
+    else go(cluster_pass<16, 8, RUNS>, 16, 8);
     mark("radix_cluster_pass");
+}
+
+// The largest input a cluster's passes can take on the current device: kClusterMax where it places
+// clusters of 16 blocks (beyond the portable 8, so the kernels must be allowed them), else
+// kClusterPortableMax.
+template <bool RUNS>
+inline int cluster_limit() {
+    auto allow = [](auto kernel) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    };
+    cudaError_t e = allow(cluster_pass<16, 4, RUNS>);
+    if (e == cudaSuccess) e = allow(cluster_pass<16, 8, RUNS>);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 16;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = scatter_smem(kClusterWarps, kClusterRadix, kClusterThreads * 8);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveClusters(&clusters, cluster_pass<16, 8, RUNS>, &cfg);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && clusters > 0 ? kClusterMax : kClusterPortableMax;
 }
 
 // Scratch words the sort needs for n keys: the count matrix and a pass's digit totals.
@@ -529,8 +563,8 @@ inline size_t scratch_words(int n) {
     return (size_t)MAX_RADIX * num_tiles(n) + MAX_RADIX;
 }
 
-// Sorts (k0, v0) by the low plan bits (a cluster plan: n <= kClusterMax), ping-ponging with (k1, v1); all four buffers hold n words.
-// With `index_payload` the input payload is each key's index and v0 is not read.  The result
+// Sorts (k0, v0) by the low plan bits, ping-ponging with (k1, v1); all four buffers hold n words (a
+// cluster plan: n <= cluster_limit()).  With `index_payload` the input payload is each key's index and v0 is not read.  The result
 // buffers are returned through keys_out / vals_out.  With `rank_out` (n words), the last pass
 // also writes rank_out[payload] = output position.  `mark(name)` is called after every kernel.
 template <class Mark>

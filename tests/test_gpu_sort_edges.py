@@ -14,7 +14,7 @@ from test_gpu_walk_edges import first_of_block
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 31, 4095, 4096, 4097, 8192, 8193, 16385, 32768, 32769, 65536,
+@pytest.mark.parametrize("n", [1, 31, 4095, 4096, 4097, 8192, 8193, 16384, 16385, 32768, 32769, 65536,
                                65537, 69632, 69633])
 @pytest.mark.parametrize("bits", [1, 9, 10, 19, 32])
 def test_sort_pairs_edges(cuda_lib, n, bits):
@@ -39,7 +39,7 @@ def test_sort_pairs_edges(cuda_lib, n, bits):
     assert np.array_equal(dev[3][1:].cpu().numpy().view(np.uint32), payload[order])
 
 
-@pytest.mark.parametrize("n", [4096, 4097, 65536, 65537])
+@pytest.mark.parametrize("n", [4096, 4097, 16384, 16385, 65536, 65537])
 def test_step_order_at_sort_edges(cuda_lib, n):
     """Two steps (the second sorts the first one's order) on both sides of the lines, against the
     oracle."""
