@@ -67,13 +67,14 @@ constexpr int kListStage = 32;
 
 // Particles per warp.  32 keep every lane of the extraction busy, but a warp works through its runs
 // one after another, so with few warps the walk lasts as long as one warp: a scene whose warps of
-// 8 (or 16) particles still all fit the chip at once (32 warps per SM: 64 registers per thread)
-// takes them.  Measured (us, at 8 / 16 / 32): 1,000 particles 18 / 21 / 25, 27,000 26 / 27 / 30,
-// 50,000 39 / 32 / 36, 70,000 48 / 36 / 40, 100,000 63 / 51 / 45.
-constexpr int kSearchWarps = 32;
-inline int search_per_warp(int n, int sms) {
-    for (int w = 8; w < 32; w *= 2)
-        if (n <= w * kSearchWarps * sms) return w;
+// 8 (16, 24) particles still all fit the chip at once (32 warps per SM of 64 registers a thread, 24 of
+// the exact variant's 80) takes them.  Measured (us, at 8 / 16 / 24 / 32): 1,000 particles 18 / 21 / - /
+// 25, 27,000 26 / 27 / - / 30, 50,000 39 / 31 / - / 36, 70,000 48 / 36 / - / 40, 100,000 63 / 52 / 41 /
+// 44, and 100,000 in exact math, where 24 no longer fit, - / - / 63 / 53.
+inline int search_per_warp(int n, int sms, bool exact) {
+    const int warps = (exact ? 24 : 32) * sms;
+    for (int w = 8; w < 32; w += 8)
+        if (n <= w * warps) return w;
     return 32;
 }
 constexpr int kPairWords = 3 * 32;  // a run's positions, two particles interleaved

@@ -333,7 +333,7 @@ void launch_search_shape(akua_pbf* s, cudaStream_t st, int density, float* feat)
     if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
         cudaFuncSetAttribute(akua::k_search<EXACT, BLOCK, STAGE>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int per_warp = akua::search_per_warp(s->n, s->sms);
+    const int per_warp = akua::search_per_warp(s->n, s->sms, EXACT);
     step_kernel(s, st, akua::k_search<EXACT, BLOCK, STAGE>,
                 grid_for(s->n, per_warp * (BLOCK / 32)), BLOCK, smem, s->d_params,
                 s->ps0, s->table, s->r2i, s->nbr, s->cnt, s->rho, s->lam, s->flags, density,

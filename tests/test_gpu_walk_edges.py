@@ -25,15 +25,15 @@ def first_of_block(n, seed):
     return sc
 
 
-@pytest.mark.parametrize("where", [9, 31, 33, 65, "8-", "8+", "16-", "16+"])
+@pytest.mark.parametrize("where", [9, 31, 33, 65, "8-", "8+", "16-", "16+", "24-", "24+"])
 def test_particles_per_warp_edges(where):
-    """Counts around a warp and around the lines where the walk goes from 8 to 16 and from 16 to
-    32 particles per warp (8 x 32 and 16 x 32 per multiprocessor)."""
+    """Counts around a warp and around the lines where the walk goes from 8 to 16, 24 and 32
+    particles per warp (8 x 24, 16 x 24 and 24 x 24 per multiprocessor in exact math)."""
     if isinstance(where, str):
         import torch
 
         sms = torch.cuda.get_device_properties(0).multi_processor_count
-        n = int(where[:-1]) * 32 * sms + (1 if where.endswith("+") else 0)
+        n = int(where[:-1]) * 24 * sms + (1 if where.endswith("+") else 0)
     else:
         n = where
     sc = first_of_block(n, seed=n)
