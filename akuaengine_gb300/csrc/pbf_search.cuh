@@ -11,8 +11,9 @@
 // flagged as mixed (several cells on one hash, or cells sharing a clamped Morton key) are walked in
 // reference order, their ranks mapped to slots.  Both give the reference's list, entry for entry.
 //
-// Warp-cooperative walk.  A warp takes 32 consecutive particles (8 or 16 in small scenes, see
-// search_per_warp); consecutive particles of the same cell (a run) share one candidate sequence: the concatenation of the 27 buckets in walk order.
+// Warp-cooperative walk.  A warp takes 32 consecutive particles (fewer in small scenes, see
+// search_per_warp); consecutive particles of the same cell (a run) share one candidate sequence: the
+// concatenation of the 27 buckets in walk order.
 //
 //   stage    lanes 0..26 look up one bucket each (the next run's lookups are in flight meanwhile),
 //            a warp scan gives each bucket's offset, and the lanes write the sequence's slots into
@@ -20,7 +21,10 @@
 //   cull     candidates out of reach of the box around the run's particles leave the sequence (the
 //            rest keep their order): half of them, as a run is about seven particles that fill
 //            part of a cell.  The test is the pair test at the box's nearest point; rounding is
-//            monotonic, so nothing a particle could accept is dropped;
+//            monotonic, so nothing a particle could accept is dropped.  A round takes 128, four per
+//            lane: a quarter of the latencies of rounds of 32, even where those load a round ahead
+//            (walk at 1M: 275 us with 32, 265 with 64, 253 with 128, 262 with 160, whose records no
+//            longer fit the registers);
 //   test     64 candidates at a time, two per lane, against the run's particles, two per round in
 //            packed FP32x2.  A round's four ballots are all it leaves behind (hit masks in the
 //            pool): no counts, no placement and no self test, two shared loads, twelve packed
@@ -38,8 +42,8 @@
 // extraction.  Measured on that scene, 394 us before: hit masks and extraction 358 us, with one
 // pool for masks and candidates 316, 64 candidates per round 279, masks with hits named by a bit
 // and the reach tests of list entries dropped 265, the next run's lookup in flight 262; the cull
-// makes the pool a third smaller and the walk's chain shorter: 270 at 1M, 2,196 against 2,231 at
-// 8M, 30 against 36 at 27k.
+// makes the pool a third smaller and the walk's chain shorter (2,196 against 2,231 at 8M, 30 against
+// 36 at 27k), and in rounds of 128: 253 at 1M, 2,060 at 8M.
 //
 // A run whose sequence does not fit the pool (pile-ups, or a walk cell much wider than h) goes
 // through the same stages in segments of the sequence and stops once every list is full; its
@@ -59,7 +63,7 @@
 
 namespace akua {
 
-// Default tile shape.  At 1M particles the walk takes 273 us with 64 or 128 threads and 32 x 32
+// Default tile shape.  With culls of 32 the walk takes 273 us at 1M particles with 64 or 128 threads and 32 x 32
 // words, 294 with 32 x 48 (fewer warps fit an SM) and 404 with 32 x 16 (a warp's runs no longer
 // fit the pool at once, so the extraction runs several times with few lanes).
 constexpr int kSearchBlock = 128;
@@ -170,23 +174,31 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
         const float lz = warp_min(own ? xi.z : inf), hz = warp_min(own ? -xi.z : inf);
         __syncwarp();
         uint32_t kept = 0;
-        uint32_t jn = lane < total ? seq[lane] : 0u;
-        float4 cn = __ldg(ps + jn);
-        for (uint32_t c0 = 0; c0 < total; c0 += 32) {
-            const uint32_t j = jn;
-            const float4 c = cn;
-            const bool live = c0 + lane < total;
-            if (c0 + 32 < total) {
-                jn = c0 + 32 + lane < total ? seq[c0 + 32 + lane] : 0u;
-                cn = __ldg(ps + jn);
-            }
+        auto reach = [&](float4 c) {
             const float dx = fmaxf(fmaxf(lx - c.x, c.x + hx), 0.f);
             const float dy = fmaxf(fmaxf(ly - c.y, c.y + hy), 0.f);
             const float dz = fmaxf(fmaxf(lz - c.z, c.z + hz), 0.f);
-            const bool keep = live && len2(dx, dy, dz) < h2;
-            const uint32_t bal = __ballot_sync(kFullWarp, keep);
-            if (keep) seq[kept + __popc(bal & below)] = j;  // at or before what is still to be read
-            kept += __popc(bal);
+            return len2(dx, dy, dz) < h2;
+        };
+        constexpr int kCull = 4;  // candidates per lane and round: their loads are in flight at once
+        for (uint32_t c0 = 0; c0 < total; c0 += 32 * kCull) {
+            uint32_t j[kCull];
+            float4 c[kCull];
+#pragma unroll
+            for (int q = 0; q < kCull; ++q) {
+                const uint32_t at = c0 + 32 * q + lane;
+                j[q] = at < total ? seq[at] : 0u;
+                c[q] = __ldg(ps + j[q]);
+            }
+            __syncwarp();  // what is kept goes where this round's candidates were read
+#pragma unroll
+            for (int q = 0; q < kCull; ++q) {
+                if (c0 + 32 * q >= total) break;
+                const bool keep = c0 + 32 * q + lane < total && reach(c[q]);
+                const uint32_t bal = __ballot_sync(kFullWarp, keep);
+                if (keep) seq[kept + __popc(bal & below)] = j[q];
+                kept += __popc(bal);
+            }
         }
         __syncwarp();
         uint2* put = reinterpret_cast<uint2*>(seq + ((kept + 1u) & ~1u));
