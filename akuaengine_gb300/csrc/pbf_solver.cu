@@ -32,7 +32,7 @@ using akua::StepParams;
 struct akua_pbf {
     int device = 0;
     int sms = 1;  // multiprocessors of the device
-    int cluster_limit = 0;  // particles a cluster's sort passes take
+    bool cluster_sort = false;  // a sort pass is one cluster
     int n = 0;
     akua_pbf_config cfg{};
     akua_lambda_corr_params corr{};
@@ -485,7 +485,7 @@ void invalidate_graph(akua_pbf* s) {
 
 void update_plans(akua_pbf* s, int sp_bits) {
     // one scene of few particles: a pass is one cluster; a batch holds many scenes' particles
-    const bool small = s->scenes.empty() && s->n <= s->cluster_limit;
+    const bool small = s->scenes.empty() && s->cluster_sort;
     auto plan = [&](int bits) {
         if (small) return akua::radix::make_cluster_plan(bits);
         akua::radix::Plan p = akua::radix::make_plan(bits);
@@ -658,7 +658,7 @@ int create_solver(int32_t n, const akua_pbf_config* cfg, const akua_lambda_corr_
     s->table_alloc = s->table_size;
     cudaGetDevice(&s->device);
     cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device);
-    s->cluster_limit = akua::radix::cluster_limit<true>();
+    s->cluster_sort = akua::radix::takes_cluster(s->n, akua::radix::places_16<true>);
     std::vector<uint16_t> sid;
     if (scenes) {
         s->scenes.assign(scenes, scenes + num_scenes);

@@ -531,11 +531,10 @@ inline void run_cluster_pass(cudaStream_t s, const uint32_t* kin, const uint32_t
     mark("radix_cluster_pass");
 }
 
-// The largest input a cluster's passes can take on the current device: kClusterMax where it places
-// clusters of 16 blocks (beyond the portable 8, so the kernels must be allowed them), else
-// kClusterPortableMax.
+// Whether the current device places clusters of 16 blocks (beyond the portable 8, so the kernels must
+// be allowed them first).
 template <bool RUNS>
-inline int cluster_limit() {
+inline bool places_16() {
     auto allow = [](auto kernel) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     };
@@ -555,7 +554,13 @@ inline int cluster_limit() {
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveClusters(&clusters, cluster_pass<16, 8, RUNS>, &cfg);
     if (e != cudaSuccess) cudaGetLastError();
-    return e == cudaSuccess && clusters > 0 ? kClusterMax : kClusterPortableMax;
+    return e == cudaSuccess && clusters > 0;
+}
+
+// Whether a sort of n pairs takes a cluster's passes; `places` is asked only where 16 blocks would run.
+template <class Places>
+inline bool takes_cluster(int n, Places&& places) {
+    return n <= kClusterPortableMax || (n <= kClusterMax && places());
 }
 
 // Scratch words the sort needs for n keys: the count matrix and a pass's digit totals.
@@ -564,7 +569,7 @@ inline size_t scratch_words(int n) {
 }
 
 // Sorts (k0, v0) by the low plan bits, ping-ponging with (k1, v1); all four buffers hold n words (a
-// cluster plan: n <= cluster_limit()).  With `index_payload` the input payload is each key's index and v0 is not read.  The result
+// cluster plan: takes_cluster(n)).  With `index_payload` the input payload is each key's index and v0 is not read.  The result
 // buffers are returned through keys_out / vals_out.  With `rank_out` (n words), the last pass
 // also writes rank_out[payload] = output position.  `mark(name)` is called after every kernel.
 template <class Mark>

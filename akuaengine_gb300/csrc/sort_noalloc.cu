@@ -52,13 +52,13 @@ namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
 uint32_t* g_scratch[kMaxDevices] = {};
-int g_cluster_limit[kMaxDevices] = {};  // pairs a cluster's passes take there
+int g_places_16[kMaxDevices] = {};  // clusters of 16 blocks there: 0 not asked yet, 1 yes, 2 no
 
 // Device address of g_sort_scratch on the current device, looked up on the first call per device
 // and kept for the life of the process (a cudaDeviceReset between calls is not supported: it
 // unloads the module that holds the array).  In host code the array's name is only a host-side
 // stand-in; the kernels need this address.
-cudaError_t scratch_address(uint32_t** out, int* cluster_limit) {
+cudaError_t scratch_address(uint32_t** out, int n, bool* cluster) {
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -69,10 +69,12 @@ cudaError_t scratch_address(uint32_t** out, int* cluster_limit) {
         e = cudaGetSymbolAddress(&p, g_sort_scratch);
         if (e != cudaSuccess) return e;
         g_scratch[dev] = static_cast<uint32_t*>(p);
-        g_cluster_limit[dev] = akua::radix::cluster_limit<false>();
     }
     *out = g_scratch[dev];
-    *cluster_limit = g_cluster_limit[dev];
+    *cluster = akua::radix::takes_cluster(n, [dev] {
+        if (!g_places_16[dev]) g_places_16[dev] = akua::radix::places_16<false>() ? 1 : 2;
+        return g_places_16[dev] == 1;
+    });
     return cudaSuccess;
 }
 
@@ -93,17 +95,16 @@ extern "C" int akua_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* 
         overlap(vals_in, vals_out, bytes))
         return AKUA_ERR_INVALID_ARGUMENT;
     uint32_t* scratch = nullptr;
-    int cluster_limit = 0;
-    cudaError_t e = scratch_address(&scratch, &cluster_limit);
+    bool cluster = false;
+    cudaError_t e = scratch_address(&scratch, n, &cluster);
     if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? AKUA_ERR_OUT_OF_MEMORY : AKUA_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint32_t* tmp_keys = scratch;
     uint32_t* tmp_vals = scratch + kMaxPairs;
     uint32_t* counts = scratch + 2 * (size_t)kMaxPairs;
     uint32_t* totals = counts + (size_t)akua::radix::MAX_RADIX * akua::radix::num_tiles(n);
-    const akua::radix::Plan plan = n <= cluster_limit
-                                       ? akua::radix::make_cluster_plan(key_bits)
-                                       : akua::radix::make_plan(key_bits);
+    const akua::radix::Plan plan =
+        cluster ? akua::radix::make_cluster_plan(key_bits) : akua::radix::make_plan(key_bits);
     const bool fused = akua::radix::num_tiles(n) <= akua::radix::kFusedTiles;
     NoMark mark;
     // pass p writes to the caller's output when (passes - 1 - p) is even, so the last pass does
