@@ -143,6 +143,45 @@ struct Terms {
     float2 v[N];
 };
 
+// for_each_neighbour with 2 or 4 lanes per particle: entries(e) gives the list's entries e and e + 1
+// (e even and below c).
+template <int LANES, int N, class E, class L, class T, class A>
+__device__ __forceinline__ void lanes_add(int i, int c, E&& entries, L&& load, T&& term, A&& add) {
+    constexpr int kStep = 2 * LANES;  // entries per step
+    const int role = threadIdx.x & (LANES - 1);
+    const int group = (threadIdx.x & 31) & ~(LANES - 1);
+    const int steps = __reduce_max_sync(0xffffffffu, (unsigned)((c + kStep - 1) / kStep));
+    auto pair = [&](int s, uint32_t& j0, uint32_t& j1) {  // this lane's entries of step s
+        const int e = kStep * s + 2 * role;
+        j0 = j1 = (uint32_t)i;
+        if (e < c) {
+            const uint2 t = entries(e);
+            j0 = t.x;
+            j1 = e + 1 < c ? t.y : t.x;
+        }
+    };
+    uint32_t j0, j1;
+    pair(0, j0, j1);
+    auto ra = load(j0), rb = load(j1);
+    pair(1, j0, j1);
+    for (int s = 0; s < steps; ++s) {
+        const Terms<N> t = term(ra, rb);
+        if (s + 1 < steps) {
+            ra = load(j0);
+            rb = load(j1);
+            pair(s + 2, j0, j1);
+        }
+#pragma unroll
+        for (int k = 0; k < kStep; ++k) {
+            float one[N];
+#pragma unroll
+            for (int q = 0; q < N; ++q)
+                one[q] = __shfl_sync(0xffffffffu, (k & 1) ? t.v[q].y : t.v[q].x, group + (k >> 1));
+            if (kStep * s + k < c) add(one);
+        }
+    }
+}
+
 // Calls add(t, k) with the N terms t[] of each neighbour of particle i, in list order: load(j)
 // gathers a neighbour's record, term(a, b) evaluates two of them.  With LANES = 1 a thread works
 // through its particle's list by itself.  With 2 or 4 lanes per particle each lane gathers and
@@ -167,40 +206,13 @@ __device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr
             }
         });
     } else {
-        constexpr int E = 2 * LANES;  // entries per step
-        const int role = threadIdx.x & (LANES - 1);
-        const int group = (threadIdx.x & 31) & ~(LANES - 1);
-        const int steps = __reduce_max_sync(0xffffffffu, (unsigned)((c + E - 1) / E));
-        auto pair = [&](int s, uint32_t& j0, uint32_t& j1) {  // this lane's entries of step s
-            const int e = E * s + 2 * role;
-            j0 = j1 = (uint32_t)i;
-            if (e < c) {
+        lanes_add<LANES, N>(
+            i, c,
+            [&](int e) {
                 const uint2* at = reinterpret_cast<const uint2*>(nbr4 + (size_t)(e >> 2) * n + i);
-                const uint2 t = __ldg(at + ((e >> 1) & 1));
-                j0 = t.x;
-                j1 = e + 1 < c ? t.y : t.x;
-            }
-        };
-        uint32_t j0, j1;
-        pair(0, j0, j1);
-        auto ra = load(j0), rb = load(j1);
-        pair(1, j0, j1);
-        for (int s = 0; s < steps; ++s) {
-            const Terms<N> t = term(ra, rb);
-            if (s + 1 < steps) {
-                ra = load(j0);
-                rb = load(j1);
-                pair(s + 2, j0, j1);
-            }
-#pragma unroll
-            for (int k = 0; k < E; ++k) {
-                float one[N];
-#pragma unroll
-                for (int q = 0; q < N; ++q)
-                    one[q] = __shfl_sync(0xffffffffu, (k & 1) ? t.v[q].y : t.v[q].x, group + (k >> 1));
-                if (E * s + k < c) add(one);
-            }
-        }
+                return __ldg(at + ((e >> 1) & 1));
+            },
+            load, term, add);
     }
 }
 

@@ -74,8 +74,19 @@ constexpr int kListStage = 32;
 // 8 (16, 24) particles still all fit the chip at once (32 warps per SM of 64 registers a thread, 24 of
 // the exact variant's 80) takes them.  Measured (us, at 8 / 16 / 24 / 32): 1,000 particles 18 / 21 / - /
 // 25, 27,000 26 / 27 / - / 30, 50,000 39 / 31 / - / 36, 70,000 48 / 36 / - / 40, 100,000 63 / 52 / 41 /
-// 44, and 100,000 in exact math, where 24 no longer fit, - / - / 63 / 53.
+// 44, and 100,000 in exact math, where 24 no longer fit, - / - / 63 / 53.  Fewer than 8 up to 12 warps
+// per SM: with 1, 2, 4 and 8 particles per warp 1,000 take 13.9 / 14.2 / 14.6 / 16.3 us, 4,000 - / 16.0 /
+// 15.9 / 16.4, 9,000 (4, 6 and 8) 17.8 / 17.5 / 18.1, 16,000 22.3 / 20.2 / 20.2.
+//
+// FEW (exact math, at most 8 particles per warp): four lanes turn a particle's masks into its list,
+// which then lies in the pool, and evaluate its terms as the pair kernels do with four lanes.  Exact
+// terms take the longest part of such a walk, a list's one after another (us before and after:
+// 1,000 particles 20.5 and 15.5, 9,000 24.1 and 20.1, 27,000 30.0 and 24.9).  In fast math the
+// longer code costs what the lanes gain (1,000: 13.9 and 14.2, 27,000: 23.3 and 23.9).
+constexpr int kFewPerWarp = 8;
 inline int search_per_warp(int n, int sms, bool exact) {
+    const int most = 12 * sms;  // warps
+    if (n <= kFewPerWarp * most) return (n + most - 1) / most;
     const int warps = (exact ? 24 : 32) * sms;
     for (int w = 8; w < 32; w += 8)
         if (n <= w * warps) return w;
@@ -98,7 +109,7 @@ __device__ __forceinline__ float warp_min(float v) {
     return r;
 }
 
-template <bool EXACT, int BLOCK, int STAGE>
+template <bool EXACT, int BLOCK, int STAGE, bool FEW>
 __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
     k_search(const StepParams* __restrict__ P, const float4* __restrict__ ps,
              const uint2* __restrict__ table, const uint32_t* __restrict__ r2i,
@@ -262,8 +273,8 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
             return j;
         }
     };
-    // Density, lambda and the network's features of this lane's finished list.
-    auto finish = [&](const DensityLambda2<EXACT>& acc, int count) {
+    // Density, lambda and the network's features of a particle's finished list.
+    auto finish = [&](const DensityLambda2<EXACT>& acc, int count, int i, float4 xi) {
         rho_out[i] = acc.rho;
         const float l = acc.lambda(p);
         lam_out[i] = l;
@@ -350,7 +361,7 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
                                                         __ldg(ps + (left >= 4 ? t.w : t.z)),
                                                         left >= 4);
                         }
-                        finish(acc, count);
+                        finish(acc, count, i, xi);
                     }
                 }
                 if (rest) e_next = lookup(rest);
@@ -385,6 +396,69 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
             starts = rest;
         }
 
+        if constexpr (FEW) {  // four lanes per particle, through lists in the pool
+            const int src = lane >> 2, role = lane & 3;
+            const int q0 = __shfl_sync(kFullWarp, my_q0, src);
+            const uint32_t kept = __shfl_sync(kFullWarp, my_kept, src);  // 0 without a run in the pool
+            const int m = __shfl_sync(kFullWarp, my_m, src);
+            const uint32_t* seq = pool + __shfl_sync(kFullWarp, my_seq, src);
+            const uint2* mask = reinterpret_cast<const uint2*>(seq + ((kept + 1u) & ~1u)) + (src - q0);
+            int total = 0;
+            for (uint32_t k = 0; 64 * k < kept; ++k) {
+                const uint2 w = mask[k * m];
+                total += __popc(w.x) + __popc(w.y);
+            }
+            const int count = min(total, cap);
+            const int room = (int)((__reduce_max_sync(kFullWarp, (unsigned)count) + 3u) & ~3u);
+            const int lists = (int)((used + 3u) & ~3u);
+            if (lists + 8 * room <= (int)kPool) {
+                uint32_t* list = pool + lists + src * room;
+                int at = 0;
+                for (uint32_t k = 0; 64 * k < kept; ++k) {  // a lane places every fourth chunk's hits
+                    const uint2 w = mask[k * m];
+                    const uint32_t first = role == (int)(2 * k & 3) ? w.x : 0u;
+                    const uint32_t second = role == (int)(2 * k + 1 & 3) ? w.y : 0u;
+                    uint32_t bits = first | second;
+                    const uint32_t* from = seq + 64 * k + (first ? 0 : 32);
+                    for (int to = first ? at : at + __popc(w.x); bits; bits &= bits - 1, ++to)
+                        if (to < count) list[to] = from[__ffs(bits) - 1];
+                    at += __popc(w.x) + __popc(w.y);
+                }
+                __syncwarp();
+                const int ip = min(base + src, n - 1);
+                for (int g = role; 4 * g < count; g += 4) {
+                    uint4 t = *reinterpret_cast<const uint4*>(list + 4 * g);
+                    const int left = count - 4 * g;  // a partial last tile repeats its last entry
+                    if (left < 2) t.y = t.x;
+                    if (left < 3) t.z = t.y;
+                    if (left < 4) t.w = t.z;
+                    out4[(size_t)g * n + ip] = t;
+                }
+                const float4 xp = make_float4(
+                    __shfl_sync(kFullWarp, xi.x, src), __shfl_sync(kFullWarp, xi.y, src),
+                    __shfl_sync(kFullWarp, xi.z, src), __shfl_sync(kFullWarp, xi.w, src));
+                const bool writes = role == 0 && q0 >= 0;
+                if (writes) {
+                    if (total >= cap) atomicOr(flags, 1u);
+                    cnt[ip] = (uint32_t)count;
+                }
+                if (density) {
+                    DensityLambda2<EXACT> acc;
+                    acc.init(xp.w, p);
+                    lanes_add<4, 6>(
+                        ip, count,
+                        [&](int e) { return *reinterpret_cast<const uint2*>(list + e); },
+                        [&](uint32_t j) { return __ldg(ps + j); },
+                        [&](float4 a, float4 b) {
+                            return DensityLambda2<EXACT>::template terms<true>(p, xp, a, b);
+                        },
+                        acc);
+                    if (writes) finish(acc, count, ip, xp);
+                }
+                __syncwarp();
+                continue;
+            }
+        }
         // extract the lists of the runs in the pool, one lane per particle
         if (my_q0 >= 0) {
             Hits hits(pool + my_seq, my_kept, lane - my_q0, my_m);
@@ -411,7 +485,7 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
                     if (left > 2) acc.template add2<true>(p, xi, c, d, left >= 4);
                 }
             }
-            if (density) finish(acc, count);
+            if (density) finish(acc, count, i, xi);
         }
         __syncwarp();
     }

@@ -330,14 +330,16 @@ void step_kernel(const akua_pbf* s, cudaStream_t st, void (*kernel)(Params...), 
 template <bool EXACT, int BLOCK, int STAGE>
 void launch_search_shape(akua_pbf* s, cudaStream_t st, int density, float* feat) {
     constexpr size_t smem = akua::search_smem(BLOCK, STAGE);
-    if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
-        cudaFuncSetAttribute(akua::k_search<EXACT, BLOCK, STAGE>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int per_warp = akua::search_per_warp(s->n, s->sms, EXACT);
-    step_kernel(s, st, akua::k_search<EXACT, BLOCK, STAGE>,
-                grid_for(s->n, per_warp * (BLOCK / 32)), BLOCK, smem, s->d_params,
-                s->ps0, s->table, s->r2i, s->nbr, s->cnt, s->rho, s->lam, s->flags, density,
-                s->speed, s->lprev, s->lacc, feat, s->psl, per_warp);
+    auto go = [&](auto kernel) {
+        if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        step_kernel(s, st, kernel, grid_for(s->n, per_warp * (BLOCK / 32)), BLOCK, smem, s->d_params,
+                    s->ps0, s->table, s->r2i, s->nbr, s->cnt, s->rho, s->lam, s->flags, density,
+                    s->speed, s->lprev, s->lacc, feat, s->psl, per_warp);
+    };
+    if (EXACT && per_warp <= akua::kFewPerWarp) go(akua::k_search<EXACT, BLOCK, STAGE, EXACT>);
+    else go(akua::k_search<EXACT, BLOCK, STAGE, false>);
 }
 
 template <bool EXACT>

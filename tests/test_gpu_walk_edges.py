@@ -25,15 +25,17 @@ def first_of_block(n, seed):
     return sc
 
 
-@pytest.mark.parametrize("where", [9, 31, 33, 65, "8-", "8+", "16-", "16+", "24-", "24+"])
+@pytest.mark.parametrize("where", [9, 31, 33, 65, "0.5-", "0.5+", "4-", "4+", "8-", "8+", "16-", "16+", "24-",
+                                   "24+"])
 def test_particles_per_warp_edges(where):
-    """Counts around a warp and around the lines where the walk goes from 8 to 16, 24 and 32
-    particles per warp (8 x 24, 16 x 24 and 24 x 24 per multiprocessor in exact math)."""
+    """Counts around a warp and around the lines where the walk goes from 1 to 2 particles per warp
+    and reaches 8 (1 x 12 and 8 x 12 per multiprocessor), then 16, 24 and 32 (8 x 24, 16 x 24 and
+    24 x 24 in exact math)."""
     if isinstance(where, str):
         import torch
 
         sms = torch.cuda.get_device_properties(0).multi_processor_count
-        n = int(where[:-1]) * 24 * sms + (1 if where.endswith("+") else 0)
+        n = int(float(where[:-1]) * 24 * sms) + (1 if where.endswith("+") else 0)
     else:
         n = where
     sc = first_of_block(n, seed=n)
