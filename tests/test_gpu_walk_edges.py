@@ -107,3 +107,26 @@ def test_lanes_per_particle_edges(where, exact):
         out.append(own[np.lexsort((own["color"][:, 0],))])
     assert len(out[0]) == n == len(out[1])
     assert_records_bitexact(out[1], out[0])
+
+
+@pytest.mark.parametrize("table_size", [None, 64], ids=["cells", "shared_buckets"])
+def test_sparse_runs(table_size):
+    """Spray: lone particles, pairs in one cell and in neighbouring cells, and clusters whose sequences
+    lie around the 64 candidates that are tested without a cull; buckets of one cell each, and a
+    table so small that lone particles find others in their buckets."""
+    rng = np.random.default_rng(3)
+    sc = first_of_block(1300, seed=3)
+    pos = sc.particles["position"]
+    pos[:] = rng.uniform(0.3, 5.7, pos.shape)  # 27,000 cells
+    pos[100:300] = pos[300:500] + rng.uniform(-0.08, 0.08, (200, 3)).astype(np.float32)
+    at = 600
+    for k, size in enumerate((31, 32, 33, 63, 64, 65, 66, 128, 129)):
+        corner = 0.5 + 0.6 * k
+        pos[at:at + size] = corner + rng.uniform(0.005, 0.095, (size, 3))
+        at += size
+    sc.box_min, sc.box_max = (0.0, 0.0, 0.0), (6.0, 6.0, 6.0)
+    cfg, corr = PBFConfig(), LambdaCorrParams()
+    o, oe = run_oracle(sc, cfg, corr, 1, table_size=table_size)
+    g, ge = run_gpu(sc, cfg, corr, 1, ak.OPT_EXACT_MATH, table_size=table_size)
+    assert_grid_equal(ge, oe, cfg.maxNeighbours)
+    assert_records_bitexact(g, o)
