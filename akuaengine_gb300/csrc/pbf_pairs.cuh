@@ -143,7 +143,7 @@ struct Terms {
     float2 v[N];
 };
 
-// for_each_neighbour with 2 or 4 lanes per particle: entries(e) gives the list's entries e and e + 1
+// for_each_neighbour with 2, 4 or 8 lanes per particle: entries(e) gives the list's entries e and e + 1
 // (e even and below c).
 template <int LANES, int N, class E, class L, class T, class A>
 __device__ __forceinline__ void lanes_add(int i, int c, E&& entries, L&& load, T&& term, A&& add) {
@@ -184,10 +184,10 @@ __device__ __forceinline__ void lanes_add(int i, int c, E&& entries, L&& load, T
 
 // Calls add(t, k) with the N terms t[] of each neighbour of particle i, in list order: load(j)
 // gathers a neighbour's record, term(a, b) evaluates two of them.  With LANES = 1 a thread works
-// through its particle's list by itself.  With 2 or 4 lanes per particle each lane gathers and
-// evaluates its own pair of every 4 or 8 entries, the next one's records in flight, and the lanes
-// hand their terms round by shuffles, so that every lane adds all of them in list order (the sums are
-// the same bit for bit) and a list takes a half or a quarter of the steps.  All lanes of a warp call
+// through its particle's list by itself.  With 2, 4 or 8 lanes per particle each lane gathers
+// and evaluates its own pair of every 4, 8 or 16 entries, the next one's records in flight, and the
+// lanes hand their terms round by shuffles, so that every lane adds all of them in list order (the
+// sums are the same bit for bit) and a list takes a half, a quarter or an eighth of the steps.  All lanes of a warp call
 // it (c = 0 for lanes without a particle).
 template <int LANES, bool WHOLE_TILE, int N, class L, class T, class A>
 __device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr4, int n, int i, int c,
@@ -218,12 +218,15 @@ __device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr
 
 // Lanes per particle of the pair kernels.  A scene too small to fill the chip is as slow as the chain
 // of gathers of one list, which more lanes shorten, until the shuffles cost more issue slots than the
-// chain costs time: about 16 warps per SM with 4 lanes (24 with exact math, whose terms are longer)
-// and 18 with 2.  Steps in us with 1 / 2 / 4 lanes: 1,000 particles 95 / 95 / 84, 8,000 121 / 108 /
+// chain costs time: about 10 warps per SM with 8 lanes (22 with exact math, whose terms are longer),
+// 16 (24) with 4 and 18 with 2.  Steps in us with 1 / 2 / 4 lanes: 1,000 particles 95 / 95 / 84, 8,000 121 / 108 /
 // 96, 27,000 139 / 128 / 132 (exact 207 / 181 / 160), 40,000 156 / 151 / 176 (exact 226 / 205 / 216),
-// 60,000 167 / 176 / 208.
+// 60,000 167 / 176 / 208.  With 4 / 8 / 16 lanes, the other kernels being faster by then: 1,000
+// particles 70 / 66 / 68, 4,000 80 / 77 / 84, 6,000 82.6 / 82.2 / 92, 8,000 85 / 87; exact 1,000
+// 88 / 75 / 72, 4,000 105 / 89 / 92, 12,000 118 / 109, 16,000 124 / 132.
 inline int pair_lanes(int n, int sms, bool exact) {
     const long long warps = 32ll * sms;  // threads of one warp per SM
+    if (8ll * n <= (exact ? 22 : 10) * warps) return 8;
     if (4ll * n <= (exact ? 24 : 16) * warps) return 4;
     return 2ll * n <= 18 * warps ? 2 : 1;
 }

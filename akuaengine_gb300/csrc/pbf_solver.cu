@@ -458,6 +458,9 @@ void enqueue_body(akua_pbf* s, cudaStream_t st, const char* aos, size_t stride, 
     mark("k_table_build");
     const bool exact = (s->options & AKUA_PBF_OPT_EXACT_MATH) != 0;
     switch (akua::pair_lanes(n, s->sms, exact)) {
+        case 8:
+            exact ? enqueue_pairs<true, 8>(s, st, mark) : enqueue_pairs<false, 8>(s, st, mark);
+            break;
         case 4:
             exact ? enqueue_pairs<true, 4>(s, st, mark) : enqueue_pairs<false, 4>(s, st, mark);
             break;

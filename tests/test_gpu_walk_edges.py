@@ -73,16 +73,17 @@ def test_runs_longer_than_the_pool(shape, kind):
 
 
 @pytest.mark.parametrize("exact", [True, False], ids=["exact", "fast"])
-@pytest.mark.parametrize("where", ["4-", "4+", "2-", "2+"])
+@pytest.mark.parametrize("where", ["8-", "8+", "4-", "4+", "2-", "2+"])
 def test_lanes_per_particle_edges(where, exact):
-    """Both sides of the lines where the pair kernels go from 4 to 2 and from 2 to 1 lanes per particle,
+    """Both sides of the lines where the pair kernels go from 8 to 4, 2 and 1 lanes per particle,
     with two masses.  Exact math: the oracle's records; fast math: those of the same particles
     stepped in a scene beyond every line (a far-away block makes up the number), whose kernels
     use one lane."""
     import torch
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    per = {"4": (24 if exact else 16) * 32 * sms // 4, "2": 18 * 32 * sms // 2}[where[0]]
+    per = {"8": (22 if exact else 10) * 32 * sms // 8, "4": (24 if exact else 16) * 32 * sms // 4,
+           "2": 18 * 32 * sms // 2}[where[0]]
     n = per + (1 if where.endswith("+") else 0)
     sc = first_of_block(n, seed=7)
     sc.particles["mass"][::3] = 0.8
