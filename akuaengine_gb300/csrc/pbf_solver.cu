@@ -492,7 +492,7 @@ void update_plans(akua_pbf* s, int sp_bits) {
     // one scene of few particles: a pass is one cluster; a batch holds many scenes' particles
     const bool small = s->scenes.empty() && s->cluster_sort;
     auto plan = [&](int bits) {
-        if (small) return akua::radix::make_cluster_plan(bits);
+        if (small) return akua::radix::make_cluster_plan(bits, s->n);
         akua::radix::Plan p = akua::radix::make_plan(bits);
         p.fused = s->scenes.empty() && akua::radix::num_tiles(s->n) <= akua::radix::kFusedTiles;
         return p;

@@ -372,21 +372,26 @@ inline void run_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, u
 // no work.  Here one cluster holds all pairs in registers: a block ranks its own (match.any and
 // per-warp digit counters, as downsweep does), reads the other blocks' digit totals through
 // distributed shared memory, scans them and scatters to global memory.
-// Sorts of random keys in three passes: 27,000 pairs 56 -> 18 us, 65,536 34 -> 24; in two, 4,096: 39 -> 8.
-// The step of 27,000 particles: 158 -> 131 us.
-constexpr int kClusterThreads = 512;  // one thread per digit in the scans
+// Sorts of random keys in three passes: 27,000 pairs 56 -> 16.5 us, 65,536 34 -> 24; in two, 4,096:
+// 39 -> 7.  The step of 27,000 particles: 158 -> 129 us.  (With 32-bit counters 27,000 took 17.9 us and
+// 4,096 7.8: the scan over the warps' counters and their zeroing are twice the shared memory.)
+constexpr int kClusterThreads = 512;
 constexpr int kClusterWarps = kClusterThreads / 32;
-constexpr int kClusterBits = 9;
-constexpr int kClusterRadix = 1 << kClusterBits;
 constexpr int kClusterMax = 16 * kClusterThreads * 8;         // 65,536: eight rounds of 16 blocks
 constexpr int kClusterPortableMax = 8 * kClusterThreads * 4;  // 16,384: four rounds of 8 blocks
-static_assert(kClusterRadix == kClusterThreads, "thread d scans digit d");
 
-inline Plan make_cluster_plan(int bits) {
+// Digits of up to 9 bits (one per thread in the scans), or of up to 11 (four) where that saves a pass
+// of 8 blocks and two or four rounds: 8,192 pairs of 19 bits 13.0 -> 10.6 us, 16,384 of 20 16.1 ->
+// 14.8.  16 blocks read twice the counts from one another (27,000 of 21 bits 17.8 -> 19.6, 65,536 of
+// 32 32.6 -> 35.3).  One round would gain little (4,096 of 20 bits 11.2 -> 10.4), and the tests hold
+// a step of 4,096 particles to 20 launches.
+inline Plan make_cluster_plan(int bits, int n) {
     Plan p;
     p.cluster = true;
     if (bits < 1) bits = 1;
-    p.passes = (bits + kClusterBits - 1) / kClusterBits;
+    const bool wide = n > 8 * kClusterThreads && n <= kClusterPortableMax;
+    const int most = wide && (bits + 8) / 9 > (bits + 10) / 11 ? 11 : 9;
+    p.passes = (bits + most - 1) / most;
     for (int k = 0, shift = 0; k < p.passes; ++k) {
         p.shift[k] = shift;
         p.width[k] = (bits - shift + (p.passes - k) - 1) / (p.passes - k);
@@ -395,11 +400,42 @@ inline Plan make_cluster_plan(int bits) {
     return p;
 }
 
-__device__ __forceinline__ uint32_t ld_remote(const uint32_t* p, uint32_t rank) {
-    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), v;
+// Counts of up to 4,096 pairs, 16 bits each: a thread's PER neighbouring digits in one access.
+template <int PER>
+struct Counts;
+template <>
+struct Counts<1> {
+    uint16_t w;
+    __device__ __forceinline__ uint32_t operator[](int) const { return w; }
+    __device__ __forceinline__ void operator+=(Counts o) { w += o.w; }
+};
+template <>
+struct __align__(8) Counts<4> {
+    uint32_t w[2];
+    __device__ __forceinline__ uint32_t operator[](int k) const {
+        return (k & 1) ? w[k >> 1] >> 16 : w[k >> 1] & 0xffffu;
+    }
+    __device__ __forceinline__ void operator+=(Counts o) {  // no half overflows
+        w[0] += o.w[0];
+        w[1] += o.w[1];
+    }
+};
+__device__ __forceinline__ Counts<1> ld_remote(const Counts<1>* p, uint32_t rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    Counts<1> c;
     asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(a) : "r"(rank));
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return v;
+    asm volatile("ld.shared::cluster.u16 %0, [%1];" : "=h"(c.w) : "r"(a) : "memory");
+    return c;
+}
+__device__ __forceinline__ Counts<4> ld_remote(const Counts<4>* p, uint32_t rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    Counts<4> c;
+    asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(a) : "r"(rank));
+    asm volatile("ld.shared::cluster.v2.u32 {%0,%1}, [%2];"
+                 : "=r"(c.w[0]), "=r"(c.w[1])
+                 : "r"(a)
+                 : "memory");
+    return c;
 }
 __device__ __forceinline__ void cluster_arrive() {
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
@@ -408,28 +444,42 @@ __device__ __forceinline__ void cluster_wait() {
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
-// One pass over the digit (key >> shift) & digit_mask, digit_mask < kClusterRadix.  Block b holds
-// the pairs from b * 512 * ROUNDS on; warp w of it 32 * ROUNDS of them, in rounds of 32.
-template <int BLOCKS, int ROUNDS, bool RUNS>
+// Dynamic shared memory of a block: the per-warp counters, whose space its pairs take once every pair
+// knows its place in the block, two words per digit, and the block's counts for the others.
+__host__ __device__ constexpr size_t cluster_smem(int bits, int pairs) {
+    const size_t a = (sizeof(uint16_t) * kClusterWarps) << bits, b = sizeof(uint2) * pairs;
+    return (a > b ? a : b) + ((2 * sizeof(uint32_t) + sizeof(uint16_t)) << bits);
+}
+
+// One pass over the digit (key >> shift) & digit_mask, digit_mask < 1 << BITS.  Block b holds the
+// pairs from b * 512 * ROUNDS on; warp w of it 32 * ROUNDS of them, in rounds of 32.
+template <int BITS, int BLOCKS, int ROUNDS, bool RUNS>
 __global__ void __launch_bounds__(kClusterThreads)
     cluster_pass(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                  uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n, int shift,
                  uint32_t digit_mask, uint32_t* __restrict__ rank_out) {
-    constexpr int kPer = kClusterThreads * ROUNDS;
+    constexpr int kPairs = kClusterThreads * ROUNDS;
+    constexpr int RADIX = 1 << BITS;
+    constexpr int PER = RADIX / kClusterThreads;  // digits per thread in the scans
+    static_assert(kPairs <= 4096, "a block's counts fit 16 bits");
     extern __shared__ __align__(16) uint8_t scatter_raw[];
-    uint32_t(*count)[kClusterRadix] = reinterpret_cast<uint32_t(*)[kClusterRadix]>(scatter_raw);
-    uint2* pair = reinterpret_cast<uint2*>(scatter_raw);  // [kPer], once the counters are done with
+    uint16_t(*count)[RADIX] = reinterpret_cast<uint16_t(*)[RADIX]>(scatter_raw);
+    uint2* pair = reinterpret_cast<uint2*>(scatter_raw);  // [kPairs], once the counters are done with
     uint32_t* start = reinterpret_cast<uint32_t*>(
-        scatter_raw + scatter_smem(kClusterWarps, kClusterRadix, kPer) -
-        2 * sizeof(uint32_t) * kClusterRadix);
-    uint32_t* to = start + kClusterRadix;  // digit's output position minus its place in the block
-    __shared__ uint32_t total[kClusterRadix];  // this block's pairs per digit, read by the others
+        scatter_raw + cluster_smem(BITS, kPairs) - (2 * sizeof(uint32_t) + sizeof(uint16_t)) * RADIX);
+    uint32_t* to = start + RADIX;  // digit's output position minus its place in the block
+    // this block's pairs per digit, read by the others
+    Counts<PER>* total = reinterpret_cast<Counts<PER>*>(to + RADIX);
     __shared__ uint32_t sums[kClusterWarps];
     const uint32_t rank = blockIdx.x;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int first = (int)rank * kPer + warp * (32 * ROUNDS) + lane;
+    const int first = (int)rank * kPairs + warp * (32 * ROUNDS) + lane;
     const uint32_t below = (1u << lane) - 1u;
     uint32_t key[ROUNDS], val[ROUNDS], pos[ROUNDS];
+    uint4* zero = reinterpret_cast<uint4*>(&count[0][0]);
+#pragma unroll
+    for (int k = 0; k < kClusterWarps * RADIX / 8 / kClusterThreads; ++k)
+        zero[k * kClusterThreads + t] = make_uint4(0u, 0u, 0u, 0u);
     wait_for_previous();
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
@@ -437,48 +487,61 @@ __global__ void __launch_bounds__(kClusterThreads)
         key[r] = at < n ? keys_in[at] : 0u;
         val[r] = at < n ? (vals_in ? vals_in[at] : (uint32_t)at) : 0u;
     }
-    uint4* zero = reinterpret_cast<uint4*>(&count[0][0]);
-#pragma unroll
-    for (int k = 0; k < kClusterWarps * kClusterRadix / 4 / kClusterThreads; ++k)
-        zero[k * kClusterThreads + t] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
         const bool live = first + 32 * r < n;
         const uint32_t d = (key[r] >> shift) & digit_mask;
         const uint32_t peers = RUNS ? __match_any_sync(0xffffffffu, live ? d : 0xffffffffu)
-                                    : same_digit<kClusterBits>(d, live);
+                                    : same_digit<BITS>(d, live);
         uint32_t before = 0;
         if (live) before = count[warp][d];
         __syncwarp();
-        if (live && lane == __ffs(peers) - 1) count[warp][d] = before + __popc(peers);
+        if (live && lane == __ffs(peers) - 1) count[warp][d] = (uint16_t)(before + __popc(peers));
         __syncwarp();
         pos[r] = before + __popc(peers & below);
     }
     __syncthreads();
-    uint32_t sum = 0;  // digit t: exclusive over the warps, then the block's total
+    Counts<PER> sum{};  // this thread's digits: exclusive over the warps, then the block's total
 #pragma unroll
     for (int w = 0; w < kClusterWarps; ++w) {
-        const uint32_t c = count[w][t];
-        count[w][t] = sum;
+        Counts<PER>* at = reinterpret_cast<Counts<PER>*>(count[w]) + t;
+        const Counts<PER> c = *at;
+        *at = sum;
         sum += c;
     }
     total[t] = sum;
     cluster_arrive();
     cluster_wait();
-    // digit t: the pairs of all blocks, and of the blocks before this one
-    uint32_t all = 0, before = 0;
+    // the pairs of all blocks, and of the blocks before this one
+    uint32_t all[PER], before[PER], mine = 0, every = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) all[k] = before[k] = 0;
 #pragma unroll
     for (uint32_t b = 0; b < BLOCKS; ++b) {
-        const uint32_t c = ld_remote(&total[t], b);
-        all += c;
-        before += b < rank ? c : 0u;
+        const Counts<PER> c = ld_remote(&total[t], b);
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            all[k] += c[k];
+            before[k] += b < rank ? c[k] : 0u;
+        }
     }
     cluster_arrive();  // this block is done with the others' totals
-    const uint32_t at = block_exclusive<kClusterWarps>(sum, sums);
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        mine += sum[k];
+        every += all[k];
+    }
+    uint32_t at = block_exclusive<kClusterWarps>(mine, sums);
     __syncthreads();  // `sums` again
-    start[t] = at;
-    to[t] = block_exclusive<kClusterWarps>(all, sums) + before - at;
+    uint32_t lower = block_exclusive<kClusterWarps>(every, sums);
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        start[t * PER + k] = at;
+        to[t * PER + k] = lower + before[k] - at;
+        at += sum[k];
+        lower += all[k];
+    }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
@@ -490,7 +553,7 @@ __global__ void __launch_bounds__(kClusterThreads)
     for (int r = 0; r < ROUNDS; ++r)
         if (first + 32 * r < n) pair[pos[r]] = make_uint2(key[r], val[r]);
     __syncthreads();
-    const int here = n - (int)rank * kPer;
+    const int here = n - (int)rank * kPairs;
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
         const int k = r * kClusterThreads + t;
@@ -515,19 +578,29 @@ inline void run_cluster_pass(cudaStream_t s, const uint32_t* kin, const uint32_t
                              Mark& mark, bool after) {
     constexpr int kRound = 8 * kClusterThreads;
     const uint32_t mask = (1u << width) - 1u;
-    auto go = [&](auto kernel, int blocks, int rounds) {
-        const size_t smem = scatter_smem(kClusterWarps, kClusterRadix, kClusterThreads * rounds);
+    auto go = [&](auto kernel, int bits, int blocks, int rounds) {
+        const size_t smem = cluster_smem(bits, kClusterThreads * rounds);
+        if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         launch(after, kernel, blocks, kClusterThreads, smem, s, blocks, kin, vin, kout, vout, n, shift,
                mask, rank_out);
     };
     // 8 blocks wait for one another sooner, 16 spread the pairs and their scattered stores over more
     // SMs.  A step with 8 and with 16: 6,000 particles 85.3 and 86.3 us, 12,000 91.1 and 91.8, 27,000
     // 115.5 and 113.9, 40,000 136.3 and 132.1, 60,000 151.5 and 147.0.
-    if (n <= kRound) go(cluster_pass<8, 1, RUNS>, 8, 1);
-    else if (n <= 2 * kRound) go(cluster_pass<8, 2, RUNS>, 8, 2);
-    else if (n <= 4 * kRound) go(cluster_pass<8, 4, RUNS>, 8, 4);
-    else if (n <= 8 * kRound) go(cluster_pass<16, 4, RUNS>, 16, 4);
-    else go(cluster_pass<16, 8, RUNS>, 16, 8);
+    if (n <= kRound) {
+        go(cluster_pass<9, 8, 1, RUNS>, 9, 8, 1);
+    } else if (n <= 2 * kRound) {
+        if (width > 9) go(cluster_pass<11, 8, 2, RUNS>, 11, 8, 2);
+        else go(cluster_pass<9, 8, 2, RUNS>, 9, 8, 2);
+    } else if (n <= 4 * kRound) {
+        if (width > 9) go(cluster_pass<11, 8, 4, RUNS>, 11, 8, 4);
+        else go(cluster_pass<9, 8, 4, RUNS>, 9, 8, 4);
+    } else if (n <= 8 * kRound) {
+        go(cluster_pass<9, 16, 4, RUNS>, 9, 16, 4);
+    } else {
+        go(cluster_pass<9, 16, 8, RUNS>, 9, 16, 8);
+    }
     mark("radix_cluster_pass");
 }
 
@@ -535,11 +608,13 @@ inline void run_cluster_pass(cudaStream_t s, const uint32_t* kin, const uint32_t
 // be allowed them first).
 template <bool RUNS>
 inline bool places_16() {
-    auto allow = [](auto kernel) {
-        return cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaError_t e = cudaSuccess;
+    auto allow = [&](auto kernel) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     };
-    cudaError_t e = allow(cluster_pass<16, 4, RUNS>);
-    if (e == cudaSuccess) e = allow(cluster_pass<16, 8, RUNS>);
+    allow(cluster_pass<9, 16, 4, RUNS>);
+    allow(cluster_pass<9, 16, 8, RUNS>);
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 16;
@@ -547,12 +622,12 @@ inline bool places_16() {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(16);
     cfg.blockDim = dim3(kClusterThreads);
-    cfg.dynamicSmemBytes = scatter_smem(kClusterWarps, kClusterRadix, kClusterThreads * 8);
+    cfg.dynamicSmemBytes = cluster_smem(9, kClusterThreads * 8);
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int clusters = 0;
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveClusters(&clusters, cluster_pass<16, 8, RUNS>, &cfg);
+        e = cudaOccupancyMaxActiveClusters(&clusters, cluster_pass<9, 16, 8, RUNS>, &cfg);
     if (e != cudaSuccess) cudaGetLastError();
     return e == cudaSuccess && clusters > 0;
 }

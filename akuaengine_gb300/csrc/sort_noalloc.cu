@@ -104,7 +104,7 @@ extern "C" int akua_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* 
     uint32_t* counts = scratch + 2 * (size_t)kMaxPairs;
     uint32_t* totals = counts + (size_t)akua::radix::MAX_RADIX * akua::radix::num_tiles(n);
     const akua::radix::Plan plan =
-        cluster ? akua::radix::make_cluster_plan(key_bits) : akua::radix::make_plan(key_bits);
+        cluster ? akua::radix::make_cluster_plan(key_bits, n) : akua::radix::make_plan(key_bits);
     const bool fused = akua::radix::num_tiles(n) <= akua::radix::kFusedTiles;
     NoMark mark;
     // pass p writes to the caller's output when (passes - 1 - p) is even, so the last pass does

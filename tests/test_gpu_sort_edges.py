@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n", [1, 31, 4095, 4096, 4097, 8192, 8193, 16384, 16385, 32768, 32769, 65536,
                                65537, 69632, 69633])
-@pytest.mark.parametrize("bits", [1, 9, 10, 19, 32])
+@pytest.mark.parametrize("bits", [1, 9, 10, 11, 19, 22, 23, 32])
 def test_sort_pairs_edges(cuda_lib, n, bits):
     """Random keys with bits above `bits`, runs of equal keys among them, arrays that start off
     a 16-byte boundary."""
