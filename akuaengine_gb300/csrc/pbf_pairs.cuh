@@ -218,17 +218,19 @@ __device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr
 
 // Lanes per particle of the pair kernels.  A scene too small to fill the chip is as slow as the chain
 // of gathers of one list, which more lanes shorten, until the shuffles cost more issue slots than the
-// chain costs time: about 10 warps per SM with 8 lanes (22 with exact math, whose terms are longer),
-// 16 (24) with 4 and 18 with 2.  Steps in us with 1 / 2 / 4 lanes: 1,000 particles 95 / 95 / 84, 8,000 121 / 108 /
+// chain costs time: about 10 warps per SM with 8 lanes (22 with exact math, whose terms are longer)
+// and 18 with 4 or 2 (24, all that fit at 80 registers).  Steps in us with 1 / 2 / 4 lanes: 1,000 particles 95 / 95 / 84, 8,000 121 / 108 /
 // 96, 27,000 139 / 128 / 132 (exact 207 / 181 / 160), 40,000 156 / 151 / 176 (exact 226 / 205 / 216),
 // 60,000 167 / 176 / 208.  With 4 / 8 / 16 lanes, the other kernels being faster by then: 1,000
 // particles 70 / 66 / 68, 4,000 80 / 77 / 84, 6,000 82.6 / 82.2 / 92, 8,000 85 / 87; exact 1,000
-// 88 / 75 / 72, 4,000 105 / 89 / 92, 12,000 118 / 109, 16,000 124 / 132.
+// 88 / 75 / 72, 4,000 105 / 89 / 92, 12,000 118 / 109, 16,000 124 / 132.  With 1 / 2 / 4: 20,000 116 /
+// 110 / 105, 27,000 120 / 111 / 114, 45,000 134 / 132, 52,000 140 / 144; exact 27,000 183 / 160 / 139,
+// 36,000 195 / 179 / 180, 52,000 210 / 196, 60,000 214 / 230.
 inline int pair_lanes(int n, int sms, bool exact) {
     const long long warps = 32ll * sms;  // threads of one warp per SM
     if (8ll * n <= (exact ? 22 : 10) * warps) return 8;
-    if (4ll * n <= (exact ? 24 : 16) * warps) return 4;
-    return 2ll * n <= 18 * warps ? 2 : 1;
+    if (4ll * n <= (exact ? 24 : 18) * warps) return 4;
+    return 2ll * n <= (exact ? 24 : 18) * warps ? 2 : 1;
 }
 
 // sum += s * (x, y, z) of each neighbour's terms (s, x, y, z), one rounding per component.

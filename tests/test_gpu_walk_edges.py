@@ -82,8 +82,8 @@ def test_lanes_per_particle_edges(where, exact):
     import torch
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    per = {"8": (22 if exact else 10) * 32 * sms // 8, "4": (24 if exact else 16) * 32 * sms // 4,
-           "2": 18 * 32 * sms // 2}[where[0]]
+    per = {"8": (22 if exact else 10) * 32 * sms // 8, "4": (24 if exact else 18) * 32 * sms // 4,
+           "2": (24 if exact else 18) * 32 * sms // 2}[where[0]]
     n = per + (1 if where.endswith("+") else 0)
     sc = first_of_block(n, seed=7)
     sc.particles["mass"][::3] = 0.8
@@ -95,7 +95,7 @@ def test_lanes_per_particle_edges(where, exact):
         assert_records_bitexact(g, o)
         return
     # one table size, so the shared particles hash alike; the filler is out of everyone's reach
-    table, extra = 1 << 24, 18 * 32 * sms
+    table, extra = 1 << 24, 24 * 32 * sms
     fill = first_of_block(extra, seed=8).particles
     fill["position"][:, 0] += sc.box_max[0] + 5.0
     box_max = (sc.box_max[0] + 40.0,) + tuple(sc.box_max[1:])
