@@ -266,33 +266,68 @@ __global__ void __launch_bounds__(kElemBlock)
 // first reference rank.  The table is all-empty between steps: k_xsph empties this step's
 // entries after the walk.
 
-// One thread per bucket start (the first reference rank carrying a hash) reads its bucket's ranks
-// (a short run of the sorted keys) and writes the entry: the length, and whether the bucket's
+// The thread of a bucket's first reference rank writes its entry: the length, and whether the bucket's
 // particles are one contiguous run of internal slots in rank order (then x = the first slot) or
 // not (several cells share the hash, or clamped cells share a Morton key: x = the first rank,
-// mixed bit set).
+// mixed bit set).  A warp reads its 32 ranks and the 32 after them at once and finds starts and
+// breaks by ballots; only a bucket that goes on beyond those is walked rank by rank.  (With a
+// thread walking each bucket, one load after another: 1M particles 14.6 -> 10.2 us, 8M 74 -> 41,
+// launch and events included; a step of 27,000 115.2 -> 113.9.)
 __global__ void __launch_bounds__(kElemBlock)
     k_table_build(const StepParams* __restrict__ P, const uint32_t* __restrict__ kr,
                   const uint32_t* __restrict__ r2i, uint2* __restrict__ table) {
+    constexpr uint32_t kAll = 0xffffffffu;
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = P->n;
+    const int lane = threadIdx.x & 31;
     after_previous_kernel();
-    if (r >= n) return;
-    const uint32_t k = kr[r];
-    if (r > 0 && kr[r - 1] == k) return;
-    const uint32_t s0 = r2i[r];
-    uint32_t prev = s0;
-    bool run = true;
-    int e = r + 1;
-    for (; e < n && kr[e] == k; ++e) {
-        const uint32_t se = r2i[e];
-        run = run && se == prev + 1u;
-        prev = se;
+    if (r - lane >= n) return;  // uniform over the warp
+    uint32_t key[2], slot[2], before = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int q = r + 32 * h;
+        key[h] = q < n ? kr[q] : 0u;
+        slot[h] = q < n ? r2i[q] : 0u;
     }
-    const uint32_t len = (uint32_t)(e - r);
-    table[k] = run ? make_uint2(s0, len) : make_uint2((uint32_t)r, len | kMixedBucket);
+    if (lane == 0 && r > 0) before = kr[r - 1];
+    // bit l: rank (warp's first) + l starts a bucket (as do all beyond the last); its slot does not
+    // follow its predecessor's
+    unsigned long long starts = 0, breaks = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int q = r + 32 * h;
+        uint32_t pk = __shfl_up_sync(kAll, key[h], 1), ps = __shfl_up_sync(kAll, slot[h], 1);
+        const uint32_t lk = __shfl_sync(kAll, key[0], 31), ls = __shfl_sync(kAll, slot[0], 31);
+        if (lane == 0) {
+            pk = h ? lk : before;
+            ps = h ? ls : 0u;  // rank r's own predecessor does not matter to a bucket starting here
+        }
+        const bool start = q >= n || q == 0 || key[h] != pk;
+        starts |= (unsigned long long)__ballot_sync(kAll, start) << (32 * h);
+        breaks |= (unsigned long long)__ballot_sync(kAll, slot[h] != ps + 1u) << (32 * h);
+    }
+    const uint32_t last = __shfl_sync(kAll, slot[1], 31);
+    if (r >= n || !((starts >> lane) & 1u)) return;
+    const unsigned long long next = starts >> (lane + 1);
+    breaks >>= lane + 1;
+    uint32_t len;
+    bool run;
+    if (next) {
+        len = (uint32_t)__ffsll((long long)next);
+        run = (breaks & ((1ull << (len - 1)) - 1)) == 0;
+    } else {  // on beyond the 64 ranks
+        run = (breaks & ((1ull << (63 - lane)) - 1)) == 0;
+        uint32_t prev = last;
+        int e = r - lane + 64;
+        for (; e < n && kr[e] == key[0]; ++e) {
+            const uint32_t se = r2i[e];
+            run = run && se == prev + 1u;
+            prev = se;
+        }
+        len = (uint32_t)(e - r);
+    }
+    table[key[0]] = run ? make_uint2(slot[0], len) : make_uint2((uint32_t)r, len | kMixedBucket);
 }
-
 
 // Writes every field of every particle into the attached records in reference order (record r
 // holds the particle of reference rank r), staged through shared memory so global writes are
