@@ -70,13 +70,16 @@ constexpr int kSearchBlock = 128;
 constexpr int kListStage = 32;
 
 // Particles per warp.  32 keep every lane of the extraction busy, but a warp works through its runs
-// one after another, so with few warps the walk lasts as long as one warp: a scene whose warps of
-// 8 (16, 24) particles still all fit the chip at once (32 warps per SM of 64 registers a thread, 24 of
-// the exact variant's 80) takes them.  Measured (us, at 8 / 16 / 24 / 32): 1,000 particles 18 / 21 / - /
-// 25, 27,000 26 / 27 / - / 30, 50,000 39 / 31 / - / 36, 70,000 48 / 36 / - / 40, 100,000 63 / 52 / 41 /
-// 44, and 100,000 in exact math, where 24 no longer fit, - / - / 63 / 53.  Fewer than 8 up to 12 warps
-// per SM: with 1, 2, 4 and 8 particles per warp 1,000 take 13.9 / 14.2 / 14.6 / 16.3 us, 4,000 - / 16.0 /
-// 15.9 / 16.4, 9,000 (4, 6 and 8) 17.8 / 17.5 / 18.1, 16,000 22.3 / 20.2 / 20.2.
+// one after another, so with few warps the walk lasts as long as one warp: a scene that would not
+// fill the chip takes fewer per warp.  In exact math 8, 16 or 24 where those warps still all fit (24
+// per SM at 80 registers; past that a second wave starts: 100,000 particles 63 us with 24, 53 with
+// 32; 66,000 54 with 16, 40 with 24).  In fast math 8 to 28 up to 20 to 28 warps per SM (32 fit; us
+// with w - 4 and w at the lines: 23,000 particles 22.0 with 8 and 22.8 with 12, 29,000 24.2 / 23.1,
+// 33,000 26.2 / 24.8; 40,000 27.0 with 12 and 26.7 with 16; 50,000 29.3 / 29.2 and 60,000 31.6 / 30.9
+// with 16 and 20; 78,000 35.3 / 35.0 with 20 and 24; 100,000 38.8 / 38.6 with 24 and 28 and 40.4 with
+// 32; 122,000 44.8 / 43.7 with 28 and 32).  Fewer than 8 up to 12 warps per SM: with 1, 2, 4 and 8
+// particles per warp 1,000 take 13.9 / 14.2 / 14.6 / 16.3 us, 4,000 - / 16.0 / 15.9 / 16.4, 9,000 (4, 6
+// and 8) 17.8 / 17.5 / 18.1, 16,000 22.3 / 20.2 / 20.2.
 //
 // FEW (exact math, at most 8 particles per warp): four lanes turn a particle's masks into its list,
 // which then lies in the pool, and evaluate its terms as the pair kernels do with four lanes.  Exact
@@ -87,9 +90,10 @@ constexpr int kFewPerWarp = 8;
 inline int search_per_warp(int n, int sms, bool exact) {
     const int most = 12 * sms;  // warps
     if (n <= kFewPerWarp * most) return (n + most - 1) / most;
-    const int warps = (exact ? 24 : 32) * sms;
-    for (int w = 8; w < 32; w += 8)
-        if (n <= w * warps) return w;
+    for (int w = 8; w < 32; w += exact ? 8 : 4) {
+        const int per_sm = exact ? 24 : w < 24 ? 16 + w / 2 : 28;
+        if (n <= w * per_sm * sms) return w;
+    }
     return 32;
 }
 constexpr int kPairWords = 3 * 32;  // a run's positions, two particles interleaved

@@ -46,6 +46,20 @@ def test_particles_per_warp_edges(where):
     assert_records_bitexact(g, o)
 
 
+@pytest.mark.parametrize("per_warp,warps_per_sm", [(8, 20), (12, 22), (20, 26), (28, 28)])
+def test_particles_per_warp_edges_fast(per_warp, warps_per_sm):
+    """One past the lines of fast math, where a warp takes 12, 16, 24 and 32 particles: the lists
+    are those of the oracle (the first walk's positions do not depend on the math)."""
+    import torch
+
+    n = per_warp * warps_per_sm * torch.cuda.get_device_properties(0).multi_processor_count + 1
+    sc = first_of_block(n, seed=n)
+    cfg, corr = PBFConfig(), LambdaCorrParams()
+    _, ge = run_gpu(sc, cfg, corr, 1, 0)
+    _, oe = run_oracle(sc, cfg, corr, 1)
+    assert_grid_equal(ge, oe, cfg.maxNeighbours)
+
+
 @pytest.mark.parametrize("shape", [(64, 16), (64, 32), (128, 48)])
 @pytest.mark.parametrize("kind", ["wide_cell", "cluster", "small_table"])
 def test_runs_longer_than_the_pool(shape, kind):
