@@ -216,8 +216,8 @@ __global__ void __launch_bounds__(kElemBlock)
              const uint32_t* __restrict__ rank_of_import, const float4* __restrict__ x4,
              const float4* __restrict__ v4, const uint32_t* __restrict__ origin,
              const uint32_t* __restrict__ rref_old, float4* __restrict__ x4g,
-             uint32_t* __restrict__ origing, float4* __restrict__ ps0, uint32_t* __restrict__ r2i, uint32_t* __restrict__ rank_of,
-             uint32_t* __restrict__ order_out,
+             uint32_t* __restrict__ origing, float4* __restrict__ ps0, uint32_t* __restrict__ r2i,
+             uint32_t* __restrict__ rank_of, uint32_t* __restrict__ order_out,
              const float* __restrict__ rho_in, const float* __restrict__ lam_in,
              const float4* __restrict__ dp_in, float* __restrict__ rho_out,
              float* __restrict__ lam_out, float4* __restrict__ dp_out, int carry,

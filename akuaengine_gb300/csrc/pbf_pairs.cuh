@@ -187,8 +187,8 @@ __device__ __forceinline__ void lanes_add(int i, int c, E&& entries, L&& load, T
 // through its particle's list by itself.  With 2, 4 or 8 lanes per particle each lane gathers
 // and evaluates its own pair of every 4, 8 or 16 entries, the next one's records in flight, and the
 // lanes hand their terms round by shuffles, so that every lane adds all of them in list order (the
-// sums are the same bit for bit) and a list takes a half, a quarter or an eighth of the steps.  All lanes of a warp call
-// it (c = 0 for lanes without a particle).
+// sums are the same bit for bit) and a list takes a half, a quarter or an eighth of the steps.  All
+// lanes of a warp call it (c = 0 for lanes without a particle).
 template <int LANES, bool WHOLE_TILE, int N, class L, class T, class A>
 __device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr4, int n, int i, int c,
                                                    L&& load, T&& term, A&& add) {
@@ -219,9 +219,7 @@ __device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr
 // Lanes per particle of the pair kernels.  A scene too small to fill the chip is as slow as the chain
 // of gathers of one list, which more lanes shorten, until the shuffles cost more issue slots than the
 // chain costs time: about 10 warps per SM with 8 lanes (22 with exact math, whose terms are longer)
-// and 18 with 4 or 2 (24, all that fit at 80 registers).  Steps in us with 1 / 2 / 4 lanes: 1,000 particles 95 / 95 / 84, 8,000 121 / 108 /
-// 96, 27,000 139 / 128 / 132 (exact 207 / 181 / 160), 40,000 156 / 151 / 176 (exact 226 / 205 / 216),
-// 60,000 167 / 176 / 208.  With 4 / 8 / 16 lanes, the other kernels being faster by then: 1,000
+// and 18 with 4 or 2 (24, all that fit at 80 registers).  Steps in us with 4 / 8 / 16 lanes: 1,000
 // particles 70 / 66 / 68, 4,000 80 / 77 / 84, 6,000 82.6 / 82.2 / 92, 8,000 85 / 87; exact 1,000
 // 88 / 75 / 72, 4,000 105 / 89 / 92, 12,000 118 / 109, 16,000 124 / 132.  With 1 / 2 / 4: 20,000 116 /
 // 110 / 105, 27,000 120 / 111 / 114, 45,000 134 / 132, 52,000 140 / 144; exact 27,000 183 / 160 / 139,

@@ -63,9 +63,9 @@
 
 namespace akua {
 
-// Default tile shape.  With culls of 32 the walk takes 273 us at 1M particles with 64 or 128 threads and 32 x 32
-// words, 294 with 32 x 48 (fewer warps fit an SM) and 404 with 32 x 16 (a warp's runs no longer
-// fit the pool at once, so the extraction runs several times with few lanes).
+// Default tile shape.  With culls of 32 the walk takes 273 us at 1M particles with 64 or 128 threads
+// and 32 x 32 words, 294 with 32 x 48 (fewer warps fit an SM) and 404 with 32 x 16 (a warp's runs no
+// longer fit the pool at once, so the extraction runs several times with few lanes).
 constexpr int kSearchBlock = 128;
 constexpr int kListStage = 32;
 

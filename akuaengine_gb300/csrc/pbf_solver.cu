@@ -472,8 +472,8 @@ void enqueue_body(akua_pbf* s, cudaStream_t st, const char* aos, size_t stride, 
     }
     if (aos) {
         step_kernel(s, st, akua::k_export, grid_for(n, akua::kIoBlock), akua::kIoBlock, 0,
-                    s->d_params, const_cast<char*>(aos), stride, n, s->r2i, s->kr, s->x4, s->v4, s->vstar4, s->dp4,
-                    s->om4, s->rho, s->lam, s->col4, s->size, s->origin, s->lacc,
+                    s->d_params, const_cast<char*>(aos), stride, n, s->r2i, s->kr, s->x4, s->v4,
+                    s->vstar4, s->dp4, s->om4, s->rho, s->lam, s->col4, s->size, s->origin, s->lacc,
                     learn_mode(s) ? s->lacc_ref : nullptr);
         mark("k_export");
     }

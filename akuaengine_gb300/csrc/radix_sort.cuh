@@ -8,9 +8,9 @@
 //
 // A sort of `bits`-bit keys runs ceil(bits / 10) passes of equal digit width (8..10 bits).  Each
 // pass: per-tile digit counts, a scan of the (tile, digit) count matrix over the tiles (for inputs of
-// few tiles in the scatter itself), and a stable scatter in
-// which warps rank their keys by ballots and per-warp running digit counters, order the tile in
-// shared memory and store it in runs.  Inputs of at most kClusterMax pairs take one launch per pass.
+// few tiles in the scatter itself), and a stable scatter in which warps rank their keys by ballots and
+// per-warp running digit counters, order the tile in shared memory and store it in runs.  Inputs of
+// at most kClusterMax pairs take one launch per pass.
 #pragma once
 
 #include <cstdint>
@@ -342,7 +342,8 @@ __global__ void __launch_bounds__(BLOCK, FUSED ? 1 : 3)
 }
 
 // One pass over the digit (key >> shift) & digit_mask; digit_mask defaults to all BITS bits.
-// `after`: the stream's previous kernel is this sort's previous pass.  `fused`: no scan launch, for inputs of few tiles (the scatters then read tiles x tiles rows).
+// `after`: the stream's previous kernel is this sort's previous pass.  `fused`: no scan launch, for
+// inputs of few tiles (the scatters then read tiles x tiles rows).
 template <int BITS, class Mark>
 inline void run_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                      uint32_t* vout, uint32_t* counts, uint32_t* totals, int n, int shift,
@@ -355,13 +356,14 @@ inline void run_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, u
     launch(after, upsweep<BITS>, tiles, BLOCK, 0, s, 1, kin, n, shift, digit_mask, counts);
     mark("radix_upsweep");
     if (!fused) {
-        launch(true, scan_tiles<BITS>, RADIX / SCAN_DIGITS, 32 * SCAN_WARPS, 0, s, 1, counts, totals, tiles);
+        launch(true, scan_tiles<BITS>, RADIX / SCAN_DIGITS, 32 * SCAN_WARPS, 0, s, 1, counts, totals,
+               tiles);
         mark("radix_scan");
-        launch(true, downsweep<BITS, false>, tiles, BLOCK, smem, s, 1, kin, vin, kout, vout, n, shift, digit_mask,
-                                                          counts, totals, tiles, rank_out);
+        launch(true, downsweep<BITS, false>, tiles, BLOCK, smem, s, 1, kin, vin, kout, vout, n, shift,
+               digit_mask, counts, totals, tiles, rank_out);
     } else {
-        launch(true, downsweep<BITS, true>, tiles, BLOCK, smem, s, 1, kin, vin, kout, vout, n, shift, digit_mask,
-                                                         counts, nullptr, tiles, rank_out);
+        launch(true, downsweep<BITS, true>, tiles, BLOCK, smem, s, 1, kin, vin, kout, vout, n, shift,
+               digit_mask, counts, nullptr, tiles, rank_out);
     }
     mark("radix_downsweep");
 }
@@ -644,9 +646,10 @@ inline size_t scratch_words(int n) {
 }
 
 // Sorts (k0, v0) by the low plan bits, ping-ponging with (k1, v1); all four buffers hold n words (a
-// cluster plan: takes_cluster(n)).  With `index_payload` the input payload is each key's index and v0 is not read.  The result
-// buffers are returned through keys_out / vals_out.  With `rank_out` (n words), the last pass
-// also writes rank_out[payload] = output position.  `mark(name)` is called after every kernel.
+// cluster plan: takes_cluster(n)).  With `index_payload` the input payload is each key's index and v0
+// is not read.  The result buffers are returned through keys_out / vals_out.  With `rank_out` (n
+// words), the last pass also writes rank_out[payload] = output position.  `mark(name)` is called after
+// every kernel.
 template <class Mark>
 inline void sort_pairs(cudaStream_t s, const Plan& plan, uint32_t* k0, uint32_t* v0, uint32_t* k1,
                        uint32_t* v1, bool index_payload, uint32_t* scratch, int n,
