@@ -28,6 +28,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "dependent_launch.cuh"
 #include "tc05.cuh"
 
 namespace akua::mlp {
@@ -183,8 +184,8 @@ __device__ __forceinline__ float output_layer(uint32_t taddr, const float* b3, c
 __device__ __forceinline__ void load_features(const float* __restrict__ feat, int i, int n,
                                               const float* norm, float (&f)[kIn]) {
     if (i < n) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(feat) + 2 * (size_t)i);
-        const float4 b = __ldg(reinterpret_cast<const float4*>(feat) + 2 * (size_t)i + 1);
+        const float4 a = reinterpret_cast<const float4*>(feat)[2 * (size_t)i];
+        const float4 b = reinterpret_cast<const float4*>(feat)[2 * (size_t)i + 1];
         f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
         f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
     } else {
@@ -219,11 +220,11 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
     // columns 8..15 of the input tile stay zero
     *reinterpret_cast<uint4*>(x + tc::kmajor_offset(t, 8, kInPad)) = make_uint4(0, 0, 0, 0);
     if (threadIdx.x < 32) tc::tmem_alloc(&S.tmem, kFwdGroups * kHid);
-    tc::wait_for_previous();
+    pdl::wait_for_previous(params, image, norm, feat);
     {
         const uint4* src = reinterpret_cast<const uint4*>(image);
         uint4* dst = reinterpret_cast<uint4*>(S.w1);
-        for (int k = threadIdx.x; k < kImageBytes / 16; k += kFwdThreads) dst[k] = __ldg(src + k);
+        for (int k = threadIdx.x; k < kImageBytes / 16; k += kFwdThreads) dst[k] = src[k];
     }
     if (threadIdx.x < kHid) {
         S.b1[t] = params[kB1 + t];
@@ -389,9 +390,9 @@ __global__ void __launch_bounds__(kGradThreads, 1)
         }
     }
     if (warp == 0) tc::tmem_alloc(&S.tmem, kGradTmem);
-    tc::wait_for_previous();
+    pdl::wait_for_previous(params, image, norm, feat, target);
     for (int k = t; k < kImageBytes / 16; k += kGradThreads)
-        reinterpret_cast<uint4*>(S.w1)[k] = __ldg(reinterpret_cast<const uint4*>(image) + k);
+        reinterpret_cast<uint4*>(S.w1)[k] = reinterpret_cast<const uint4*>(image)[k];
     if (t < kHid) {
         S.b1[t] = params[kB1 + t];
         S.b2[t] = params[kB2 + t];
@@ -644,7 +645,7 @@ __global__ void k_mlp_adam(float* __restrict__ params, float* __restrict__ grad,
                            uint8_t* __restrict__ image, float lr, float beta1, float beta2,
                            float eps, float bc1, float bc2) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    tc::wait_for_previous();
+    pdl::wait_for_previous(params, grad, m, v);
     if (k > kParams) return;
     if (k == kParams) {
         grad[k] = 0.f;

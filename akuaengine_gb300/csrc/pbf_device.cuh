@@ -11,6 +11,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "dependent_launch.cuh"
+
 namespace akua {
 
 // Everything a kernel of one step reads besides the particle arrays.  Lives in device memory and is
@@ -75,12 +77,6 @@ struct StepParams {
     float sdf_min_dist;
     float sdf_stiffness;
 };
-
-// Programmatic dependent launch: the step's kernels are set up while the one before them ends, and
-// wait here for its stores.
-__device__ __forceinline__ void after_previous_kernel() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 
 // The parameters of the scene particle (or reference rank, or internal slot) i belongs to.
 __device__ __forceinline__ const StepParams& params_for(const StepParams* P, int i) {

@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kElemBlock)
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = P->n;
     const int lane = threadIdx.x & 31;
-    after_previous_kernel();
+    pdl::wait_for_previous(kr, r2i);
     if (r - lane >= n) return;  // uniform over the warp
     uint32_t key[2], slot[2], before = 0;
 #pragma unroll
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kIoBlock)
     const int r0 = blockIdx.x * kIoBlock;
     const int cnt = min(kIoBlock, n - r0);
     const int t = threadIdx.x;
-    after_previous_kernel();
+    pdl::wait_for_previous(v4);
     if (t < cnt) {
         const int r = r0 + t;
         const uint32_t s = r2i[r];

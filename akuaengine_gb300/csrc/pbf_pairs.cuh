@@ -96,9 +96,9 @@ __device__ __forceinline__ void spiky2(const StepParams& p, float2 sx, float2 sy
 // 98).
 __device__ __forceinline__ uint4 ld_tile(const uint4* p) {
     uint4 t;
-    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-        : "=r"(t.x), "=r"(t.y), "=r"(t.z), "=r"(t.w)
-        : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(t.x), "=r"(t.y), "=r"(t.z), "=r"(t.w)
+                 : "l"(p));
     return t;
 }
 
@@ -210,7 +210,7 @@ __device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr
             i, c,
             [&](int e) {
                 const uint2* at = reinterpret_cast<const uint2*>(nbr4 + (size_t)(e >> 2) * n + i);
-                return __ldg(at + ((e >> 1) & 1));
+                return at[(e >> 1) & 1];
             },
             load, term, add);
     }
@@ -248,10 +248,10 @@ struct Rec8 {
 };
 __device__ __forceinline__ Rec8 ld_rec8(const float4* __restrict__ rec, uint32_t j) {
     Rec8 r;
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(r.x.x), "=f"(r.x.y), "=f"(r.x.z), "=f"(r.x.w), "=f"(r.v.x), "=f"(r.v.y),
-          "=f"(r.v.z), "=f"(r.v.w)
-        : "l"(rec + 2 * (size_t)j));
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(r.x.x), "=f"(r.x.y), "=f"(r.x.z), "=f"(r.x.w), "=f"(r.v.x), "=f"(r.v.y),
+                   "=f"(r.v.z), "=f"(r.v.w)
+                 : "l"(rec + 2 * (size_t)j));
     return r;
 }
 
@@ -327,12 +327,12 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    after_previous_kernel();
+    pdl::wait_for_previous(ps);
     const float4 xi = ps[i];
     DensityLambda2<EXACT> acc;
     acc.init(xi.w, p);
     for_each_neighbour<LANES, true, 6>(
-        nbr4, n, i, live ? (int)cnt[i] : 0, [&](uint32_t j) { return __ldg(ps + j); },
+        nbr4, n, i, live ? (int)cnt[i] : 0, [&](uint32_t j) { return ps[j]; },
         [&](float4 a, float4 b) { return DensityLambda2<EXACT>::terms(p, xi, a, b); }, acc);
     if (!writes<LANES>(live)) return;
     rho_out[i] = acc.rho;
@@ -374,7 +374,7 @@ __device__ __forceinline__ float3 position_delta(const StepParams& p, float4 xi,
                                                  const float* __restrict__ lam,
                                                  const uint4* __restrict__ nbr4, int i, int c) {
     Sum3 d;
-    auto load = [&](uint32_t j) { return Rec5{__ldg(ps + j), __ldg(lam + j)}; };
+    auto load = [&](uint32_t j) { return Rec5{ps[j], lam[j]}; };
     auto term = [&](const Rec5& ra, const Rec5& rb) {
         const float4 a = ra.x, b = rb.x;
         const float2 lj = make_float2(ra.l, rb.l);
@@ -406,7 +406,7 @@ __device__ __forceinline__ float3 position_delta_uniform(const StepParams& p,
                                                          int c) {
     const float4 xl = psl[i];
     Sum3 d;
-    auto load = [&](uint32_t j) { return __ldg(psl + j); };
+    auto load = [&](uint32_t j) { return psl[j]; };
     auto term = [&](float4 a, float4 b) {
         const float2 sx = diff2(xl.x, a.x, b.x);
         const float2 sy = diff2(xl.y, a.y, b.y);
@@ -431,8 +431,8 @@ __device__ __forceinline__ float3 delta_of(const StepParams& p, int i, float4 xi
                                            const float4* __restrict__ psl,
                                            const uint32_t* __restrict__ mass_bits,
                                            const uint4* __restrict__ nbr4, int c) {
-    if (__ldg(mass_bits) == 0u) {
-        const float m = __uint_as_float(__ldg(mass_bits + 1));
+    if (mass_bits[0] == 0u) {
+        const float m = __uint_as_float(mass_bits[1]);
         return p.corr_n_int == 4
                    ? position_delta_uniform<EXACT, true, LANES>(p, psl, m, nbr4, i, c)
                    : position_delta_uniform<EXACT, false, LANES>(p, psl, m, nbr4, i, c);
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(P->n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    after_previous_kernel();
+    pdl::wait_for_previous(lam, psl, nbr4, cnt);
     const float4 xi = ps_in[i];
     const float3 d = delta_of<EXACT, LANES>(p, i, xi, ps_in, lam, psl, mass_bits, nbr4,
                                             live ? (int)cnt[i] : 0);
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(P->n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    after_previous_kernel();
+    pdl::wait_for_previous(lam, psl, nbr4, cnt);
     const float4 xi = ps_in[i];
     float nx = xi.x, ny = xi.y, nz = xi.z;
     float3 d = make_float3(0.f, 0.f, 0.f);
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    after_previous_kernel();
+    pdl::wait_for_previous(x4, v4, xv8);
     const float4 xi = x4[i], vi = v4[i];
     Sum3 w;
     auto load = [&](uint32_t j) { return ld_rec8(xv8, j); };
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(kMaxPairBlock, LANES == 1 ? 5 : 1)
     const bool live = particle_of_thread<LANES>(n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    after_previous_kernel();
+    pdl::wait_for_previous(om4, xw4);
     const float4 xi = x4[i], vi = v4[i], wi = om4[i];
     const float rho_i = rho[i];
     const int c = live ? (int)cnt[i] : 0;
@@ -649,13 +649,13 @@ __global__ void __launch_bounds__(kMaxPairBlock, LANES == 1 ? 5 : 1)
         t.v[0] = mul2(mj, sub2(f2(wi.w), wj));
         return t;
     };
-    if (__ldg(mass_bits) == 0u) {  // one mass: (x, |omega|) in one gather, the same products
-        const float m = __uint_as_float(__ldg(mass_bits + 1));
-        auto load = [&](uint32_t j) { return __ldg(xw4 + j); };
+    if (mass_bits[0] == 0u) {  // one mass: (x, |omega|) in one gather, the same products
+        const float m = __uint_as_float(mass_bits[1]);
+        auto load = [&](uint32_t j) { return xw4[j]; };
         auto term = [&](float4 a, float4 b) { return pair(a, b, f2(m), make_float2(a.w, b.w)); };
         for_each_neighbour<LANES, false, 4>(nbr4, n, i, c, load, term, eta);
     } else {
-        auto load = [&](uint32_t j) { return Rec5{__ldg(x4 + j), __ldg(&om4[j].w)}; };
+        auto load = [&](uint32_t j) { return Rec5{x4[j], om4[j].w}; };
         auto term = [&](const Rec5& a, const Rec5& b) {
             return pair(a.x, b.x, make_float2(a.x.w, b.x.w), make_float2(a.l, b.l));
         };
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(kMaxPairBlock)
     const bool live = particle_of_thread<LANES>(n, i);
     if (LANES == 1 && !live) return;
     const StepParams& p = params_for(P, i);
-    after_previous_kernel();
+    pdl::wait_for_previous(xv8);
     if (writes<LANES>(live)) {
         // the walk is done: empty this step's bucket entries (particle i: the bucket starting at
         // rank i)

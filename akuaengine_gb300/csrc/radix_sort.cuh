@@ -16,6 +16,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "dependent_launch.cuh"
+
 namespace akua {
 namespace radix {
 
@@ -81,13 +83,10 @@ __device__ __forceinline__ uint32_t same_digit(uint32_t digit, bool live) {
     return peers;
 }
 
-// Programmatic dependent launch: a kernel launched with `after` is set up while the stream's previous
-// kernel ends, and waits here for its stores.  No kernel lets the next one start before its own
-// blocks are done: blocks that wait take the room of blocks that work (2^20 pairs launched one by
-// one: 68 us without, 58 with an early start, 47 like this; replayed from a graph 48, 55, 46).
-__device__ __forceinline__ void wait_for_previous() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// A kernel launched with `after` is set up while the stream's previous kernel ends, and waits for its
+// stores (dependent_launch.cuh).  No kernel lets the next one start before its own blocks are done:
+// blocks that wait take the room of blocks that work (2^20 pairs launched one by one: 68 us without,
+// 58 with an early start, 47 like this; replayed from a graph 48, 55, 46).
 template <class... Params, class... Args>
 inline cudaError_t launch(bool after, void (*kernel)(Params...), int grid, int block, size_t smem,
                           cudaStream_t st, int cluster, Args... args) {
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(BLOCK) upsweep(const uint32_t* __restrict__ ke
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int t = threadIdx.x; t < WARPS * RADIX; t += BLOCK) (&hist[0][0])[t] = 0;
     __syncthreads();
-    wait_for_previous();
+    pdl::wait_for_previous(keys);
     const int base = blockIdx.x * TILE + warp * WARP_ITEMS + lane;
     uint32_t key[ROUNDS];  // all loads in flight at once: 14.4 -> 8.8 us at 1M, launch included
 #pragma unroll
@@ -158,8 +157,8 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS)
     const int digit = lane % SCAN_DIGITS, part = lane / SCAN_DIGITS;
     const int per = (tiles + SCAN_WARPS * PARTS - 1) / (SCAN_WARPS * PARTS);
     const int t0 = min((warp * PARTS + part) * per, tiles), t1 = min(t0 + per, tiles);
+    pdl::wait_for_previous(counts);
     uint32_t* col = counts + blockIdx.x * SCAN_DIGITS + digit;
-    wait_for_previous();
     uint32_t sum = 0;
 #pragma unroll 8
     for (int t = t0; t < t1; ++t) sum += col[(size_t)t * RADIX];
@@ -245,7 +244,7 @@ __global__ void __launch_bounds__(BLOCK, FUSED ? 1 : 3)
     for (int t = threadIdx.x; t < WARPS * RADIX; t += BLOCK) (&count[0][0])[t] = 0;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const int tile0 = blockIdx.x * TILE;
-    wait_for_previous();
+    pdl::wait_for_previous(counts, totals);
     const int base = tile0 + warp * WARP_ITEMS + lane;
     uint32_t key[ROUNDS], val[ROUNDS], pos[ROUNDS];
 #pragma unroll
@@ -482,7 +481,7 @@ __global__ void __launch_bounds__(kClusterThreads)
 #pragma unroll
     for (int k = 0; k < kClusterWarps * RADIX / 8 / kClusterThreads; ++k)
         zero[k * kClusterThreads + t] = make_uint4(0u, 0u, 0u, 0u);
-    wait_for_previous();
+    pdl::wait_for_previous(keys_in, vals_in);
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
         const int at = first + 32 * r;

@@ -27,6 +27,7 @@
 #include <new>
 
 #include "akua_pbf.h"
+#include "dependent_launch.cuh"
 
 namespace {
 
@@ -112,13 +113,10 @@ struct Queue {
     unsigned long long part[kQueue];  // particle | part << 32
 };
 
-// Programmatic dependent launch: the next kernel of the stream may start once every block has got
-// here, and waits for this one's completion itself.
+// The next kernel of the stream may start once every block has got here, and waits for this one's
+// completion itself (dependent_launch.cuh).
 __device__ __forceinline__ void let_next_start() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void wait_for_previous() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Draws the pixels first, first + step, ... of a sprite.
@@ -202,7 +200,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_splat_large(SplatParams P, const char* __restrict__ aos, uint64_t stride,
                   unsigned long long* __restrict__ zbuf, const Queue* __restrict__ queue) {
-    wait_for_previous();
+    akua::pdl::wait_for_previous(aos, zbuf, queue);
     let_next_start();
     const uint32_t count = min(__ldcg(&queue->count), kQueue), warps = gridDim.x * (blockDim.x / 32);
     const int lane = threadIdx.x & 31;
@@ -225,7 +223,7 @@ __global__ void __launch_bounds__(256)
     k_splat_resolve(SplatParams P, const char* __restrict__ aos, uint64_t stride,
                     unsigned long long* __restrict__ zbuf, Queue* __restrict__ queue,
                     uint32_t* __restrict__ rgba) {
-    wait_for_previous();
+    akua::pdl::wait_for_previous(aos, zbuf, queue);
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p == 0) queue->count = 0u;  // for the next frame
     if (p >= P.width * P.height) return;

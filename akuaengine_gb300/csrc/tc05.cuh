@@ -98,13 +98,6 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
         : "memory");
 }
 
-// --- programmatic dependent launch ---------------------------------------------------------------
-// Waits for the stores of the stream's previous kernel (a kernel launched with the attribute may be set
-// up while that one ends; without it this does nothing).
-__device__ __forceinline__ void wait_for_previous() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // --- reductions to global memory ------------------------------------------------------------------
 // p[0..3] += v, one 16-byte reduction (p 16-byte aligned).
 __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
