@@ -307,10 +307,13 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
             const int m = q1 - q0;
             const uint2 e = e_next;
             const uint32_t blen = e.y & ~kMixedBucket;
-            // A lone particle's only candidate is itself.  Warps of spray have a run per particle and
-            // end last, so a run that needs nothing more than its lookup counts (300,000 particles
-            // between obstacles: walk 101 -> 96 us).
-            if (m == 1 && __reduce_add_sync(kFullWarp, blen) == 1u) {
+            // A lone particle whose only candidate is itself has an empty list.  (A bucket of one is
+            // never mixed: e.x is its slot.  With a walk cell that is not the smoothing radius the only
+            // candidate may be another particle, which then counts as two.)  Warps of spray have a run
+            // per particle and end last, so a run that needs nothing more than its lookup counts
+            // (300,000 particles between obstacles: walk 101 -> 96 us).
+            const uint32_t others = blen == 1u && e.x != (uint32_t)(base + q0) ? 2u : blen;
+            if (m == 1 && __reduce_add_sync(kFullWarp, others) == 1u) {
                 if (lane == q0) {
                     my_seq = used;
                     my_q0 = q0;

@@ -145,3 +145,36 @@ def test_sparse_runs(table_size):
     g, ge = run_gpu(sc, cfg, corr, 1, ak.OPT_EXACT_MATH, table_size=table_size)
     assert_grid_equal(ge, oe, cfg.maxNeighbours)
     assert_records_bitexact(g, o)
+
+
+def pairs_out_of_sight(cell):
+    """Lone particles within each other's reach, at rest.  A walk over cells of another size than the
+    smoothing radius looks up buckets that need not hold the particle itself, so a single candidate
+    may be its neighbour."""
+    if cell in (0.2, 0.25):
+        pos = np.array({0.2: [(0.41, 0.42, 0.41), (0.39, 0.39, 0.39)],
+                        0.25: [(0.31, 0.05, 0.05), (0.24, 0.05, 0.05)]}[cell])
+    else:
+        rng = np.random.default_rng(12)
+        axis = np.arange(6) * 0.35 + 0.1
+        at = np.stack(np.meshgrid(axis, axis, axis, indexing="ij"), -1).reshape(-1, 3)
+        at = at + rng.uniform(-0.05, 0.05, at.shape)
+        d = rng.normal(size=at.shape)
+        d *= rng.uniform(0.05, 0.095, (len(at), 1)) / np.linalg.norm(d, axis=1, keepdims=True)
+        pos = np.concatenate([at, at + d])
+    p = scene.lattice_block((len(pos), 1, 1), 0.0, (0.0, 0.0, 0.0))
+    p["position"] = pos.astype(np.float32)
+    return scene.Scene(p, (-1.0, -1.0, -1.0), (3.0, 3.0, 3.0), 0.0083, "pairs")
+
+
+@pytest.mark.parametrize("exact", [True, False], ids=["exact", "fast"])
+@pytest.mark.parametrize("cell", [0.09, 0.11, 0.13, 0.2, 0.25])
+def test_lone_particles_under_another_walk_cell(cell, exact):
+    sc = pairs_out_of_sight(cell)
+    cfg, corr = PBFConfig(spatialHashCellSize=cell, gravity=(0.0, 0.0, 0.0)), LambdaCorrParams()
+    o, oe = run_oracle(sc, cfg, corr, 1, table_size=1 << 20)
+    assert oe["cnt"].any()  # the lists the oracle finds
+    g, ge = run_gpu(sc, cfg, corr, 1, ak.OPT_EXACT_MATH if exact else 0, table_size=1 << 20)
+    assert_grid_equal(ge, oe, cfg.maxNeighbours)
+    if exact:
+        assert_records_bitexact(g, o)
