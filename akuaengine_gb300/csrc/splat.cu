@@ -312,6 +312,7 @@ struct akua_splat {
     int width = 0, height = 0;
     unsigned long long* zbuf = nullptr;  // empty between frames
     Queue* queue = nullptr;
+    bool dirty = false;  // a frame was not launched whole: they may not be
 };
 
 extern "C" {
@@ -416,6 +417,11 @@ int akua_splat_render(akua_splat* r, const void* particles, size_t stride, int32
     for (int k = 0; k < 3; ++k) P.eye[k] = camera->position[k];
     cudaStream_t st = (cudaStream_t)stream;
     const size_t pixels = (size_t)r->width * r->height;
+    if (r->dirty) {  // the last frame failed between its first and its last launch
+        cudaError_t e = cudaMemsetAsync(r->zbuf, 0xFF, sizeof(unsigned long long) * pixels, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(&r->queue->count, 0, sizeof(uint32_t), st);
+        if (e != cudaSuccess) return status_of(e);
+    }
     const char* aos = static_cast<const char*>(particles);
     if (n > 0) {
         const int per_warp = splat_per_warp(n, r->sms), per_block = 8 * per_warp;
@@ -426,7 +432,15 @@ int akua_splat_render(akua_splat* r, const void* particles, size_t stride, int32
     }
     launch_after(k_splat_resolve, (unsigned)((pixels + 255) / 256), st, P, aos, (uint64_t)stride,
                  r->zbuf, r->queue, rgba);
-    return status_of(cudaGetLastError());
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        r->dirty = true;
+    } else if (r->dirty) {  // cleared now, unless the stream is being captured and nothing has run
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+        if (cudaStreamIsCapturing(st, &capture) == cudaSuccess)
+            r->dirty = capture != cudaStreamCaptureStatusNone;
+    }
+    return status_of(e);
 }
 
 }  // extern "C"

@@ -323,7 +323,9 @@ typedef struct akua_splat akua_splat;
 int akua_splat_create(int32_t width, int32_t height, akua_splat** out);
 int akua_splat_destroy(akua_splat* renderer);
 /* Renders n particle records (device memory, strideBytes apart) into deviceRGBA (width * height
- * pixels, R in the low byte, row 0 at the top); asynchronous on cudaStream. */
+ * pixels, R in the low byte, row 0 at the top); asynchronous on cudaStream.  A renderer's frames use
+ * its one depth buffer one after another: frames on several streams, or from several threads, must
+ * be ordered by the caller. */
 int akua_splat_render(akua_splat* renderer, const void* deviceParticles, size_t strideBytes,
                       int32_t n, const akua_camera* camera, uint32_t* deviceRGBA,
                       void* cudaStream);
