@@ -31,9 +31,9 @@ def nvcc_path() -> str:
 
 
 def sources() -> list[str]:
-    return [os.path.join(CSRC, "pbf_solver.cu"), os.path.join(CSRC, "sort_noalloc.cu"),
-            os.path.join(CSRC, "mlp.cu"), os.path.join(CSRC, "state_io.cpp"),
-            os.path.join(CSRC, "splat.cu")]
+    return [os.path.join(CSRC, f) for f in (
+        "pbf_solver.cu", "pbf_fast.cu", "pbf_exact.cu", "pbf_shapes.cu", "sort_noalloc.cu", "mlp.cu",
+        "state_io.cpp", "splat.cu")]
 
 
 def headers() -> list[str]:
@@ -52,8 +52,8 @@ def _stale(target: str, deps: list[str]) -> bool:
 
 
 def nvcc_command(output: str, extra: list[str] | None = None) -> list[str]:
-    # -no-compress: nvcc packs large device images, and unpacking the solver's took 7.5 ms of a
-    # process's first step (10.2 ms from creation to the first step's end, 2.8 with it)
+    # -no-compress: nvcc packs large device images, and unpacking the solver's, when it was one image,
+    # took 7 ms of a process's first step (10.2 ms from creation to the first step's end, 3.1 with it)
     return [
         nvcc_path(), *ARCH_FLAGS, "-no-compress", "-O3", "-lineinfo", "-std=c++17", "--fmad=false",
         "-Xcompiler", "-fPIC,-ffp-contract=off,-O3", "-shared",

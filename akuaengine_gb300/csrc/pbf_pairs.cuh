@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(kMaxPairBlock, LANES == 1 ? 5 : 1)
 
 // XSPH viscosity (IntegrationCUDA.cu:167-195) from the confined-velocity snapshot in the records
 // (x, m / rho | v).  Also leaves the bucket table all-empty for the next step.
-template <int LANES>
+template <bool EXACT, int LANES>  // the same in both modes
 __global__ void __launch_bounds__(kMaxPairBlock)
     k_xsph(const StepParams* __restrict__ P, const float4* __restrict__ xv8,
            const uint4* __restrict__ nbr4, const uint32_t* __restrict__ cnt,

@@ -22,117 +22,14 @@
 #include <vector>
 
 #include "akua_pbf.h"
-#include "mlp_handle.h"
+#include "pbf_handle.cuh"
 #include "pbf_kernels.cuh"
-#include "pbf_learned.cuh"
-#include "radix_sort.cuh"
 
+using akua::grid_for;
+using akua::learn_mode;
+using akua::Marker;
+using akua::step_kernel;
 using akua::StepParams;
-
-struct akua_pbf {
-    int device = 0;
-    int sms = 1;  // multiprocessors of the device
-    bool cluster_sort = false;  // a sort pass is one cluster
-    int n = 0;
-    akua_pbf_config cfg{};
-    akua_lambda_corr_params corr{};
-    uint32_t table_size = 0;
-    uint32_t table_alloc = 0;
-    float restitution = 0.0f;
-    float friction = 0.95f;
-    uint32_t options = 0;
-    cudaStream_t stream = nullptr;          // caller's stream (nullptr = legacy default stream)
-    cudaStream_t capture_stream = nullptr;  // private stream used only for graph capture
-    char* attached = nullptr;
-    size_t stride = 0;
-    bool state_valid = false;  // device state holds the particles (resident mode)
-    bool stepped = false;      // the reference-order tables describe the current state
-
-    StepParams* d_params = nullptr;
-    // state, internal order
-    float4 *x4 = nullptr, *v4 = nullptr, *col4 = nullptr;
-    float* size = nullptr;
-    uint32_t* rref = nullptr;
-    float *rho = nullptr, *lam = nullptr;
-    float4* dp4 = nullptr;
-    // gathered copies and per-step arrays
-    float4 *x4g = nullptr, *ps0 = nullptr, *ps1 = nullptr;
-    uint32_t *origin = nullptr, *origing = nullptr;  // a slot's colour and size: their import index
-    float4 *vstar4 = nullptr, *om4 = nullptr, *xv8 = nullptr, *dpg = nullptr;
-    float *rhog = nullptr, *lamg = nullptr;
-    uint32_t *rrefg = nullptr, *rank_of_import = nullptr, *r2i = nullptr, *order = nullptr;
-    // sorts: reference order (A) and Morton order (B)
-    uint32_t *ka0 = nullptr, *va0 = nullptr, *ka1 = nullptr, *va1 = nullptr;
-    uint32_t *kb0 = nullptr, *vb0 = nullptr, *kb1 = nullptr, *vb1 = nullptr;
-    uint32_t* sort_scratch = nullptr;
-    uint32_t* sort_scratch_b = nullptr;  // the Morton sort's, which runs beside the hash sort
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    uint2* table = nullptr;
-    uint32_t *nbr = nullptr, *cnt = nullptr, *flags = nullptr;
-    float4* psl = nullptr;          // (x*, lambda) of the current iteration, for uniform masses
-    akua::SdfShape* shapes = nullptr;  // SDF obstacles (device), AKUA_SDF_MAX_SHAPES
-    int num_shapes = 0;
-    float sdf_min_dist = 0.025f, sdf_stiffness = 0.5f;
-    uint32_t* mass_bits = nullptr;  // {another mass seen, record 0's mass bits} of this step
-    char* staging = nullptr;
-    size_t staging_bytes = 0;
-
-    akua::radix::Plan plan_ref, plan_sp;
-    int sp_bits = 0;
-    uint32_t *kr = nullptr, *refperm = nullptr, *spperm = nullptr;  // sort results (set at enqueue)
-
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    bool graph_ok = false;
-    uint32_t graph_options = 0;
-    const char* graph_aos = nullptr;
-    size_t graph_stride = 0;
-    int graph_sp_bits = -1;
-    int graph_captures = 0;
-    int body_launches = 0;
-    bool chain = false;  // the body's kernels are set up while the previous one ends
-
-    // learned warm start (allocated on first use): features, predicted velocity (.w = density),
-    // the step's accumulated lambda, the previous step's (internal order) and the export copy
-    // (reference order, read back at import)
-    akua_mlp* warm = nullptr;
-    bool track = false;  // accumulate lambda and compute features every step
-    float* cap_feat = nullptr;
-    float* cap_target = nullptr;
-    float *feat = nullptr, *lacc = nullptr, *lprev = nullptr, *lacc_ref = nullptr;
-    float* speed = nullptr;
-    uint32_t* err_max = nullptr;
-    double* err_sum = nullptr;
-    int graph_learn = 0;
-
-    // batches of independent scenes (akua_pbf_create_batch); empty for a single scene
-    std::vector<akua_scene_desc> scenes;
-    std::vector<uint32_t> scene_first;  // first particle of each scene
-    uint16_t* scene_of = nullptr;       // device: the scene of every particle
-    int scene_bits = 0;                 // bits of the scene index in the Morton sort key
-
-    // block sizes of the neighbour-pair kernels (akua_pbf_set_pair_blocks / akua_pbf_autotune)
-    int pair_block[AKUA_PBF_PAIR_KERNELS] = {128, 128, 128, 128, 128, 128};
-    // the walk's tile shape (akua_pbf_set_search_shape / akua_pbf_autotune)
-    int search_block = akua::kSearchBlock;
-    int search_stage = akua::kListStage;
-
-    int64_t steps = 0;
-    uint64_t device_bytes = 0;
-
-    // profiling (akua_pbf_profile_begin/end): one event after every kernel of a step
-    bool prof_active = false;
-    int prof_steps_left = 0;
-    std::vector<cudaEvent_t> prof_events;
-    std::vector<const char*> prof_names;  // nullptr marks the start of a step
-    size_t prof_next = 0;
-};
-
-namespace akua::mlp {
-int enqueue_forward(const akua_mlp* m, const float* feat, int n, float* out, float* out2,
-                    float* out4, cudaStream_t st);
-}
 
 namespace {
 
@@ -282,12 +179,6 @@ std::vector<StepParams> make_batch_params(const akua_pbf* s, float dt) {
     return out;
 }
 
-inline int grid_for(int n, int block) { return (n + block - 1) / block; }
-
-// 0: plain step; 1: features and accumulated lambda are tracked (training capture); 2: and the
-// network's prediction replaces iteration 1's lambda.
-int learn_mode(const akua_pbf* s) { return s->warm ? 2 : ((s->track || s->cap_feat) ? 1 : 0); }
-
 cudaError_t ensure_learn_buffers(akua_pbf* s) {
     if (s->feat) return cudaSuccess;
     const int n = s->n;
@@ -301,117 +192,6 @@ cudaError_t ensure_learn_buffers(akua_pbf* s) {
     if (e == cudaSuccess) e = cudaMemset(s->lacc, 0, sizeof(float) * n);
     if (e == cudaSuccess) e = cudaMemset(s->lacc_ref, 0, sizeof(float) * n);
     return e;
-}
-
-// Counts launches and, while profiling (never during capture), records an event after each.
-struct Marker {
-    akua_pbf* s;
-    cudaStream_t st;
-    bool record;
-    int launches = 0;
-    void operator()(const char* name) {
-        ++launches;
-        if (record && s->prof_next < s->prof_events.size()) {
-            cudaEventRecord(s->prof_events[s->prof_next], st);
-            s->prof_names[s->prof_next] = name;
-            ++s->prof_next;
-        }
-    }
-};
-
-// A kernel of the body's chain.
-template <class... Params, class... Args>
-void step_kernel(const akua_pbf* s, cudaStream_t st, void (*kernel)(Params...), int grid, int block,
-                 size_t smem, Args... args) {
-    akua::radix::launch(s->chain, kernel, grid, block, smem, st, 1, args...);
-}
-
-// The walk at one tile shape (BLOCK threads, a pool of 32 x STAGE words per warp).
-template <bool EXACT, int BLOCK, int STAGE>
-void launch_search_shape(akua_pbf* s, cudaStream_t st, int density, float* feat) {
-    constexpr size_t smem = akua::search_smem(BLOCK, STAGE);
-    const int per_warp = akua::search_per_warp(s->n, s->sms, EXACT);
-    auto go = [&](auto kernel) {
-        if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        step_kernel(s, st, kernel, grid_for(s->n, per_warp * (BLOCK / 32)), BLOCK, smem, s->d_params,
-                    s->ps0, s->table, s->r2i, s->nbr, s->cnt, s->rho, s->lam, s->flags, density,
-                    s->speed, s->lprev, s->lacc, feat, s->psl, per_warp);
-    };
-    if (EXACT && per_warp <= akua::kFewPerWarp) go(akua::k_search<EXACT, BLOCK, STAGE, EXACT>);
-    else go(akua::k_search<EXACT, BLOCK, STAGE, false>);
-}
-
-template <bool EXACT>
-void launch_search(akua_pbf* s, cudaStream_t st, int density, float* feat) {
-    const int b = s->search_block, g = s->search_stage;
-    if (g == 48) {  // 64 or 128 threads (akua_pbf_set_search_shape refuses 256)
-        if (b == 64) launch_search_shape<EXACT, 64, 48>(s, st, density, feat);
-        else launch_search_shape<EXACT, 128, 48>(s, st, density, feat);
-    } else if (g == 16) {
-        if (b == 64) launch_search_shape<EXACT, 64, 16>(s, st, density, feat);
-        else if (b == 256) launch_search_shape<EXACT, 256, 16>(s, st, density, feat);
-        else launch_search_shape<EXACT, 128, 16>(s, st, density, feat);
-    } else {
-        if (b == 64) launch_search_shape<EXACT, 64, 32>(s, st, density, feat);
-        else if (b == 256) launch_search_shape<EXACT, 256, 32>(s, st, density, feat);
-        else launch_search_shape<EXACT, 128, 32>(s, st, density, feat);
-    }
-}
-
-template <bool EXACT, int LANES>
-void enqueue_pairs(akua_pbf* s, cudaStream_t st, Marker& mark) {
-    const int n = s->n;
-    const int* pb = s->pair_block;  // per kernel: density, delta, last delta, vort., conf., XSPH
-    auto gp = [&](int k) { return grid_for(n, pb[k] / LANES); };
-    const int iters = s->cfg.solverIterations;
-    float4* ps[2] = {s->ps0, s->ps1};
-    const uint4* nbr4 = reinterpret_cast<const uint4*>(s->nbr);
-    const int learn = learn_mode(s);
-    launch_search<EXACT>(s, st, iters > 0 ? 1 : 0, learn ? s->feat : nullptr);
-    mark("k_search");
-    if (learn == 2) {
-        akua::mlp::enqueue_forward(s->warm, s->feat, n, s->lam, s->lacc, &s->psl->w, st);
-        mark("k_mlp_forward");
-    }
-    for (int it = 0; it < iters; ++it) {
-        float4* cur = ps[it & 1];
-        float4* nxt = ps[(it + 1) & 1];
-        if (it > 0) {
-            step_kernel(s, st, akua::k_density_lambda<EXACT, LANES>, gp(0), pb[0], 0,
-                        s->d_params, cur, nbr4, s->cnt, s->rho, s->lam,
-                        learn == 1 ? s->lacc : nullptr, s->psl);  // warm: the network's estimate is the sum
-            mark("k_density_lambda");
-        }
-        if (it + 1 < iters) {
-            step_kernel(s, st, akua::k_delta_correct<EXACT, LANES>, gp(1), pb[1], 0,
-                        s->d_params, cur, s->lam, nbr4, s->cnt, nxt, s->dp4, s->psl, s->mass_bits);
-            mark("k_delta_correct");
-        } else {
-            step_kernel(s, st, akua::k_delta_final<EXACT, LANES>, gp(2), pb[2], 0,
-                        s->d_params, cur, s->lam, nbr4, s->cnt, s->x4g, s->x4, s->v4, s->vstar4, s->dp4,
-                        s->origing, s->origin, s->rrefg, s->rref, s->rhog, s->lamg, s->dpg,
-                        s->rho, nullptr, 1, s->psl, s->mass_bits, s->xv8);  // lam_out: zero iterations only
-            mark("k_delta_final");
-        }
-    }
-    if (iters == 0) {
-        step_kernel(s, st, akua::k_delta_final<EXACT, LANES>, gp(2), pb[2], 0,
-                    s->d_params, s->ps0, nullptr, nbr4, s->cnt, s->x4g, s->x4, s->v4, s->vstar4, s->dp4,
-                    s->origing, s->origin, s->rrefg, s->rref, s->rhog, s->lamg, s->dpg,
-                    s->rho, s->lam, 0, s->psl, s->mass_bits, s->xv8);  // no delta: lambda is not read
-        mark("k_delta_final");
-    }
-    // psl is free after the last delta: it carries (x, |omega|) to confinement
-    step_kernel(s, st, akua::k_vorticity<EXACT, LANES>, gp(3), pb[3], 0,
-                s->d_params, s->x4, s->v4, s->xv8, nbr4, s->cnt, s->om4, s->psl);
-    mark("k_vorticity");
-    step_kernel(s, st, akua::k_confine<EXACT, LANES>, gp(4), pb[4], 0,
-                s->d_params, s->x4, s->v4, s->om4, s->rho, nbr4, s->cnt, s->xv8, s->psl, s->mass_bits);
-    mark("k_confine");
-    step_kernel(s, st, akua::k_xsph<LANES>, gp(5), pb[5], 0,
-                s->d_params, s->xv8, nbr4, s->cnt, s->v4, s->kr, s->table);
-    mark("k_xsph");
 }
 
 // Everything of a step after the parameter upload and the import: the captured body.
@@ -456,20 +236,8 @@ void enqueue_body(akua_pbf* s, cudaStream_t st, const char* aos, size_t stride, 
     step_kernel(s, st, akua::k_table_build, ge, akua::kElemBlock, 0,
                 s->d_params, s->kr, s->r2i, s->table);
     mark("k_table_build");
-    const bool exact = (s->options & AKUA_PBF_OPT_EXACT_MATH) != 0;
-    switch (akua::pair_lanes(n, s->sms, exact)) {
-        case 8:
-            exact ? enqueue_pairs<true, 8>(s, st, mark) : enqueue_pairs<false, 8>(s, st, mark);
-            break;
-        case 4:
-            exact ? enqueue_pairs<true, 4>(s, st, mark) : enqueue_pairs<false, 4>(s, st, mark);
-            break;
-        case 2:
-            exact ? enqueue_pairs<true, 2>(s, st, mark) : enqueue_pairs<false, 2>(s, st, mark);
-            break;
-        default:
-            exact ? enqueue_pairs<true, 1>(s, st, mark) : enqueue_pairs<false, 1>(s, st, mark);
-    }
+    if (s->options & AKUA_PBF_OPT_EXACT_MATH) akua::enqueue_pairs_exact(s, st, mark);
+    else akua::enqueue_pairs_fast(s, st, mark);
     if (aos) {
         step_kernel(s, st, akua::k_export, grid_for(n, akua::kIoBlock), akua::kIoBlock, 0,
                     s->d_params, const_cast<char*>(aos), stride, n, s->r2i, s->kr, s->x4, s->v4,
