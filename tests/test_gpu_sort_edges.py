@@ -49,3 +49,18 @@ def test_step_order_at_sort_edges(cuda_lib, n):
     o, oe = run_oracle(sc, cfg, corr, 2)
     assert_grid_equal(ge, oe, cfg.maxNeighbours)
     assert_records_bitexact(g, o)
+
+
+@pytest.mark.parametrize("n", [262143, 262144, 262145, 266241])
+@pytest.mark.parametrize("bits", [8, 9, 20, 27])
+def test_sort_pairs_around_64_tiles(cuda_lib, n, bits):
+    """Up to 64 tiles a pass's scatter adds the tiles' counts up itself, beyond them the scan does: 64
+    tiles but for a pair, 64, 65 (an uneven split of the scan's work) and 66 of one pair; passes of
+    8, 9 and 10 bits."""
+    test_sort_pairs_edges(cuda_lib, n, bits)
+
+
+@pytest.mark.parametrize("n", [262144, 262145])
+def test_step_order_around_64_tiles(cuda_lib, n):
+    """The order of two steps on both sides of that line, against the oracle."""
+    test_step_order_at_sort_edges(cuda_lib, n)
