@@ -200,8 +200,8 @@ __device__ __forceinline__ void load_features(const float* __restrict__ feat, in
 //
 // Bound by the SiLU epilogues' issue slots and by a tile's chain of three MMAs, which the other
 // warpgroups' epilogues fill: two CTAs of four warpgroups per SM (64 registers a thread).
-// 1M samples: 72 -> 67 us against five CTAs of one warpgroup with scalar epilogues, 155,648: 20.5 ->
-// 16.4 (the hardware tanh of 192 activations a sample alone takes about 40 at 1M).
+// 1M samples: 74 -> 65 us against five CTAs of one warpgroup with scalar epilogues, 155,648: 20.7 ->
+// 12.9 (the hardware tanh of 192 activations a sample alone takes about 40 at 1M).
 __global__ void __launch_bounds__(kFwdThreads, 2)
     k_mlp_forward(const float* __restrict__ params, const uint8_t* __restrict__ image,
                   const float* __restrict__ norm, const float* __restrict__ feat, int n,

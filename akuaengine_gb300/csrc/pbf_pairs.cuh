@@ -219,7 +219,7 @@ __device__ __forceinline__ void for_each_neighbour(const uint4* __restrict__ nbr
 // Lanes per particle of the pair kernels.  A scene too small to fill the chip is as slow as the chain
 // of gathers of one list, which more lanes shorten, until the shuffles cost more issue slots than the
 // chain costs time: about 10 warps per SM with 8 lanes (22 with exact math, whose terms are longer)
-// and 18 with 4 or 2 (24, all that fit at 80 registers).  Steps in us with 4 / 8 / 16 lanes: 1,000
+// and 18 with 4 or 2 (24 with exact math: all that fit of its kernels of up to 80 registers).  Steps in us with 4 / 8 / 16 lanes: 1,000
 // particles 70 / 66 / 68, 4,000 80 / 77 / 84, 6,000 82.6 / 82.2 / 92, 8,000 85 / 87; exact 1,000
 // 88 / 75 / 72, 4,000 105 / 89 / 92, 12,000 118 / 109, 16,000 124 / 132.  With 1 / 2 / 4: 20,000 116 /
 // 110 / 105, 27,000 120 / 111 / 114, 45,000 134 / 132, 52,000 140 / 144; exact 27,000 183 / 160 / 139,
@@ -620,8 +620,9 @@ __global__ void __launch_bounds__(kMaxPairBlock)
 
 // Vorticity confinement (IntegrationCUDA.cu:130-165); writes the confined velocity to the
 // particle records (x, m_i / rho_i | v) for the XSPH pass.
-// Capped at 48 registers (five 256-thread blocks per SM): 80 µs against 84 at 60 registers on the
-// 1M scene, although 36 bytes spill; the same cap slowed vorticity and the last delta pass.
+// Capped at 48 registers (five 256-thread blocks per SM; 40 bytes spill, 60 in exact math), which slowed
+// vorticity and the last delta pass.  1M particles capped and not: exact math 114 and 117 us, fast math
+// 74 and 70 (80 and 84 before the pair loop took fewer instructions).
 template <bool EXACT, int LANES>
 __global__ void __launch_bounds__(kMaxPairBlock, LANES == 1 ? 5 : 1)
     k_confine(const StepParams* __restrict__ P, const float4* __restrict__ x4,

@@ -15,10 +15,9 @@ namespace akua {
 template <bool EXACT, int BLOCK, int STAGE>
 void launch_search_shape(akua_pbf* s, cudaStream_t st, int density, float* feat) {
     constexpr size_t smem = search_smem(BLOCK, STAGE);
+    static_assert(smem <= 48 * 1024, "above the default limit of dynamic shared memory");
     const int per_warp = search_per_warp(s->n, s->sms, EXACT);
     auto go = [&](auto kernel) {
-        if (smem > 48 * 1024)  // above the default limit of dynamic shared memory
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         step_kernel(s, st, kernel, grid_for(s->n, per_warp * (BLOCK / 32)), BLOCK, smem, s->d_params,
                     s->ps0, s->table, s->r2i, s->nbr, s->cnt, s->rho, s->lam, s->flags, density,
                     s->speed, s->lprev, s->lacc, feat, s->psl, per_warp);

@@ -257,7 +257,10 @@ void invalidate_graph(akua_pbf* s) {
 }
 
 void update_plans(akua_pbf* s, int sp_bits) {
-    // one scene of few particles: a pass is one cluster; a batch holds many scenes' particles
+    // A single scene sorts by its size: one cluster a pass, scatters that add up the counts, or the scan
+    // beside them.  A batch takes the scan at any size: it is there for many scenes at once (256 scenes:
+    // 5 M particles), where the other two forms do not apply.  (What they would give a batch of a few
+    // small scenes is not measured.)
     const bool small = s->scenes.empty() && s->cluster_sort;
     auto plan = [&](int bits) {
         if (small) return akua::radix::make_cluster_plan(bits, s->n);

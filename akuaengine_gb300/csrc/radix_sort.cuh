@@ -10,7 +10,8 @@
 // pass: per-tile digit counts, a scan of the (tile, digit) count matrix over the tiles (for inputs of
 // few tiles in the scatter itself), and a stable scatter in which warps rank their keys by ballots and
 // per-warp running digit counters, order the tile in shared memory and store it in runs.  Inputs of
-// at most kClusterMax pairs take one launch per pass.
+// at most kClusterMax pairs take one launch per pass, with digits of up to 9 or 11 bits
+// (make_cluster_plan).
 #pragma once
 
 #include <cstdint>
@@ -370,12 +371,13 @@ inline void run_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, u
 // ---- Sorts of up to kClusterMax pairs: a pass in one kernel, on one cluster of blocks.
 //
 // A tiled pass over a small input is three launches, each a few microseconds of latency for next to
-// no work.  Here one cluster holds all pairs in registers: a block ranks its own (match.any and
-// per-warp digit counters, as downsweep does), reads the other blocks' digit totals through
-// distributed shared memory, scans them and scatters to global memory.
-// Sorts of random keys in three passes: 27,000 pairs 56 -> 16.5 us, 65,536 34 -> 24; in two, 4,096:
-// 39 -> 7.  The step of 27,000 particles: 158 -> 129 us.  (With 32-bit counters 27,000 took 17.9 us and
-// 4,096 7.8: the scan over the warps' counters and their zeroing are twice the shared memory.)
+// no work.  Here one cluster holds all pairs in registers: a block ranks its own (ballots or match.any,
+// and per-warp digit counters), reads the other blocks' digit totals through distributed shared memory,
+// scans them and scatters to global memory.
+// Sorts of random keys in three passes: 27,000 pairs 56 -> 16.7 us, 65,536 34 -> 24.3; in two, 4,096:
+// 39 -> 7.4.  The step of 27,000 particles went from 158 to 129 us with it.  (With 32-bit counters 27,000
+// took 17.9 us and 4,096 7.8: the scan over the warps' counters and their zeroing are twice the shared
+// memory.)
 constexpr int kClusterThreads = 512;
 constexpr int kClusterWarps = kClusterThreads / 32;
 constexpr int kClusterMax = 16 * kClusterThreads * 8;         // 65,536: eight rounds of 16 blocks
@@ -384,8 +386,7 @@ constexpr int kClusterPortableMax = 8 * kClusterThreads * 4;  // 16,384: four ro
 // Digits of up to 9 bits (one per thread in the scans), or of up to 11 (four) where that saves a pass
 // of 8 blocks and two or four rounds: 8,192 pairs of 19 bits 13.0 -> 10.6 us, 16,384 of 20 16.1 ->
 // 14.8.  16 blocks read twice the counts from one another (27,000 of 21 bits 17.8 -> 19.6, 65,536 of
-// 32 32.6 -> 35.3).  One round would gain little (4,096 of 20 bits 11.2 -> 10.4), and the tests hold
-// a step of 4,096 particles to 20 launches.
+// 32 32.6 -> 35.3).  One round would gain 0.8 us of a step of 80 (4,096 of 20 bits 11.2 -> 10.4).
 inline Plan make_cluster_plan(int bits, int n) {
     Plan p;
     p.cluster = true;
@@ -571,8 +572,8 @@ __global__ void __launch_bounds__(kClusterThreads)
 
 // One pass of a sort of n <= kClusterMax pairs.  RUNS: neighbouring pairs mostly have equal digits
 // (a scene's particles, which come in the previous step's order), so a warp's match.any finds few
-// distinct values; it then beats a ballot per bit (27,000 particles: 136 against 140 us a step, but
-// 27 against 22 us for a sort of as many random keys).
+// distinct values; it then beats a ballot per bit (27,000 particles 110.5 against 111.6 us a step,
+// 60,000 143 against 146, but 19.5 against 16.7 us for a sort of 27,000 random keys).
 template <bool RUNS, class Mark>
 inline void run_cluster_pass(cudaStream_t s, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                              uint32_t* vout, int n, int shift, int width, uint32_t* rank_out,

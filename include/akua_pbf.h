@@ -337,8 +337,8 @@ int akua_splat_render(akua_splat* renderer, const void* deviceParticles, size_t 
  * the step; with a network attached, a step's first Jacobi iteration uses that prediction instead
  * of the one-step estimate and the remaining iterations run unchanged.
  * Features (float[8] per particle): rho/rho0 - 1, neighbours / 32, the lambda denominator without
- * epsilon, iteration 1's lambda, the previous step's accumulated lambda, the mean rho_j/rho0 - 1
- * of the neighbours, the SPH divergence of the predicted velocity, |predicted velocity|.
+ * epsilon, iteration 1's lambda, the previous step's accumulated lambda, |grad_i C_i|, its component
+ * along gravity, |predicted velocity|.
  * Parameters (float[AKUA_MLP_PARAMS], FP32 master copy): W1[64][8], b1[64], W2[64][64], b2[64],
  * W3[64][64], b3[64], w4[64], b4.  Normalisation (float[AKUA_MLP_NORM]): mean[8], inv_std[8] of
  * the features, the output scale (the network's output times it is the estimate p of the
