@@ -11,10 +11,11 @@
 // none of these loads is an .nc one, whose data must not change while the kernel is resident.
 //
 // What kernels before the previous one wrote is complete when a kernel starts (the previous one's
-// blocks have all passed their own wait by then), so within a chain only the previous kernel's output
-// is passed, and the rest is read as ever.  With every input passed a step of 1M particles takes 1,154
-// us against 1,129 (the walk 278 against 259: its loads then keep their place among the warp
-// barriers).  Without the launch attribute the wait does nothing.
+// blocks have all passed their own wait by then, or it was launched without the attribute), so within
+// a chain only the previous kernel's output is passed, and the rest is read as ever.  (With every input
+// passed, and the walk waiting too, a step of 1M particles takes 1,154 us against 1,129: the walk's
+// loads then keep their place among the warp barriers.)  Without the launch attribute the wait does
+// nothing.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -138,7 +138,6 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
     const float4* pair_xy = reinterpret_cast<const float4*>(pairs);  // (xa, xb, ya, yb)
     const float2* pair_z = reinterpret_cast<const float2*>(pairs + 64);
 
-    pdl::wait_for_previous(table);
     const float4 xi = valid ? ps[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int cx = cell_coord(xi.x, p.search_cell);
     const int cy = cell_coord(xi.y, p.search_cell);
@@ -168,8 +167,8 @@ __global__ void __launch_bounds__(BLOCK, (EXACT ? 768 : 1024) / BLOCK)
         const StepParams& pr = P[__shfl_sync(kFullWarp, sid, q)];  // the run's scene
         uint2 e = make_uint2(0u, 0u);
         if (lane < 27)
-            e = table[pr.table_offset +
-                      cell_hash(rx + bdx, ry + bdy, rz + bdz, pr.table_size, pr.table_magic)];
+            e = __ldg(table + pr.table_offset +
+                      cell_hash(rx + bdx, ry + bdy, rz + bdz, pr.table_size, pr.table_magic));
         return e;
     };
 

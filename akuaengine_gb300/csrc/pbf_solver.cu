@@ -200,9 +200,9 @@ void enqueue_body(akua_pbf* s, cudaStream_t st, const char* aos, size_t stride, 
     const int ge = grid_for(n, akua::kElemBlock);
     Marker mark{s, st, record};
     const bool carry = s->cfg.solverIterations == 0;
-    // Each kernel from the table build on is set up while the one before it ends (the gather joins two
-    // branches): 3 to 4 us of a step up to 100,000 particles (119.7 -> 116.6 at 27,000), nothing
-    // at 1M.  Not between the events of a profile.
+    // Each kernel from the table build on but the walk is set up while the one before it ends (the gather
+    // joins two branches): 3 to 4 us of a step up to 100,000 particles (119.7 -> 116.6 at 27,000),
+    // nothing at 1M.  Not between the events of a profile.
     s->chain = !record;
     uint32_t* dummy = nullptr;
     // The two sorts are independent: reference order, stable by (hash, previous reference rank),

@@ -57,7 +57,6 @@ def test_one_wait():
 # that one wrote is complete when a kernel starts.
 PREVIOUS = {
     "k_table_build": {"r2i"},                           # k_gather
-    "k_search": {"table"},                              # k_table_build
     "k_density_lambda": {"ps"},                         # k_delta_correct
     "k_delta_correct": {"lam", "psl", "nbr4", "cnt"},   # k_search, k_mlp_forward, k_density_lambda
     "k_delta_final": {"lam", "psl", "nbr4", "cnt"},
@@ -80,6 +79,16 @@ def _waiting():
 def test_waiting_kernels_are_found():
     names = {k[1] for k in _waiting()}
     assert set(PREVIOUS) | {"k_mlp_forward", "k_mlp_grad", "k_splat_large", "k_splat_resolve"} == names
+
+
+def test_kernels_set_up_early_wait():
+    """The kernels of a step that are launched with the attribute (step_kernel)."""
+    names = {k[1] for k in _waiting()}
+    early = set()
+    for text in _sources().values():
+        early |= set(re.findall(r"\bstep_kernel\(s, st, (?:akua::)?(k_\w+)", text))
+        assert not re.search(r"\bstep_kernel\(s, st, (?!(?:akua::)?k_)", text)
+    assert {"k_table_build", "k_density_lambda", "k_export"} <= early <= names, early - names
 
 
 @pytest.mark.parametrize("kernel", _waiting(), ids=lambda k: k[1])
