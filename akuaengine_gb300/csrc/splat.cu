@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <new>
 
 #include "akua_pbf.h"
@@ -93,24 +94,36 @@ __device__ __forceinline__ unsigned long long seen(const unsigned long long* z) 
     return v;
 }
 
-// A warp draws `per_warp` particles: a sprite of at most 2 * per_warp pixels by its own lane, a larger
-// one by the whole warp, one after another.  32 particles per warp keep the lanes of a large scene
-// busy; a scene too small to fill the chip that way has fewer per warp (splat_per_warp), or its
-// large sprites would wait for each other (1,000 particles of 40 pixels across: 171 us against 17).
-// A sprite of more than kQueuePixels is queued, in parts, for k_splat_large: particles near the eye
-// come cell by cell, and warps that draw 32 of them keep the frame waiting (1M particles with the
-// eye among them: 5.5 ms; a warp for every particle 0.94; queued 0.12).
-// 1M particles at 1280 x 720: a frame 57 -> 21 us (projection and its buffers, 35 us of atomics and
-// a cleared depth buffer before); 4M at 1920 x 1080: 182 -> 45.
-constexpr int kQueuePixels = 256;
-constexpr int kPartPixels = 1024;       // of a queued sprite per part, at least
-constexpr int kMaxParts = 64;
-constexpr uint32_t kQueue = 1u << 20;   // parts; a frame with more draws the rest by their warps
+// A warp takes `per_warp` particles.  A sprite of at most `lane_pixels` is drawn by its own lane, which
+// reads a pixel's key before it sends an atomic (there are most particles, and most hidden ones, where
+// sprites are small); a larger one by the whole warp, one sprite after another, with plain atomics:
+// 32 in flight at once wait for nothing, where a read first made each 32 pixels wait for L2 (30,000
+// sprites of 13 pixels across 47 us with reads, 35 without, 25 across 118 and 70).  A sprite of more
+// than `warp_pixels` is queued, in parts, for k_splat_large: particles near the eye come cell by cell,
+// and warps that draw all of theirs keep the frame waiting.
+// 32 particles per warp keep the lanes of a large scene busy; a scene too small to fill the chip that
+// way has fewer per warp (splat_per_warp), or its sprites would wait for each other (1,000 particles of
+// 40 pixels across: 171 us against 17).
+// Frames of 1280 x 720 in us with a warp per particle, a projection pass and a cleared depth buffer, and
+// like this: 1M particles with sprites of 1 to 4 pixels 176 and 37, of 12 across 628 and 424; 30,000
+// with sprites of 5, 13 and 25 across 23, 37, 75 and 18, 35, 70; the eye among 27,000 particles 1,396 and
+// 54, among 1M 836 and 164, in front of 100,000 with small sprites 33 and 35; 4M particles 657 and 93.
+struct Shape {
+    int per_warp;     // particles
+    int lane_pixels;  // most pixels of a lane's sprite
+    int warp_pixels;  // most pixels of a warp's sprite
+};
+constexpr int kPartPixels = 1024;      // of a queued sprite per part, at least
+constexpr int kMaxParts = 64;          // of a sprite
+constexpr uint32_t kQueue = 1u << 20;  // parts; a frame with more draws the rest by their warps
+// Parts a frame may want before its sprites get at most 16, and 4: 30,000 sprites of half the image,
+// which want 1.9M parts, 14.9 ms where the first half of the queue went to sprites in 64 parts 20.4.
+constexpr unsigned long long kWantedFew = kQueue / 4, kWantedMany = kQueue;
 constexpr unsigned long long kNoPart = ~0ull;
 struct Queue {
-    uint32_t count;  // parts asked for, 0 between frames
-    uint32_t pad;
-    unsigned long long part[kQueue];  // particle | part << 32
+    unsigned long long count;   // parts asked for, 0 between frames
+    unsigned long long wanted;  // parts wanted at kMaxParts a sprite, 0 between frames
+    unsigned long long part[kQueue];  // particle | part << 32 | parts << 40
 };
 
 // The next kernel of the stream may start once every block has got here, and waits for this one's
@@ -119,7 +132,6 @@ __device__ __forceinline__ void let_next_start() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Draws the pixels first, first + step, ... of a sprite.
 struct Sprite {
     float4 q;
     unsigned long long key;
@@ -135,49 +147,103 @@ struct Sprite {
         ny = max(0, y1 - y0 + 1);
         key = ((unsigned long long)__float_as_uint(fmaxf(q.z, 0.0f)) << 32) | (unsigned)i;
     }
-    __device__ __forceinline__ int parts() const {
-        return min(kMaxParts, (nx * ny + kPartPixels - 1) / kPartPixels);
+    __device__ __forceinline__ uint32_t parts(int most) const {
+        return (uint32_t)min(most, (nx * ny + kPartPixels - 1) / kPartPixels);
     }
+    // The place of pixel k in the depth buffer, if it lies in the disc.
+    __device__ __forceinline__ bool pixel(const SplatParams& P, int k, float inv, size_t& at) const {
+        const int row = k / nx, px = x0 + (k - row * nx), py = y0 + row;
+        at = (size_t)py * P.width + px;
+        return in_disc(((float)px + 0.5f) - q.x, ((float)py + 0.5f) - q.y, q.w, inv);
+    }
+    // Draws the pixels first, first + step, ...
     __device__ __forceinline__ void draw(const SplatParams& P, unsigned long long* zbuf, int first,
                                          int step) const {
         const float inv = 1.0f / q.w;
         const int count = nx * ny;
         for (int k = first; k < count; k += step) {
-            const int row = k / nx, px = x0 + (k - row * nx), py = y0 + row;
-            unsigned long long* at = zbuf + (size_t)py * P.width + px;
-            if (in_disc(((float)px + 0.5f) - q.x, ((float)py + 0.5f) - q.y, q.w, inv) &&
-                key < seen(at))
-                atomicMin(at, key);
+            size_t at;
+            if (pixel(P, k, inv, at)) atomicMin(zbuf + at, key);
+        }
+    }
+    // Draws all pixels where the key read is farther; the reads of two are in flight at once.
+    __device__ __forceinline__ void draw_nearer(const SplatParams& P, unsigned long long* zbuf) const {
+        const float inv = 1.0f / q.w;
+        const int count = nx * ny;
+        for (int k = 0; k < count; k += 2) {
+            size_t at[2];
+            unsigned long long z[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                z[u] = k + u < count && pixel(P, k + u, inv, at[u]) ? seen(zbuf + at[u]) : 0ull;
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (key < z[u]) atomicMin(zbuf + at[u], key);
         }
     }
 };
 
-__global__ void __launch_bounds__(256)
-    k_splat_raster(SplatParams P, const char* __restrict__ aos, uint64_t stride, int n,
-                   int per_warp, unsigned long long* __restrict__ zbuf,
-                   Queue* __restrict__ queue) {
-    const int lane = threadIdx.x & 31;
-    const int64_t at0 = ((int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) * per_warp;
-    if (at0 >= n) return;  // uniform over the warp (and a block that ends lets the next one start)
-    const int i = (int)at0 + lane;
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (lane < per_warp && i < n) q = project(P, reinterpret_cast<const float*>(aos + (uint64_t)i * stride));
-    Sprite me(P, q, i);
-    const int count = me.nx * me.ny;
-    bool whole = count > 2 * per_warp;
-    if (!whole) {
-        me.draw(P, zbuf, 0, 1);
-    } else if (count > kQueuePixels) {
-        const uint32_t parts = (uint32_t)me.parts();
-        // a full queue is not counted further, so the count cannot wrap
-        const uint32_t at = *(volatile uint32_t*)&queue->count < kQueue
-                                ? atomicAdd(&queue->count, parts)
-                                : kQueue;
-        whole = at > kQueue - kMaxParts;  // no room: the slots that exist hold nothing
-        for (uint32_t k = 0; k < parts && at + k < kQueue && at < kQueue; ++k)
-            queue->part[at + k] =
-                whole ? kNoPart : (unsigned long long)k << 32 | (unsigned long long)(uint32_t)i;
+constexpr int kRasterWarps = 8;
+
+// Sum of `v` over the lower threads of the block; sums[kRasterWarps] becomes the block's.
+__device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* sums) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t upto = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += x;
     }
+    __syncthreads();  // `sums` may still be read from an earlier call
+    if (lane == 31) sums[warp] = upto;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t all = 0;
+        for (int w = 0; w < kRasterWarps; ++w) {
+            const uint32_t x = sums[w];
+            sums[w] = all;
+            all += x;
+        }
+        sums[kRasterWarps] = all;
+    }
+    __syncthreads();
+    return sums[warp] + (upto - v);
+}
+
+// Six blocks per SM (40 registers; with 44 and five blocks 4M particles take 98 us instead of 93).
+__global__ void __launch_bounds__(32 * kRasterWarps, 6)
+    k_splat_raster(SplatParams P, const char* __restrict__ aos, uint64_t stride, int n, Shape shape,
+                   unsigned long long* __restrict__ zbuf, Queue* __restrict__ queue) {
+    const int lane = threadIdx.x & 31;
+    const int64_t i = ((int64_t)blockIdx.x * kRasterWarps + (threadIdx.x >> 5)) * shape.per_warp + lane;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane < shape.per_warp && i < n)
+        q = project(P, reinterpret_cast<const float*>(aos + (uint64_t)i * stride));
+    Sprite me(P, q, (int)i);
+    const int count = me.nx * me.ny;
+    bool whole = count > shape.lane_pixels;
+    const bool large = count > shape.warp_pixels;
+    if (__syncthreads_or(large)) {  // one reservation per block: 1 ns each on one address
+        __shared__ uint32_t sums[kRasterWarps + 1];
+        __shared__ unsigned long long wanted, from;
+        uint32_t parts = large ? me.parts(kMaxParts) : 0u;
+        uint32_t below = block_prefix(parts, sums);
+        if (threadIdx.x == 0)
+            wanted = atomicAdd(&queue->wanted, (unsigned long long)sums[kRasterWarps]);
+        __syncthreads();
+        if (wanted >= kWantedFew) {
+            parts = large ? me.parts(wanted < kWantedMany ? 16 : 4) : 0u;
+            below = block_prefix(parts, sums);
+        }
+        if (threadIdx.x == 0) from = atomicAdd(&queue->count, (unsigned long long)sums[kRasterWarps]);
+        __syncthreads();
+        const unsigned long long at = from + below;
+        if (large) whole = at + parts > kQueue;  // no room: the slots that exist hold nothing
+        for (uint32_t k = 0; k < parts && at + k < kQueue; ++k)
+            queue->part[at + k] =
+                whole ? kNoPart : (unsigned long long)(parts << 8 | k) << 32 | (uint32_t)i;
+    }
+    if (count <= shape.lane_pixels) me.draw_nearer(P, zbuf);
     unsigned big = __ballot_sync(0xffffffffu, whole);
     while (big) {
         const int src = __ffs(big) - 1;
@@ -202,15 +268,16 @@ __global__ void __launch_bounds__(256)
                   unsigned long long* __restrict__ zbuf, const Queue* __restrict__ queue) {
     akua::pdl::wait_for_previous(aos, zbuf, queue);
     let_next_start();
-    const uint32_t count = min(__ldcg(&queue->count), kQueue), warps = gridDim.x * (blockDim.x / 32);
+    const uint32_t count = (uint32_t)min(__ldcg(&queue->count), (unsigned long long)kQueue);
+    const uint32_t warps = gridDim.x * (blockDim.x / 32);
     const int lane = threadIdx.x & 31;
     for (uint32_t e = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); e < count; e += warps) {
         const unsigned long long part = __ldcg(&queue->part[e]);
         if (part == kNoPart) continue;
         const uint32_t i = (uint32_t)part;
-        const float4 q = project(P, reinterpret_cast<const float*>(aos + (uint64_t)i * stride));
-        const Sprite s(P, q, (int)i);
-        s.draw(P, zbuf, 32 * (int)(part >> 32) + lane, 32 * s.parts());
+        const int k = (int)(part >> 32) & 0xff, parts = (int)(part >> 40);  // parts is at least 1
+        const Sprite s(P, project(P, reinterpret_cast<const float*>(aos + (uint64_t)i * stride)), (int)i);
+        s.draw(P, zbuf, 32 * k + lane, 32 * parts);
     }
 }
 
@@ -225,7 +292,7 @@ __global__ void __launch_bounds__(256)
                     uint32_t* __restrict__ rgba) {
     akua::pdl::wait_for_previous(aos, zbuf, queue);
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) queue->count = 0u;  // for the next frame
+    if (p == 0) queue->count = queue->wanted = 0ull;  // for the next frame
     if (p >= P.width * P.height) return;
     const int px = p % P.width, py = p / P.width;
     const unsigned long long key = __ldcg(zbuf + p);  // not an older one in this SM's L1
@@ -247,11 +314,25 @@ __global__ void __launch_bounds__(256)
 }
 
 // Particles per warp: the most (a power of two, at most 32) at which the warps still fill the chip
-// once, 32 of them per SM.
+// once, 32 of them per SM.  (64 of them: 100,000 particles with small sprites 20.5 us against 16.5, 120,000
+// with sprites of 5 pixels across 31 against 33.)
 int splat_per_warp(int n, int sms) {
     int w = 1;
     while (w < 32 && (int64_t)n >= 2ll * w * 32 * sms) w *= 2;
     return w;
+}
+
+// Up to 64 warps of 32 particles per SM a frame lasts as long as its warps' chains, so few pixels go
+// one after another and sprites go to the queue early; beyond that it is bound by atomics, and a lane's
+// reads save them.  us with 9 and 64 pixels per lane: 120,000 sprites of 5 across 33 and 45, 300,000 of
+// 9 across 90 and 118, but 1M of 3 to 5 132 and 92.  With 96 and 256 pixels per warp: the eye in front
+// of 100,000 particles 33 and 41, among 300,000 35 and 45, but 1M sprites of 12 across 551 (128 pixels)
+// and 424.
+Shape splat_shape(int n, int sms) {
+    const int w = splat_per_warp(n, sms);
+    const bool crowded = n > 64ll * 32 * sms;
+    const int lane = std::min(2 * w, crowded ? 64 : 9);
+    return {w, lane, std::max(lane, crowded ? 256 : 96)};
 }
 
 // A launch that may begin while the stream's previous kernel ends (the kernel waits for it).
@@ -381,7 +462,7 @@ int akua_splat_create(int32_t width, int32_t height, akua_splat** out) {
     cudaError_t e = cudaMalloc(&r->zbuf, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&r->queue, sizeof(Queue));
     if (e == cudaSuccess) e = cudaMemset(r->zbuf, 0xFF, bytes);
-    if (e == cudaSuccess) e = cudaMemset(&r->queue->count, 0, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(r->queue, 0, offsetof(Queue, part));
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // any stream may render next
     if (e != cudaSuccess) {
         cudaFree(r->zbuf);
@@ -419,14 +500,15 @@ int akua_splat_render(akua_splat* r, const void* particles, size_t stride, int32
     const size_t pixels = (size_t)r->width * r->height;
     if (r->dirty) {  // the last frame failed between its first and its last launch
         cudaError_t e = cudaMemsetAsync(r->zbuf, 0xFF, sizeof(unsigned long long) * pixels, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(&r->queue->count, 0, sizeof(uint32_t), st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(r->queue, 0, offsetof(Queue, part), st);
         if (e != cudaSuccess) return status_of(e);
     }
     const char* aos = static_cast<const char*>(particles);
     if (n > 0) {
-        const int per_warp = splat_per_warp(n, r->sms), per_block = 8 * per_warp;
-        k_splat_raster<<<(unsigned)((n + (int64_t)per_block - 1) / per_block), 256, 0, st>>>(
-            P, aos, stride, n, per_warp, r->zbuf, r->queue);
+        const Shape shape = splat_shape(n, r->sms);
+        const int per_block = kRasterWarps * shape.per_warp;
+        k_splat_raster<<<(unsigned)((n + (int64_t)per_block - 1) / per_block), 32 * kRasterWarps, 0, st>>>(
+            P, aos, stride, n, shape, r->zbuf, r->queue);
         launch_after(k_splat_large, 8 * r->sms, st, P, aos, (uint64_t)stride, r->zbuf,
                      static_cast<const Queue*>(r->queue));
     }

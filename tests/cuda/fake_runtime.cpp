@@ -30,9 +30,9 @@ int set(void* p, int v, size_t n) {
 bool marked() {
     for (size_t k = 0; k < allocated[0].second; ++k)
         if (allocated[0].first[k] != 0xFF) return true;
-    unsigned count;
-    std::memcpy(&count, allocated[1].first, sizeof(count));
-    return count != 0;
+    unsigned long long counts[2];  // of the queue's parts
+    std::memcpy(counts, allocated[1].first, sizeof(counts));
+    return counts[0] != 0 || counts[1] != 0;
 }
 }  // namespace
 
@@ -51,11 +51,11 @@ static int launch(const void* func) {
     if (launches++ == fake_fail_launch) return last_error = 719;
     if (fake_capturing) return 0;
     const std::string& name = names()[func];
-    const unsigned one = 1;
+    const unsigned long long one[2] = {1, 1};
     if (name.find("k_splat_raster") != std::string::npos) {
         if (marked()) ++fake_dirty_frames;
         std::memset(allocated[0].first, 0x11, allocated[0].second);
-        std::memcpy(allocated[1].first, &one, sizeof(one));
+        std::memcpy(allocated[1].first, one, sizeof(one));
     } else if (name.find("k_splat_resolve") != std::string::npos) {
         std::memset(allocated[0].first, 0xFF, allocated[0].second);
         std::memset(allocated[1].first, 0, sizeof(one));
