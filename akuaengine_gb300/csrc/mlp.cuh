@@ -251,14 +251,14 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
         asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kTile) : "memory");
         if (t == 0) tc::fence_after_sync();
     };
-    // after a wait that ran out nothing waits again and nothing is written
+    // after a wait that ran out nothing is issued or written any more
     auto wait = [&]() {
         if (ok) ok = tc::mbar_wait(&S.bar[group], phase);
         phase ^= 1;
         tc::fence_after_sync();
     };
     auto layer = [&](uint32_t sw) {
-        if (t == 0) {
+        if (t == 0 && ok) {
 #pragma unroll
             for (int s = 0; s < kHid / 16; ++s)
                 tc::mma_bf16(tmem, tc::smem_desc(sh + 256 * s, 128, kHid * 16),
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
             make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
                        pack_bf16(f[6], f[7]));
         publish();
-        if (t == 0) {
+        if (t == 0 && ok) {
             tc::mma_bf16(tmem, dx, dw1, idesc, 0);
             tc::mma_commit(&S.bar[group]);
         }
